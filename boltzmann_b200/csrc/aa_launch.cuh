@@ -69,11 +69,22 @@ StepArgs<Real> make_step_args(const lbm_sim& s, bool write_moments) {
   return a;
 }
 
-template <class Real>
-void step_geometry(const StepArgs<Real>& a, dim3& grid, dim3& block) {
-  const int bx = a.nz >= 256 ? 256 : ((a.nz + 31) / 32) * 32;
-  block = dim3(bx, 1, 1);
-  grid = dim3((a.nz + bx - 1) / bx, a.ny < 65535 ? a.ny : 65535, a.nx < 65535 ? a.nx : 65535);
+// Launches a step kernel as a programmatic dependent of the previous one on the stream (the kernels
+// wait for it on the device before they touch memory).
+template <class... Params, class... Args>
+cudaError_t launch_step_kernel(void (*kern)(Params...), unsigned grid, unsigned threads,
+                               size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // Ring depth of the TMA kernel: as many stages as fit in ~50 KB per CTA (2-4), so that three or
@@ -184,8 +195,7 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
                                                               TracerLattice<L::D>::type::Q);
     maps.use = ok ? 1 : 0;
   }
-  kern<<<(unsigned)grid, threads, smem, stream>>>(a, maps);
-  return cudaGetLastError();
+  return launch_step_kernel(kern, (unsigned)grid, threads, smem, stream, a, maps);
 }
 
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
@@ -209,10 +219,11 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
       return e;
     }
   }
-  dim3 grid, block;
-  step_geometry(a, grid, block);
-  aa_step_kernel<L, TRT, K, EVEN, NT, KT><<<grid, block, 0, stream>>>(a);
-  const cudaError_t e = cudaGetLastError();
+  const DirectArgs d = make_direct_args<L>(a, sizeof(typename Pop<K>::type),
+                                           sizeof(typename TracerPop<KT>::type));
+  const unsigned grid = (unsigned)(((long long)d.cells + kDirectThreads - 1) / kDirectThreads);
+  const cudaError_t e = launch_step_kernel(aa_step_kernel<L, TRT, K, EVEN, NT, KT>, grid,
+                                           kDirectThreads, 0, stream, a, d);
   if (e == cudaSuccess) ++launches[0];
   return e;
 }

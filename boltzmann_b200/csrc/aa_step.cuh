@@ -44,6 +44,29 @@ struct TracerArgs {
   int trt;
 };
 
+// Division of a 32-bit dividend by a run-time constant as one high multiply, an add and two shifts
+// (T. Granlund, P. Montgomery, "Division by invariant integers using multiplication", PLDI 1994):
+// with l = ceil(log2 d), mul = floor(2^32 (2^l - d) / d) + 1, exact for every dividend.
+struct FastDiv {
+  unsigned d = 1, mul = 1, sh1 = 0, sh2 = 0;
+  FastDiv() = default;
+  explicit FastDiv(unsigned divisor) : d(divisor) {
+    unsigned l = 0;
+    while (l < 32 && (1ull << l) < d) ++l;
+    mul = (unsigned)((((1ull << l) - d) << 32) / d) + 1;
+    sh1 = l < 1 ? l : 1;
+    sh2 = l < 1 ? 0 : l - 1;
+  }
+  __host__ __device__ unsigned div(unsigned n) const {
+#ifdef __CUDA_ARCH__
+    const unsigned t = __umulhi(mul, n);
+#else
+    const unsigned t = (unsigned)(((unsigned long long)mul * n) >> 32);
+#endif
+    return (t + ((n - t) >> sh1)) >> sh2;
+  }
+};
+
 template <class Real>
 struct StepArgs {
   void* f;             // [Q][N] in the storage type
@@ -51,7 +74,7 @@ struct StepArgs {
   Real* vel;           // [N][D]
   const uint8_t* flags;
   int nx, ny, nz;      // 2D domains use nx = 1, (ny, nz) = the reference's (x, y) counts
-  long long n;         // cell count
+  long long n;         // cells between the slots of a population array
   Real om_pos, om_neg; // BGK uses om_pos
   int acc_mode;        // 0: none, 1: constant acceleration acc[], 2: Boussinesq
   Real force[3];       // velocity shift per unit buoyancy: acc / om_pos (constant acceleration,
@@ -67,6 +90,35 @@ struct StepArgs {
   int* status;         // bit 0 set when a non-finite density or velocity is produced
   unsigned spin_limit; // polls of a staged kernel's pipeline waits before it gives up (bit 1)
 };
+
+// The first element of each slot of the population array and of the first tracer's: constant-bank
+// operands of the kernels that take them, so a population's address is one multiply-add of the cell
+// index.
+struct SlotTable {
+  void* f[27];
+  void* g[7];
+};
+
+// What the direct kernels take besides StepArgs.
+struct DirectArgs {
+  FastDiv by_nz, by_ny;
+  unsigned cells;  // nx * ny * nz
+  SlotTable slots;
+};
+
+template <class L, class Real>
+DirectArgs make_direct_args(const StepArgs<Real>& a, size_t pop_bytes, size_t tracer_bytes) {
+  DirectArgs d{};
+  d.by_nz = FastDiv((unsigned)a.nz);
+  d.by_ny = FastDiv((unsigned)a.ny);
+  d.cells = (unsigned)a.nx * (unsigned)a.ny * (unsigned)a.nz;
+  for (int i = 0; i < L::Q; ++i)
+    d.slots.f[i] = static_cast<char*>(a.f) + (size_t)i * (size_t)a.n * pop_bytes;
+  if (a.ntracers > 0)
+    for (int i = 0; i < TracerLattice<L::D>::type::Q; ++i)
+      d.slots.g[i] = static_cast<char*>(a.tr[0].g) + (size_t)i * (size_t)a.n * tracer_bytes;
+  return d;
+}
 
 enum AccMode : int { kAccNone = 0, kAccConstant = 1, kAccBoussinesq = 2 };
 
@@ -111,16 +163,24 @@ struct CellPos {
   }
 };
 
+// Slot i of a [q][n] population array: from the table of slot bases among the kernel arguments
+// (TABLE), or from the array's base and the slot stride n.
+template <bool TABLE, class T>
+__device__ __forceinline__ T* slot_ptr(void* base, void* const* table, long long n, int i) {
+  return TABLE ? static_cast<T*>(table[i]) : static_cast<T*>(base) + (size_t)i * n;
+}
+
 // AA load of one velocity set's populations for this cell: deviations d_i = f_i - W_i when DEV,
 // full values otherwise.
-template <class L, class P, bool EVEN, bool DEV>
-__device__ __forceinline__ void aa_load(const typename P::type* __restrict__ f, long long n,
+template <class L, class P, bool EVEN, bool DEV, bool TABLE = false>
+__device__ __forceinline__ void aa_load(void* base, void* const* table, long long n,
                                         const CellPos& c, typename P::real (&v)[L::Q]) {
   using Real = typename P::real;
+  using T = typename P::type;
 #pragma unroll
   for (int i = 0; i < L::Q; ++i) {
-    const typename P::type* p =
-        EVEN ? (f + (size_t)i * n) + c.upstream<L>(i) : (f + (size_t)opp(i) * n) + c.cell;
+    const T* p = EVEN ? slot_ptr<TABLE, T>(base, table, n, i) + c.upstream<L>(i)
+                      : slot_ptr<TABLE, T>(base, table, n, opp(i)) + c.cell;
     // Slot i (even) and slot opp(i) (odd) share the weight of direction i.
     if constexpr (DEV)
       v[i] = P::load_dev(p, weight<L, Real>(i));
@@ -130,13 +190,14 @@ __device__ __forceinline__ void aa_load(const typename P::type* __restrict__ f, 
 }
 
 // AA store matching aa_load.
-template <class L, class P, bool EVEN, bool DEV>
-__device__ __forceinline__ void aa_store(typename P::type* __restrict__ f, long long n,
+template <class L, class P, bool EVEN, bool DEV, bool TABLE = false>
+__device__ __forceinline__ void aa_store(void* base, void* const* table, long long n,
                                          const CellPos& c, const typename P::real (&v)[L::Q]) {
   using Real = typename P::real;
+  using T = typename P::type;
 #pragma unroll
   for (int i = 0; i < L::Q; ++i) {
-    typename P::type* p = (f + (size_t)i * n) + (EVEN ? c.upstream<L>(i) : c.cell);
+    T* p = slot_ptr<TABLE, T>(base, table, n, i) + (EVEN ? c.upstream<L>(i) : c.cell);
     const Real val = EVEN ? v[opp(i)] : v[i];
     if constexpr (DEV)
       P::store_dev(p, val, weight<L, Real>(i));
@@ -145,19 +206,35 @@ __device__ __forceinline__ void aa_store(typename P::type* __restrict__ f, long 
   }
 }
 
+// The same position as far as the values go, but opaque to the compiler: addresses formed from it
+// are computed anew instead of being kept, two registers each, since the loads.
+template <bool EVEN>
+__device__ __forceinline__ CellPos renewed(CellPos c) {
+  asm volatile("" : "+r"(c.cell));
+  if constexpr (EVEN)
+    asm volatile("" : "+r"(c.ox[0]), "+r"(c.ox[1]), "+r"(c.ox[2]), "+r"(c.oy[0]), "+r"(c.oy[1]),
+                 "+r"(c.oy[2]), "+r"(c.oz[0]), "+r"(c.oz[1]), "+r"(c.oz[2]));
+  return c;
+}
+
 // Where update_cell puts the post-collision populations: the AA store straight to HBM. (The
 // TMA kernel passes a sink that writes them into its shared-memory stage instead, from where whole
-// row segments go back with bulk copies.)
+// row segments go back with bulk copies.) TABLE: see slot_ptr. RENEW: addresses computed anew.
+template <bool TABLE = false, bool RENEW = false>
 struct GlobalSink {
+  const SlotTable* table = nullptr;
+
   template <class L, class P, bool EVEN, bool DEV>
-  __device__ __forceinline__ void fluid(typename P::type* f, long long n, const CellPos& c,
+  __device__ __forceinline__ void fluid(void* f, long long n, const CellPos& c,
                                         const typename P::real (&v)[L::Q]) const {
-    aa_store<L, P, EVEN, DEV>(f, n, c, v);
+    aa_store<L, P, EVEN, DEV, TABLE>(f, TABLE ? table->f : nullptr, n,
+                                     RENEW ? renewed<EVEN>(c) : c, v);
   }
   template <class TL, class TP, bool EVEN>
-  __device__ __forceinline__ void tracer(typename TP::type* g, long long n, const CellPos& c,
+  __device__ __forceinline__ void tracer(void* g, long long n, const CellPos& c,
                                          const typename TP::real (&v)[TL::Q]) const {
-    aa_store<TL, TP, EVEN, false>(g, n, c, v);
+    aa_store<TL, TP, EVEN, false, TABLE>(g, TABLE ? table->g : nullptr, n,
+                                         RENEW ? renewed<EVEN>(c) : c, v);
   }
 };
 
@@ -380,7 +457,7 @@ __device__ __forceinline__ void moments_packed(float (&v)[L::Q], float& dr, floa
 // (src/lib.cl:102-189, 303-405), with its populations already loaded into g. TRT tracers take
 // the pair update of the fluid's TRT with their own rates, both 1 on fixed-value cells (the
 // D2Q5 / D3Q7 TRT kernels of python/boltzmann/kernel_gen.py:368-421).
-template <class TL, class TP, bool EVEN, bool PACK, class Real, class Sink = GlobalSink>
+template <class TL, class TP, bool EVEN, bool PACK, class Real, class Sink = GlobalSink<>>
 __device__ __forceinline__ void tracer_update(const TracerArgs<Real>& tr, long long n,
                                               const CellPos& c, int flag, Real (&g)[TL::Q],
                                               const Real (&u)[3], Real uu, bool keep,
@@ -406,7 +483,7 @@ __device__ __forceinline__ void tracer_update(const TracerArgs<Real>& tr, long l
     else
       collide<TL, false, false>(g, rt, rt, u, uu, om, om);
   }
-  sink.template tracer<TL, TP, EVEN>(static_cast<typename TP::type*>(tr.g), n, c, g);
+  sink.template tracer<TL, TP, EVEN>(tr.g, n, c, g);
   if (keep && !tfixed) tr.val[c.cell] = rt;
 }
 
@@ -439,7 +516,7 @@ __device__ __forceinline__ CellPos make_cellpos(const StepArgs<Real>& a, int x, 
 // KT: storage kind of the fused tracers' populations (TracerPop).
 // UNFORCED: no body force, coupling or relaxation field by construction (batched ensembles), so
 // their per-cell checks are left out (+5% on the FP16 ensemble kernel).
-template <class L, bool TRT, int K, bool EVEN, int NT, class Sink = GlobalSink,
+template <class L, bool TRT, int K, bool EVEN, int NT, class Sink = GlobalSink<>,
           int KT = default_tracer_kind<K>(), bool UNFORCED = false>
 __device__ __forceinline__ void update_cell(const StepArgs<typename Pop<K>::real>& a,
                                             const CellPos& c, int flag,
@@ -451,7 +528,6 @@ __device__ __forceinline__ void update_cell(const StepArgs<typename Pop<K>::real
                                             const Sink& sink = Sink()) {
   using P = Pop<K>;
   using Real = typename P::real;
-  using T = typename P::type;
   using TL = typename TracerLattice<L::D>::type;
   using TP = TracerPop<KT>;
   constexpr int Q = L::Q;
@@ -539,7 +615,7 @@ __device__ __forceinline__ void update_cell(const StepArgs<typename Pop<K>::real
     collide_packed<L, TRT, true>(f, r, dr, u, uu, om_pos, om_neg);
   else
     collide<L, TRT, true>(f, r, dr, u, uu, om_pos, om_neg);
-  sink.template fluid<L, P, EVEN, true>(static_cast<T*>(a.f), a.n, c, f);
+  sink.template fluid<L, P, EVEN, true>(a.f, a.n, c, f);
 
   if (a.write_moments && !fixed) {
     a.rho[c.cell] = r;
@@ -555,44 +631,81 @@ __device__ __forceinline__ void update_cell(const StepArgs<typename Pop<K>::real
   } else if constexpr (NT < 0) {
     for (int t = 0; t < a.ntracers; ++t) {
       Real gt[TL::Q];
-      aa_load<TL, TP, EVEN, false>(static_cast<const typename TP::type*>(a.tr[t].g), a.n, c, gt);
+      aa_load<TL, TP, EVEN, false>(a.tr[t].g, nullptr, a.n, c, gt);
       const bool keep = a.write_moments || (a.acc_mode == kAccBoussinesq && t == a.coupled);
       tracer_update<TL, TP, EVEN, pack_collide<TL, K>()>(a.tr[t], a.n, c, flag, gt, u, uu, keep);
     }
   }
 }
 
-// Direct variant: one cell per thread and grid row, loads straight into registers.
+// Programmatic dependent launch: the next step's grid may be scheduled as soon as every CTA of this
+// one has started (launch_dependents), so its launch, its index arithmetic and this grid's tail
+// overlap; it touches memory only after this grid has completed (wait).
+__device__ __forceinline__ void grid_trigger_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+constexpr int kDirectThreads = 128;
+// How the direct kernel of a lattice, storage and tracer form addresses populations, and the CTAs
+// an SM its registers must allow. A D3Q27 cell has 54 addresses; kept from the loads to the stores
+// they cost 114-142 registers a thread (four CTAs an SM, too few loads in flight). Formed anew for
+// the stores, from slot bases in the constant bank, they leave 84-113: 180 x 100 x 90 TRT with a
+// tracer 90.2 -> 79.2 us a step, 200^3 BGK 312 -> 292 (FP32), 234 -> 221 (FP16). Five CTAs for
+// FP32 (six spill, 15% slower on 32^3), six for 16-bit populations. FP64 and D2Q9 without a tracer
+// are better off keeping them (256^2: 2.22 us a step against 2.32; the constant-bank table, cold in
+// every CTA, 2.57); D2Q9 with a tracer gains from forming them anew at ten CTAs (300^2: 3.15 ->
+// 2.81).
+template <class L, int K, int NT>
+struct DirectForm {
+  static constexpr bool k27 = L::Q >= 27;
+  static constexpr bool table = k27 && K != kF64;
+  static constexpr bool renew = table || (NT == 1 && (k27 || K != kF64));
+  static constexpr int blocks =
+      K == kF64 ? (k27 ? 3 : 5) : (k27 ? (K == kF32 ? 5 : 6) : (NT == 1 ? 10 : 8));
+};
+
+// Direct variant: one cell per thread, loads straight into registers; for domains whose rows do not
+// split into whole tiles, and small ones. Bound by the latency of one dependent chain per step on
+// small domains, by the instruction stream and the loads in flight on large ones.
+// Threads take the cells in order whatever the row length (two divisions by invariants): a CTA per
+// row left lanes without a cell on rows that are no multiple of 32 (half of them on 48 x 62 x 17)
+// and short CTAs on long ones. With the dependent launches: 64^2 1.94 -> 1.56 us a step, 300^2 with
+// a tracer 3.83 -> 3.15, 1000 x 501 7.13 -> 6.00, 100 x 90 x 35 (BF16, tracer) 20.5 -> 11.6.
 // NT: number of fused tracers known at compile time (0 or 1), or -1 for a runtime count.
 // Every load a cell needs is issued before the first branch on any loaded value, so each thread
 // has one memory phase (walls load populations they then ignore; they are a small fraction).
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
-__global__ void __launch_bounds__(256)
-    aa_step_kernel(const __grid_constant__ StepArgs<typename Pop<K>::real> a) {
+__global__ void __launch_bounds__(kDirectThreads, DirectForm<L, K, NT>::blocks)
+    aa_step_kernel(const __grid_constant__ StepArgs<typename Pop<K>::real> a,
+                   const __grid_constant__ DirectArgs d) {
   using P = Pop<K>;
   using Real = typename P::real;
-  using T = typename P::type;
   using TL = typename TracerLattice<L::D>::type;
   using TP = TracerPop<KT>;
+  using Form = DirectForm<L, K, NT>;
 
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  if (z >= a.nz) return;
-
-  for (int x = blockIdx.z; x < a.nx; x += gridDim.z) {
-    for (int y = blockIdx.y; y < a.ny; y += gridDim.y) {
-      const CellPos c = make_cellpos(a, x, y, z, EVEN);
-      const int flag = a.flags[c.cell];
-      Real f[L::Q];
-      aa_load<L, P, EVEN, dev_in<K>()>(static_cast<const T*>(a.f), a.n, c, f);
-      Real g[NT == 1 ? TL::Q : 1];
-      if constexpr (NT == 1)
-        aa_load<TL, TP, EVEN, false>(static_cast<const typename TP::type*>(a.tr[0].g), a.n, c, g);
-      Real cval = 0;
-      if (a.acc_mode == kAccBoussinesq) cval = a.coupled_val[c.cell];
-      update_cell<L, TRT, K, EVEN, NT, GlobalSink, KT>(a, c, flag, f, g, cval, a.om_pos,
-                                                      a.om_neg);
-    }
-  }
+  grid_trigger_next();
+  const unsigned cell = blockIdx.x * (unsigned)kDirectThreads + threadIdx.x;
+  const unsigned row = d.by_nz.div(cell);
+  const int z = (int)(cell - row * (unsigned)a.nz);
+  const unsigned x = L::D == 2 ? 0u : d.by_ny.div(row);
+  const CellPos c = make_cellpos(a, (int)x, (int)(row - x * (unsigned)a.ny), z, EVEN);
+  grid_wait_previous();
+  if (cell >= d.cells) return;
+  const int flag = a.flags[c.cell];
+  Real f[L::Q];
+  aa_load<L, P, EVEN, dev_in<K>(), Form::table>(a.f, d.slots.f, a.n, c, f);
+  Real g[NT == 1 ? TL::Q : 1];
+  if constexpr (NT == 1)
+    aa_load<TL, TP, EVEN, false, Form::table>(a.tr[0].g, d.slots.g, a.n, c, g);
+  Real cval = 0;
+  if (a.acc_mode == kAccBoussinesq) cval = a.coupled_val[c.cell];
+  update_cell<L, TRT, K, EVEN, NT, GlobalSink<Form::table, Form::renew>, KT>(
+      a, c, flag, f, g, cval, a.om_pos, a.om_neg,
+      GlobalSink<Form::table, Form::renew>{Form::table ? &d.slots : nullptr});
 }
 
 }  // namespace lbm

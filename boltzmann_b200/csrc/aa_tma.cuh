@@ -287,8 +287,8 @@ struct StageSink {
   int tid;
 
   template <class LL, class P, bool EVEN, bool DEV>
-  __device__ __forceinline__ void fluid(typename P::type*, long long, const CellPos&,
-                                        const typename P::real (&v)[LL::Q]) const {
+  __device__ __forceinline__ void fluid(void*, long long, const CellPos&,
+                                        const Real (&v)[LL::Q]) const {
     using T = typename P::type;
     T* base = reinterpret_cast<T*>(st);
 #pragma unroll
@@ -311,8 +311,8 @@ struct StageSink {
     }
   }
   template <class TLL, class TP, bool EVEN>
-  __device__ __forceinline__ void tracer(typename TP::type*, long long, const CellPos&,
-                                         const typename TP::real (&v)[TLL::Q]) const {
+  __device__ __forceinline__ void tracer(void*, long long, const CellPos&,
+                                         const Real (&v)[TLL::Q]) const {
     using TT = typename TP::type;
     TT* base = reinterpret_cast<TT*>(st + St::off_trc);
 #pragma unroll
@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(tma_threads<PAIR>(), tma_min_blocks<L, K, PAIR
   using TT = typename TP::type;
   constexpr int Q = L::Q;
 
+  grid_trigger_next();
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)S * St::bytes);
   uint64_t* empty = full + S;
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(tma_threads<PAIR>(), tma_min_blocks<L, K, PAIR
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  grid_wait_previous();
 
   if (warp == CW) {
     // ---- producer warp. Each lane owns up to two copy jobs (job = lane, lane + 32), fixed for

@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(512)
     const int flagA = a.flags[c[0].cell];
     const int flagB = hasB ? a.flags[c[1].cell] : 1;  // a missing cell acts as a wall
     Real fa[D2Q9::Q], fb[D2Q9::Q];
-    aa_load<D2Q9, P, EVEN, lbm::dev_in<K>()>(static_cast<const T*>(a.f), a.n, c[0], fa);
-    if (hasB) aa_load<D2Q9, P, EVEN, lbm::dev_in<K>()>(static_cast<const T*>(a.f), a.n, c[1], fb);
+    aa_load<D2Q9, P, EVEN, lbm::dev_in<K>()>(a.f, nullptr, a.n, c[0], fa);
+    if (hasB) aa_load<D2Q9, P, EVEN, lbm::dev_in<K>()>(a.f, nullptr, a.n, c[1], fb);
     Real g[1];
     update_cell<D2Q9, TRT, K, EVEN, 0>(a, c[0], flagA, fa, g, Real(0), (Real)dom.om_pos,
                                        (Real)dom.om_neg);
@@ -177,7 +177,7 @@ struct RowStoreSink {
   T* const* rows;  // slot i's row, at its position 0
 
   template <class L, class P, bool EVEN, bool DEV>
-  __device__ __forceinline__ void fluid(T*, long long, const lbm::CellPos& c,
+  __device__ __forceinline__ void fluid(void*, long long, const lbm::CellPos& c,
                                         const Real (&v)[L::Q]) const {
 #pragma unroll
     for (int i = 0; i < L::Q; ++i) {
@@ -191,8 +191,8 @@ struct RowStoreSink {
     }
   }
   template <class TL, class TP, bool EVEN>
-  __device__ __forceinline__ void tracer(typename TP::type*, long long, const lbm::CellPos&,
-                                         const typename TP::real (&)[TL::Q]) const {}
+  __device__ __forceinline__ void tracer(void*, long long, const lbm::CellPos&,
+                                         const Real (&)[TL::Q]) const {}
 };
 
 template <bool TRT, int K, bool EVEN>
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kRowThreads)
         update_cell<D2Q9, TRT, K, EVEN, 0, RowStoreSink<K>, default_tracer_kind<K>(), true>(
             a, c, flag, fv, g, Real(0), om_p, om_n, RowStoreSink<K>{out_rows});
       else
-        update_cell<D2Q9, TRT, K, EVEN, 0, GlobalSink, default_tracer_kind<K>(), true>(
+        update_cell<D2Q9, TRT, K, EVEN, 0, GlobalSink<>, default_tracer_kind<K>(), true>(
             a, c, flag, fv, g, Real(0), om_p, om_n);
     }
     __syncwarp();
@@ -539,12 +539,14 @@ cudaError_t launch_per_domain(lbm_ensemble* e, bool even, bool write_moments) {
     a.nz = dom.ny;
     a.om_pos = dom.om_pos;
     a.om_neg = dom.om_neg;
-    const int bx = a.nz >= 256 ? 256 : ((a.nz + 31) / 32) * 32;
-    const dim3 grid((a.nz + bx - 1) / bx, a.ny, 1);
+    const lbm::DirectArgs args = lbm::make_direct_args<lbm::D2Q9>(a, sizeof(T), 0);
+    const unsigned grid = (args.cells + lbm::kDirectThreads - 1) / lbm::kDirectThreads;
     if (even)
-      lbm::aa_step_kernel<lbm::D2Q9, TRT, K, true, 0><<<grid, bx, 0, e->stream>>>(a);
+      lbm::aa_step_kernel<lbm::D2Q9, TRT, K, true, 0>
+          <<<grid, lbm::kDirectThreads, 0, e->stream>>>(a, args);
     else
-      lbm::aa_step_kernel<lbm::D2Q9, TRT, K, false, 0><<<grid, bx, 0, e->stream>>>(a);
+      lbm::aa_step_kernel<lbm::D2Q9, TRT, K, false, 0>
+          <<<grid, lbm::kDirectThreads, 0, e->stream>>>(a, args);
     cudaError_t r = cudaGetLastError();
     if (r != cudaSuccess) return r;
   }
