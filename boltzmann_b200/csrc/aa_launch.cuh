@@ -162,8 +162,7 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
   // steps whose results go back through the stage (D3Q27 TRT needs more than the 128 registers
   // three CTAs a SM leave a thread, and spills); D2Q9 BGK / TRT with none or one fused tracer, on
   // every step.
-  constexpr bool PAIR = dev_in<K>() && ((L::Q >= 27 && !TRT && NT == 0 && (!EVEN || WR)) ||
-                                        (L::D == 2 && NT >= 0 && NT <= 1));
+  constexpr bool PAIR = pair_form<L, TRT, K, NT>() && (L::D == 2 || !EVEN || WR);
   constexpr int threads = tma_threads<PAIR>();
   auto kern = aa_tma_kernel<L, TRT, K, EVEN, NT, S, WR, PAIR, KT>;
   static std::once_flag once;
@@ -221,6 +220,15 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
   }
   const DirectArgs d = make_direct_args<L>(a, sizeof(typename Pop<K>::type),
                                            sizeof(typename TracerPop<KT>::type));
+  if constexpr (pair_form<L, TRT, K, NT>()) {
+    if ((long long)d.cells >= kPairDirectCells) {
+      const unsigned grid = (unsigned)(((long long)d.cells + 2 * kDirectThreads - 1) / (2 * kDirectThreads));
+      const cudaError_t e = launch_step_kernel(aa_step2_kernel<L, TRT, K, EVEN, NT, KT>, grid,
+                                               kDirectThreads, 0, stream, a, d);
+      if (e == cudaSuccess) ++launches[0];
+      return e;
+    }
+  }
   const unsigned grid = (unsigned)(((long long)d.cells + kDirectThreads - 1) / kDirectThreads);
   const cudaError_t e = launch_step_kernel(aa_step_kernel<L, TRT, K, EVEN, NT, KT>, grid,
                                            kDirectThreads, 0, stream, a, d);

@@ -280,4 +280,110 @@ __device__ __forceinline__ void update_cell2(const StepArgs<float>& a, const Sin
   }
 }
 
+// update_cell2's results straight to HBM, like GlobalSink.
+template <bool RENEW>
+struct GlobalPairSink {
+  const SlotTable& table;
+  const CellPos &cA, &cB;
+
+  template <class L, class P, bool EVEN>
+  __device__ __forceinline__ void fluid(bool skipA, bool skipB, const float2 (&v)[L::Q]) const {
+    using T = typename P::type;
+    put<L, P, EVEN, true, T>(table.f, skipA, skipB, v);
+  }
+  template <class TL, class TP, bool EVEN>
+  __device__ __forceinline__ void tracer(bool skipA, bool skipB, const float2 (&v)[TL::Q]) const {
+    using T = typename TP::type;
+    put<TL, TP, EVEN, false, T>(table.g, skipA, skipB, v);
+  }
+
+ private:
+  template <class L, class P, bool EVEN, bool DEV, class T>
+  __device__ __forceinline__ void put(void* const* slots, bool skipA, bool skipB,
+                                      const float2 (&v)[L::Q]) const {
+    const CellPos eA = RENEW ? renewed<EVEN>(cA) : cA, eB = RENEW ? renewed<EVEN>(cB) : cB;
+#pragma unroll
+    for (int i = 0; i < L::Q; ++i) {
+      T* slot = static_cast<T*>(slots[i]);
+      T* pa = slot + (EVEN ? eA.upstream<L>(i) : eA.cell);
+      T* pb = slot + (EVEN ? eB.upstream<L>(i) : eB.cell);
+      const float2 val = EVEN ? v[opp(i)] : v[i];
+      if constexpr (DEV) {
+        if (!skipA) P::store_dev(pa, val.x, 0.0f);
+        if (!skipB) P::store_dev(pb, val.y, 0.0f);
+      } else {
+        if (!skipA) P::store(pa, val.x, 0.0f);
+        if (!skipB) P::store(pb, val.y, 0.0f);
+      }
+    }
+  }
+};
+
+// Whether a simulation's 16-bit kernels update two cells a thread: D3Q27 BGK without a tracer, and
+// D2Q9 with none or one. (D3Q27 TRT needs more registers than that leaves a thread, and spills.)
+template <class L, bool TRT, int K, int NT>
+constexpr bool pair_form() {
+  return dev_in<K>() && ((L::Q >= 27 && !TRT && NT == 0) || (L::D == 2 && (NT == 0 || NT == 1)));
+}
+// Smallest domain (cells) for the direct two-cell kernel, 1024 cells an SM: below it the CTAs of
+// 256 cells would leave SMs short of warps.
+constexpr long long kPairDirectCells = 148LL * 1024;
+
+// The direct kernel with two cells a thread, for 16-bit populations: cells t and t + 128 of the
+// CTA's 256 consecutive cells. A 16-bit cell keeps half the bytes of an FP32 one in flight and
+// spends as many instructions; two cells on packed instructions mend both. 200^3 BGK 221 -> 194
+// us a step, 3000 x 1001 TRT with a 16-bit tracer 41.9 -> 38.6, 2000 x 1000 18.4 -> 16.1. Four CTAs
+// an SM for D3Q27 (three 220, five 214), six for D2Q9 (five 42.4, eight 45.0).
+template <class L, bool TRT, int K, bool EVEN, int NT, int KT>
+__global__ void __launch_bounds__(kDirectThreads, L::Q >= 27 ? 4 : 6)
+    aa_step2_kernel(const __grid_constant__ StepArgs<float> a,
+                    const __grid_constant__ DirectArgs d) {
+  using P = Pop<K>;
+  using T = typename P::type;
+  using TL = typename TracerLattice<L::D>::type;
+  using TP = TracerPop<KT>;
+  using TT = typename TP::type;
+
+  grid_trigger_next();
+  const unsigned first = blockIdx.x * (unsigned)(2 * kDirectThreads) + threadIdx.x;
+  CellPos c[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    unsigned cell = first + (unsigned)(k * kDirectThreads);
+    if (cell >= d.cells) cell = first < d.cells ? first : 0u;  // a missing cell: see its flag
+    const unsigned row = d.by_nz.div(cell);
+    const unsigned x = L::D == 2 ? 0u : d.by_ny.div(row);
+    c[k] = make_cellpos(a, (int)x, (int)(row - x * (unsigned)a.ny),
+                        (int)(cell - row * (unsigned)a.nz), EVEN);
+  }
+  grid_wait_previous();
+  if (first >= d.cells) return;
+  const bool hasB = d.cells - first > (unsigned)kDirectThreads;
+  const int flagA = a.flags[c[0].cell];
+  const int flagB = hasB ? a.flags[c[1].cell] : 1;  // a missing cell acts as a wall
+  float2 f[L::Q];
+#pragma unroll
+  for (int i = 0; i < L::Q; ++i) {
+    const T* slot = static_cast<const T*>(d.slots.f[EVEN ? i : opp(i)]);
+    f[i] = make_float2(
+        P::load_dev(slot + (EVEN ? c[0].template upstream<L>(i) : c[0].cell), 0.0f),
+        P::load_dev(slot + (EVEN ? c[1].template upstream<L>(i) : c[1].cell), 0.0f));
+  }
+  float2 g[NT == 1 ? TL::Q : 1];
+  if constexpr (NT == 1) {
+#pragma unroll
+    for (int i = 0; i < TL::Q; ++i) {
+      const TT* slot = static_cast<const TT*>(d.slots.g[EVEN ? i : opp(i)]);
+      g[i] = make_float2(
+          TP::load(slot + (EVEN ? c[0].template upstream<TL>(i) : c[0].cell), 0.0f),
+          TP::load(slot + (EVEN ? c[1].template upstream<TL>(i) : c[1].cell), 0.0f));
+    }
+  }
+  float2 cval = make_float2(0.0f, 0.0f);
+  if (a.acc_mode == kAccBoussinesq)
+    cval = make_float2(a.coupled_val[c[0].cell], a.coupled_val[c[1].cell]);
+  update_cell2<L, TRT, K, EVEN, NT, KT>(a, GlobalPairSink<true>{d.slots, c[0], c[1]}, c[0], c[1], flagA,
+                                        flagB, f, g, cval);
+}
+
 }  // namespace lbm
