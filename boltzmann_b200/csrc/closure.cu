@@ -5,17 +5,18 @@
 // activations.
 //
 //   layer   forward                       backward
-//   1 (4->32)   CUDA cores (36 MAC/out)    weights: CUDA cores; no input gradient
+//   1 (4->32)   CUDA cores (36 MAC/out)    weights: mma.sync; no input gradient
 //   2 (32->32)  tcgen05 BF16, FP32 acc     data: tcgen05 (transposed conv, fused GELU');
 //               (TMEM accumulators)        weights: mma.sync (cells are the reduction axis)
 //               mma.sync kept selectable (lbm_closure_set_layer2_kernel)
-//   3 (32->1)   CUDA cores                 data + weights: CUDA cores (fused GELU')
+//   3 (32->1)   CUDA cores                 data: CUDA cores (fused GELU'); weights: mma.sync, dy
+//                                          as the exact sum of three BF16 parts
 //
 // Every product sum takes BF16 operands (weights, activations, pre-activation gradients rounded
 // to nearest even) and accumulates in FP32. Reductions over cells run per tile in a fixed order
 // into per-CTA partial rows, which one kernel adds row by row: results are deterministic.
 //
-// Cell tiles are 4 rows (x) by 64 columns (y, the contiguous axis). Shared-memory tiles keep 40
+// Cell tiles are 4 rows (x) by 64 columns (y, the contiguous axis) unless a kernel says otherwise. Shared-memory tiles keep 40
 // BF16 per cell (80 bytes): eight consecutive cells then start in eight different 16-byte bank
 // groups, so ldmatrix reads them without conflicts. Weight rows (one per output channel) are
 // padded from 288 to 296 BF16 (592 bytes) for the same reason.
@@ -73,11 +74,13 @@ struct Grid {
   }
 };
 
-Grid make_grid(int64_t nx, int64_t ny, int64_t batch) {
-  Grid g{nx, ny, batch, (nx + kTX - 1) / kTX, (ny + kTY - 1) / kTY, 0};
+// The domains of a batch in tiles of rows x cols cells.
+Grid tiles_of(int64_t nx, int64_t ny, int64_t batch, int rows, int cols) {
+  Grid g{nx, ny, batch, (nx + rows - 1) / rows, (ny + cols - 1) / cols, 0};
   g.tiles = g.tx * g.ty * batch;
   return g;
 }
+Grid make_grid(int64_t nx, int64_t ny, int64_t batch) { return tiles_of(nx, ny, batch, kTX, kTY); }
 
 // ---------------------------------------------------------------------------------------------
 // Scalar helpers
@@ -159,16 +162,96 @@ __device__ __forceinline__ void load_cells32(const bf16* __restrict__ src, const
   }
 }
 
-// The 4-channel input features with the halo, into dst[cell][4].
-__device__ __forceinline__ void load_cells4(const bf16* __restrict__ src, const Grid& g, int64_t b,
-                                            int64_t x0, int64_t y0, bf16* dst) {
-  for (int i = threadIdx.x; i < kHX * kHY; i += blockDim.x) {
-    const int r = i / kHY, c = i - r * kHY;
-    const int64_t x = x0 - 1 + r, y = y0 - 1 + c;
-    uint2 v = make_uint2(0, 0);
-    if (x >= 0 && x < g.nx && y >= 0 && y < g.ny)
-      v = __ldg(reinterpret_cast<const uint2*>(src + g.cell(b, x, y) * 4));
-    *reinterpret_cast<uint2*>(dst + i * 4) = v;
+// A 16-byte asynchronous copy into shared memory, zeros when !valid (src is then not read).
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// load_cells32 by asynchronous copies (the caller commits and waits).
+template <int ROWS, int COLS>
+__device__ __forceinline__ void load_cells32_async(const bf16* __restrict__ src, const Grid& g,
+                                                   int64_t b, int64_t xs, int64_t ys, bf16* dst) {
+  for (int i = threadIdx.x; i < ROWS * COLS * 4; i += blockDim.x) {
+    const int chunk = i & 3, cell = i >> 2;
+    const int r = cell / COLS, c = cell - r * COLS;
+    const int64_t x = xs + r, y = ys + c;
+    const bool in = x >= 0 && x < g.nx && y >= 0 && y < g.ny;
+    cp_async16(dst + cell * kCS + chunk * 8, in ? src + g.cell(b, x, y) * C + chunk * 8 : src, in);
+  }
+}
+
+// A tile's 4-channel features with the halo in registers (zero outside the domain): loaded a tile
+// ahead, then handed cell by cell (index in the kHX x kHY region) to `f`.
+template <int THREADS>
+struct FeatureTile {
+  static constexpr int N = (kHX * kHY + THREADS - 1) / THREADS;
+  uint2 v[N];
+  __device__ __forceinline__ void load(const bf16* __restrict__ src, const Grid& g, int64_t t) {
+    int64_t b, x0, y0;
+    g.tile(t, b, x0, y0);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int i = threadIdx.x + k * THREADS;
+      const int r = i / kHY, c = i - r * kHY;
+      const int64_t x = x0 - 1 + r, y = y0 - 1 + c;
+      v[k] = make_uint2(0, 0);
+      if (i < kHX * kHY && x >= 0 && x < g.nx && y >= 0 && y < g.ny)
+        v[k] = __ldg(reinterpret_cast<const uint2*>(src + g.cell(b, x, y) * 4));
+    }
+  }
+  template <class F>
+  __device__ __forceinline__ void each(F f) const {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int i = threadIdx.x + k * THREADS;
+      if (i < kHX * kHY) f(i, v[k]);
+    }
+  }
+};
+
+// Two FP32 fused multiply-adds on one packed instruction, each rounded as fmaf.
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// gelu of two values, its multiplications and additions on packed instructions (the same bits).
+__device__ __forceinline__ float2 gelu2(float2 z) {
+  const float2 zz = __fmul2_rn(z, z);
+  const float2 v = __fmul2_rn(z, ffma2(make_float2(kGeluB, kGeluB), zz, make_float2(kGeluA, kGeluA)));
+  const float2 d = __fadd2_rn(make_float2(1.0f, 1.0f), make_float2(__expf(-v.x), __expf(-v.y)));
+  return make_float2(__fdividef(z.x, d.x), __fdividef(z.y, d.y));
+}
+
+__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t pack_bf2(float2 v) { return pack_bf2(v.x, v.y); }
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
+// The element-wise kernels of layers 1 and 3 give a cell to two neighbouring lanes (g2 = lane & 1),
+// 16 channels each in four groups of four: channels 8 k + 4 g2 .. + 3, k = 0 .. 3. FP32 rows then
+// move as full 32-byte sectors (two lanes x 16 bytes), and after a swap between the two lanes the
+// BF16 rows too: `w` holds the lane's packed groups; afterwards lane g2 = 0 has channels 0-7 and
+// 16-23, lane 1 channels 8-15 and 24-31, which it stores at 16-byte chunks g2 and g2 + 2.
+__device__ __forceinline__ void store_bf16_row(bf16* row, uint32_t (&w)[4][2], int g2, bool valid) {
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const uint32_t s0 = g2 ? w[k][0] : w[k + 1][0], s1 = g2 ? w[k][1] : w[k + 1][1];
+    const uint32_t r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
+    const uint32_t r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+    const uint4 v = g2 ? make_uint4(r0, r1, w[k + 1][0], w[k + 1][1])
+                       : make_uint4(w[k][0], w[k][1], r0, r1);
+    if (valid) reinterpret_cast<uint4*>(row)[k + g2] = v;
   }
 }
 
@@ -275,67 +358,94 @@ __global__ void features_kernel(const float* __restrict__ rho, const float* __re
 }
 
 // ---------------------------------------------------------------------------------------------
-// Layer 1 forward (CUDA cores): 36 MACs per output.
+// Layer 1 forward (CUDA cores): 36 MACs per output, in FP32 on packed instructions (two channels
+// each). Bound by the FMA pipe (1152 a cell) beside 200 bytes a cell of traffic. A warp takes one row
+// of the tile, two lanes a cell (store_bf16_row) and four cells a lane, so that each shared-memory
+// weight load feeds eight FMAs; the inputs lie in shared memory as (v, v) pairs, the packed
+// instruction's operand. Batch 8 x 1024 x 512: 635 -> 336 us.
 
-__global__ void __launch_bounds__(256)
+constexpr int kC1Threads = 32 * kTX;
+constexpr int kC1Cells = kTY / 16;  // cells a lane
+constexpr int kC1PerSm = 3;
+
+__global__ void __launch_bounds__(kC1Threads, kC1PerSm)
     conv1_fwd_kernel(Grid g, const bf16* __restrict__ x, const bf16* __restrict__ w1,
                      const float* __restrict__ b1, float* __restrict__ z1, bf16* __restrict__ a1) {
-  __shared__ __align__(16) bf16 xs[kHX * kHY * 4];
-  __shared__ __align__(16) float ws[9 * 4 * C];  // [tap][ci][co]
+  __shared__ __align__(16) float xs[kHX * kHY * 8];  // [cell][ci] as (v, v)
+  __shared__ __align__(16) float ws[9 * 4 * C];      // [tap][ci][co]
   for (int i = threadIdx.x; i < 9 * 4 * C; i += blockDim.x) {
     const int co = i / 36, r = i - co * 36;  // w1 is [co][tap][ci]
     ws[r * C + co] = bf(w1[i]);
   }
-  const int ti = threadIdx.x / kTY, tj = threadIdx.x % kTY;
+  const int ti = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g2 = lane & 1, lc = lane >> 1;
+  float4 bias[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float* b = b1 + 8 * k + 4 * g2;
+    bias[k] = make_float4(b[0], b[1], b[2], b[3]);
+  }
+  FeatureTile<kC1Threads> in;  // the next tile's features, loaded while this one is computed
+  if ((int64_t)blockIdx.x < g.tiles) in.load(x, g, blockIdx.x);
   for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
     int64_t b, x0, y0;
     g.tile(t, b, x0, y0);
     __syncthreads();
-    load_cells4(x, g, b, x0, y0, xs);
+    in.each([&](int i, uint2 v) {
+      float4* d = reinterpret_cast<float4*>(xs + i * 8);
+      d[0] = make_float4(bf_lo(v.x), bf_lo(v.x), bf_hi(v.x), bf_hi(v.x));
+      d[1] = make_float4(bf_lo(v.y), bf_lo(v.y), bf_hi(v.y), bf_hi(v.y));
+    });
     __syncthreads();
-    const int64_t xx = x0 + ti, yy = y0 + tj;
-    if (xx >= g.nx || yy >= g.ny) continue;
-    float acc[C];
+    if (t + gridDim.x < g.tiles) in.load(x, g, t + gridDim.x);
+    float2 acc[kC1Cells][8];
 #pragma unroll
-    for (int co = 0; co < C; ++co) acc[co] = 0.0f;
+    for (int p = 0; p < kC1Cells; ++p)
 #pragma unroll
+      for (int q = 0; q < 8; ++q) acc[p][q] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
     for (int tap = 0; tap < 9; ++tap) {
       const int dx = tap / 3 - 1, dy = tap % 3 - 1;
-      const bf16* xv = xs + ((ti + 1 + dx) * kHY + tj + 1 + dy) * 4;
+      const float* xc = xs + ((ti + 1 + dx) * kHY + lc + 1 + dy) * 8;
+      const float* wt = ws + tap * 4 * C + 4 * g2;
 #pragma unroll
-      for (int ci = 0; ci < 4; ++ci) {
-        const float v = bf(xv[ci]);
-        const float4* wr = reinterpret_cast<const float4*>(ws + (tap * 4 + ci) * C);
+      for (int h = 0; h < 2; ++h) {  // input channels 2 h, 2 h + 1
+        float4 v[kC1Cells];
 #pragma unroll
-        for (int q = 0; q < C / 4; ++q) {
-          const float4 w = wr[q];
-          acc[4 * q + 0] = fmaf(v, w.x, acc[4 * q + 0]);
-          acc[4 * q + 1] = fmaf(v, w.y, acc[4 * q + 1]);
-          acc[4 * q + 2] = fmaf(v, w.z, acc[4 * q + 2]);
-          acc[4 * q + 3] = fmaf(v, w.w, acc[4 * q + 3]);
+        for (int p = 0; p < kC1Cells; ++p)
+          v[p] = *reinterpret_cast<const float4*>(xc + p * 16 * 8 + 4 * h);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 w = *reinterpret_cast<const float4*>(wt + (2 * h + e) * C + 8 * k);
+#pragma unroll
+            for (int p = 0; p < kC1Cells; ++p) {
+              const float2 vv = e ? make_float2(v[p].z, v[p].w) : make_float2(v[p].x, v[p].y);
+              acc[p][2 * k] = ffma2(vv, make_float2(w.x, w.y), acc[p][2 * k]);
+              acc[p][2 * k + 1] = ffma2(vv, make_float2(w.z, w.w), acc[p][2 * k + 1]);
+            }
+          }
         }
       }
     }
-    const int64_t cell = g.cell(b, xx, yy);
-    uint32_t packed[C / 2];
+    const int64_t xx = x0 + ti;
 #pragma unroll
-    for (int co = 0; co < C; co += 2) {
-      const float za = acc[co] + b1[co], zb = acc[co + 1] + b1[co + 1];
-      acc[co] = za;
-      acc[co + 1] = zb;
-      packed[co / 2] = (uint32_t)__bfloat16_as_ushort(to_bf(gelu(za))) |
-                       ((uint32_t)__bfloat16_as_ushort(to_bf(gelu(zb))) << 16);
+    for (int p = 0; p < kC1Cells; ++p) {
+      const int64_t yy = y0 + lc + 16 * p;
+      const bool valid = xx < g.nx && yy < g.ny;
+      const int64_t cell = valid ? g.cell(b, xx, yy) : 0;
+      uint32_t w[4][2];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 z = make_float4(acc[p][2 * k].x + bias[k].x, acc[p][2 * k].y + bias[k].y,
+                                     acc[p][2 * k + 1].x + bias[k].z, acc[p][2 * k + 1].y + bias[k].w);
+        if (z1 != nullptr && valid) *reinterpret_cast<float4*>(z1 + cell * C + 8 * k + 4 * g2) = z;
+        w[k][0] = pack_bf2(gelu2(make_float2(z.x, z.y)));
+        w[k][1] = pack_bf2(gelu2(make_float2(z.z, z.w)));
+      }
+      store_bf16_row(a1 + cell * C, w, g2, valid);
     }
-    if (z1 != nullptr) {
-      float4* zp = reinterpret_cast<float4*>(z1 + cell * C);
-#pragma unroll
-      for (int q = 0; q < C / 4; ++q)
-        zp[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-    }
-    uint4* ap = reinterpret_cast<uint4*>(a1 + cell * C);
-#pragma unroll
-    for (int q = 0; q < C / 8; ++q)
-      ap[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
   }
 }
 
@@ -476,53 +586,68 @@ __global__ void __launch_bounds__(kConv32Threads)
 
 // ---------------------------------------------------------------------------------------------
 // Layer-2 weight gradient on tensor cores: dW[co][tap][ci] = sum_p dz[p][co] a1[p + tap][ci].
-// One warp per tap: M = 32 output channels (2 m-tiles), N = 32 input channels (4 n-tiles),
-// K = the cells of the CTA's tiles, 16 per k-step.
+// M = 32 output channels (2 m-tiles), N = 32 input channels (4 n-tiles), K = the cells of the CTA's
+// tiles, 16 per k-step. Warp (i, dx) takes tile row i and the three taps (dx, -1 .. 1): the dz
+// fragments it loads serve 24 MMAs (one warp a tap loaded them for eight). The next tile's operands
+// arrive (asynchronous copies) while this one's are multiplied. Bound by shared-memory reads (eight
+// ldmatrix a 24 MMAs). Batch 8 x 1024 x 512: 366 -> 311 us.
 
-constexpr int kDw2Threads = 9 * 32;
-constexpr size_t kDw2Smem = (size_t)(kTX * kTY * kCS + kHX * kHY * kCS) * sizeof(bf16);
+constexpr int kDw2Threads = 3 * kTX * 32;
+constexpr int kDw2Stage = (kTX * kTY + kHX * kHY) * kCS;  // BF16 elements of one stage
+constexpr size_t kDw2Smem = (size_t)2 * kDw2Stage * sizeof(bf16);
+static_assert((size_t)C * 288 * 4 <= kDw2Smem, "the cross-row sums must fit the stages");
 
-__global__ void __launch_bounds__(kDw2Threads)
+__global__ void __launch_bounds__(kDw2Threads, 1)
     conv32_wgrad_kernel(Grid g, const bf16* __restrict__ a1, const bf16* __restrict__ dz2,
                         float* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* dzs = reinterpret_cast<bf16*>(smem_raw);  // [kTX * kTY][kCS]
-  bf16* as = dzs + kTX * kTY * kCS;               // [kHX * kHY][kCS]
-  const int tap = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int dx = tap / 3 - 1, dy = tap % 3 - 1;
+  bf16* stages = reinterpret_cast<bf16*>(smem_raw);  // [2][dz [kTX * kTY][kCS], a1 [kHX * kHY][kCS]]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int dx = warp % 3 - 1, row = warp / 3;
   const int mi = lane >> 3, rr = lane & 7;
 
-  float acc[2][4][4];
+  float acc[3][2][4][4];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int d = 0; d < 3; ++d)
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[mt][nt][e] = 0.0f;
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[d][mt][nt][e] = 0.0f;
 
-  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
+  auto fetch = [&](int64_t t, int s) {
     int64_t b, x0, y0;
     g.tile(t, b, x0, y0);
+    bf16* st = stages + s * kDw2Stage;
+    load_cells32_async<kTX, kTY>(dz2, g, b, x0, y0, st);
+    load_cells32_async<kHX, kHY>(a1, g, b, x0 - 1, y0 - 1, st + kTX * kTY * kCS);
+  };
+  int s = 0;
+  if ((int64_t)blockIdx.x < g.tiles) fetch(blockIdx.x, 0);
+  cp_async_commit();
+  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, s ^= 1) {
+    if (t + gridDim.x < g.tiles) fetch(t + gridDim.x, s ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
     __syncthreads();
-    load_cells32<kTX, kTY>(dz2, g, b, x0, y0, dzs);
-    load_cells32<kHX, kHY>(a1, g, b, x0 - 1, y0 - 1, as);
-    __syncthreads();
+    const bf16* dzs = stages + s * kDw2Stage;
+    const bf16* as = dzs + kTX * kTY * kCS;
 #pragma unroll 1
-    for (int i = 0; i < kTX; ++i) {
+    for (int c = 0; c < kTY / 16; ++c) {
+      const int k0 = c * 16 + (mi >> 1) * 8 + rr, k1 = c * 16 + (mi & 1) * 8 + rr;
+      uint32_t afrag[2][4];
 #pragma unroll
-      for (int c = 0; c < kTY / 16; ++c) {
-        uint32_t afrag[2][4];
+      for (int mt = 0; mt < 2; ++mt)
+        ldsm_x4_t(afrag[mt], dzs + (row * kTY + k0) * kCS + mt * 16 + (mi & 1) * 8);
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          const int p = i * kTY + c * 16 + (mi >> 1) * 8 + rr;
-          ldsm_x4_t(afrag[mt], dzs + p * kCS + mt * 16 + (mi & 1) * 8);
-        }
+      for (int d = 0; d < 3; ++d) {
+        const bf16* ap = as + ((row + 1 + dx) * kHY + k1 + d) * kCS + (mi >> 1) * 8;
         uint32_t bfrag[4][2];
 #pragma unroll
         for (int np = 0; np < 2; ++np) {
           uint32_t r[4];
-          const int col = c * 16 + (mi & 1) * 8 + rr;
-          ldsm_x4_t(r, as + ((i + 1 + dx) * kHY + col + 1 + dy) * kCS + (2 * np + (mi >> 1)) * 8);
+          ldsm_x4_t(r, ap + np * 16);
           bfrag[2 * np][0] = r[0];
           bfrag[2 * np][1] = r[1];
           bfrag[2 * np + 1][0] = r[2];
@@ -531,251 +656,556 @@ __global__ void __launch_bounds__(kDw2Threads)
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt) mma_bf16(acc[mt][nt], afrag[mt], bfrag[nt][0], bfrag[nt][1]);
+          for (int nt = 0; nt < 4; ++nt)
+            mma_bf16(acc[d][mt][nt], afrag[mt], bfrag[nt][0], bfrag[nt][1]);
       }
     }
+    __syncthreads();  // stage s is free for the tile after the next
   }
+  cp_async_wait<0>();
+  __syncthreads();
 
-  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W2;
+  // The four tile rows' sums, added in row order, then this CTA's partial row.
+  float* sums = reinterpret_cast<float*>(smem_raw);  // [co][288]
   const int gq = lane >> 2, tq = lane & 3;
+  for (int r = 0; r < kTX; ++r) {
+    if (row == r) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int co = mt * 16 + gq + 8 * h, ci = nt * 8 + 2 * tq;
+              float2* p = reinterpret_cast<float2*>(sums + co * 288 + ((dx + 1) * 3 + d) * 32 + ci);
+              float2 v = make_float2(acc[d][mt][nt][2 * h], acc[d][mt][nt][2 * h + 1]);
+              if (r > 0) {
+                const float2 o = *p;
+                v = make_float2(o.x + v.x, o.y + v.y);
+              }
+              *p = v;
+            }
+    }
+    __syncthreads();
+  }
+  float* out = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W2;
+  for (int i = threadIdx.x; i < C * 288; i += blockDim.x) out[i] = sums[i];
+}
+
+// ---------------------------------------------------------------------------------------------
+// Layer 3 (32 -> 1) forward: y[p] = b3 + sum_{tap,ci} w3[tap][ci] a2[p + tap][ci], as one product per
+// cell, P[q][tap] = sum_ci w3[tap][ci] a2[q][ci], whose nine shifted values each output adds: every
+// activation is read and widened once instead of nine times. FP32 on packed instructions (two
+// channels each): tensor cores would do it for less, but their accumulation leans to one side, and
+// the loss, an average over all cells, shows it. Three cells a thread, so that each shared-memory
+// weight load feeds four of them. Batch 8 x 1024 x 512: 216 -> 118 us.
+
+constexpr int kC3R = 30;                          // output rows of a tile (kTY columns)
+constexpr int kC3RegR = kC3R + 2, kC3RegC = kHY;  // region with the halo
+constexpr int kC3Cells = kC3RegR * kC3RegC;       // 2112
+constexpr int kC3Per = 2, kC3Threads = 352;       // three passes of two cells a thread
+constexpr size_t kConv3Smem = (size_t)9 * kC3Cells * 4 + (size_t)9 * C * 4;
+static_assert(kC3Cells % (kC3Threads * kC3Per) == 0 && kC3Threads % 32 == 0, "whole passes");
+
+__global__ void __launch_bounds__(kC3Threads, 2)
+    conv3_fwd_kernel(Grid g, const bf16* __restrict__ a2, const bf16* __restrict__ w3,
+                     const float* __restrict__ b3, float* __restrict__ y) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* ps = reinterpret_cast<float*>(smem_raw);  // [9][kC3Cells]
+  float* ws = ps + 9 * kC3Cells;                   // [tap][ci]
+  for (int i = threadIdx.x; i < 9 * C; i += blockDim.x) ws[i] = bf(w3[i]);
+  const float bias = b3[0];
+  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
+    int64_t b, x0, y0;
+    {
+      const int64_t per = g.tx * g.ty;  // this kernel's tiles are kC3R x kTY (see the launcher)
+      b = t / per;
+      const int64_t r = t - b * per;
+      x0 = (r / g.ty) * kC3R;
+      y0 = (r % g.ty) * kTY;
+    }
+    __syncthreads();  // the previous tile's P has been read (and, at first, ws written)
+#pragma unroll 1
+    for (int q0 = threadIdx.x; q0 < kC3Cells; q0 += kC3Per * kC3Threads) {
+      uint4 v[kC3Per][C / 8];
+#pragma unroll
+      for (int p = 0; p < kC3Per; ++p) {
+        const int q = q0 + p * kC3Threads;
+        const int r = q / kC3RegC, c = q - r * kC3RegC;
+        const int64_t x = x0 - 1 + r, yy = y0 - 1 + c;
+        const bool in = x >= 0 && x < g.nx && yy >= 0 && yy < g.ny;
+        const uint4* src = reinterpret_cast<const uint4*>(a2 + (in ? g.cell(b, x, yy) : 0) * C);
+#pragma unroll
+        for (int k = 0; k < C / 8; ++k) v[p][k] = in ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
+      }
+      float2 acc[kC3Per][9];
+#pragma unroll
+      for (int p = 0; p < kC3Per; ++p)
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap) acc[p][tap] = make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int k = 0; k < C / 8; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float2 a[kC3Per][2];
+#pragma unroll
+          for (int p = 0; p < kC3Per; ++p) {
+            const uint32_t u0 = h ? v[p][k].z : v[p][k].x, u1 = h ? v[p][k].w : v[p][k].y;
+            a[p][0] = make_float2(bf_lo(u0), bf_hi(u0));
+            a[p][1] = make_float2(bf_lo(u1), bf_hi(u1));
+          }
+#pragma unroll
+          for (int tap = 0; tap < 9; ++tap) {
+            const float4 w = *reinterpret_cast<const float4*>(ws + tap * C + k * 8 + 4 * h);
+#pragma unroll
+            for (int p = 0; p < kC3Per; ++p) {
+              acc[p][tap] = ffma2(a[p][0], make_float2(w.x, w.y), acc[p][tap]);
+              acc[p][tap] = ffma2(a[p][1], make_float2(w.z, w.w), acc[p][tap]);
+            }
+          }
+        }
+#pragma unroll
+      for (int p = 0; p < kC3Per; ++p)
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap)
+          ps[tap * kC3Cells + q0 + p * kC3Threads] = acc[p][tap].x + acc[p][tap].y;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kC3R * kTY; i += kC3Threads) {
+      const int r = i / kTY, c = i - r * kTY;
+      const int64_t x = x0 + r, yy = y0 + c;
+      if (x >= g.nx || yy >= g.ny) continue;
+      float s = 0.0f;
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap)
+        s += ps[tap * kC3Cells + (r + tap / 3) * kC3RegC + c + tap % 3];
+      y[g.cell(b, x, yy)] = s + bias;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Layer 3 backward. Per tile:
+//   dz2[q][ci] = BF16( GELU'(z2[q][ci]) sum_tap w3[tap][ci] dy[q - tap] )
+//   dW3[tap][ci] += sum_q a2[q][ci] dy[q - tap],  db3 += sum_q dy[q],  db2[ci] += sum_q dz2[q][ci]
+// The first line in FP32 on packed instructions, two lanes a cell (store_bf16_row) and two cells a
+// lane. The weight gradient on tensor cores: M = (part, tap), N = ci, K = cells, where dy enters as
+// the exact sum of three BF16 parts (8 + 8 + 8 significant bits), so that every product is that of
+// the FP32 value; the parts' sums are added at the end. (One thread an output over the tile's 256
+// cells was the kernel's longest part by far.) Bound by 260 bytes a cell. Batch 8 x 1024 x 512: 978 -> 332 us.
+
+constexpr int kB3Threads = 256;
+constexpr int kDyS = kHY + 2;  // BF16 elements of a row of a dy part (a multiple of 2)
+// A stage holds the tile's a2 [cell][kCS] and z2 [cell][C], whose 16-byte chunk c of cell p lies at
+// chunk c ^ 2 (p % 4): four cells' chunks, which a quarter warp reads at once, in different banks.
+constexpr size_t kB3OffZ = (size_t)kTX * kTY * kCS * 2;
+constexpr size_t kB3Stage = kB3OffZ + (size_t)kTX * kTY * C * 4;
+constexpr size_t kB3OffDy2 = 2 * kB3Stage;                             // dy as (v, v) pairs
+constexpr size_t kB3OffPart = kB3OffDy2 + (size_t)kHX * kHY * 8;       // [part][shift][kHX][kDyS]
+constexpr size_t kB3OffW = kB3OffPart + (size_t)3 * 2 * kHX * kDyS * 2;
+constexpr size_t kConv3BwdSmem = kB3OffW + (size_t)9 * C * 4;
+static_assert(kB3OffPart % 16 == 0 && kB3OffW % 16 == 0, "aligned parts");
+constexpr int kB3Sums = 27 * C + C + 1;  // a warp's sums at the end: dW3 parts, db2, db3
+static_assert((size_t)(kB3Threads / 32) * kB3Sums * 4 <= kConv3BwdSmem, "the sums must fit");
+
+__global__ void __launch_bounds__(kB3Threads, 2)
+    conv3_bwd_kernel(Grid g, const bf16* __restrict__ a2, const float* __restrict__ z2,
+                     const bf16* __restrict__ w3, const float* __restrict__ dy,
+                     bf16* __restrict__ dz2, float* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* dy2 = reinterpret_cast<float2*>(smem_raw + kB3OffDy2);     // [kHX * kHY]
+  bf16* dyp = reinterpret_cast<bf16*>(smem_raw + kB3OffPart);
+  float* ws = reinterpret_cast<float*>(smem_raw + kB3OffW);          // [tap][ci]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g2 = lane & 1, lc = lane >> 1, gq = lane >> 2, tq = lane & 3;
+  const int mi = lane >> 3, rr = lane & 7;
+  const int ti = warp >> 1, tj = (warp & 1) * 32;  // this warp's 32 cells: row ti, columns tj ..
+  for (int i = threadIdx.x; i < 9 * C; i += blockDim.x) ws[i] = bf(w3[i]);
+  for (int i = threadIdx.x; i < 3 * 2 * kHX * kDyS; i += blockDim.x) dyp[i] = to_bf(0.0f);
+
+  // A fragments of the weight gradient: rows m = gq, gq + 8 of the two m-tiles, m = 9 part + tap
+  // (rows 27 .. 31: none). Element k of row m is dy part `part` at column j - dyy + 1 (with the
+  // halo) of tile row ti - dx + 1; pairs (k, k + 1) at an odd column come from the copy that is
+  // shifted by one element.
+  int aoff[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int m = gq + 8 * e;
+    aoff[e] = -1;
+    if (m < 27) {
+      const int part = m / 9, tap = m % 9;
+      const int col = tj + 1 - (tap % 3 - 1), r = ti + 1 - (tap / 3 - 1), odd = col & 1;
+      aoff[e] = ((part * 2 + odd) * kHX + r) * kDyS + col - odd + 2 * tq;
+    }
+  }
+  float acc[2][4][4];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int co = mt * 16 + gq + 8 * h, ci = nt * 8 + 2 * tq;
-        row[co * 288 + tap * 32 + ci] = acc[mt][nt][2 * h];
-        row[co * 288 + tap * 32 + ci + 1] = acc[mt][nt][2 * h + 1];
-      }
-}
+      for (int e = 0; e < 4; ++e) acc[mt][nt][e] = 0.0f;
+  float bsum[16];  // db2 of this lane's channels 8 k + 4 g2 + e
+#pragma unroll
+  for (int k = 0; k < 16; ++k) bsum[k] = 0.0f;
+  float dsum = 0.0f;  // db3
 
-// ---------------------------------------------------------------------------------------------
-// Layer 3 (32 -> 1) forward, CUDA cores: y[p] = b3 + sum_{tap,ci} w3[tap][ci] a2[p + tap][ci].
-
-constexpr size_t kConv3Smem = (size_t)kHX * kHY * kCS * sizeof(bf16);
-
-__global__ void __launch_bounds__(256)
-    conv3_fwd_kernel(Grid g, const bf16* __restrict__ a2, const bf16* __restrict__ w3,
-                     const float* __restrict__ b3, float* __restrict__ y) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* as = reinterpret_cast<bf16*>(smem_raw);
-  __shared__ float ws[9 * C];
-  for (int i = threadIdx.x; i < 9 * C; i += blockDim.x) ws[i] = bf(w3[i]);
-  const int ti = threadIdx.x / kTY, tj = threadIdx.x % kTY;
-  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
+  // The next tile's operands are in flight while this one is computed: a2 and z2 by asynchronous
+  // copies, dy in registers.
+  constexpr int kDyN = (kHX * kHY + kB3Threads - 1) / kB3Threads;
+  float dyv[kDyN];
+  auto fetch = [&](int64_t t, int s) {
     int64_t b, x0, y0;
     g.tile(t, b, x0, y0);
-    __syncthreads();
-    load_cells32<kHX, kHY>(a2, g, b, x0 - 1, y0 - 1, as);
-    __syncthreads();
-    const int64_t xx = x0 + ti, yy = y0 + tj;
-    if (xx >= g.nx || yy >= g.ny) continue;
-    float acc = 0.0f;
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-      const int dx = tap / 3 - 1, dy = tap % 3 - 1;
-      const bf16* av = as + ((ti + 1 + dx) * kHY + tj + 1 + dy) * kCS;
-#pragma unroll
-      for (int q = 0; q < C / 8; ++q) {
-        const uint4 v = *reinterpret_cast<const uint4*>(av + q * 8);
-        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float lo = __uint_as_float(w4[e] << 16), hi = __uint_as_float(w4[e] & 0xffff0000u);
-          acc = fmaf(lo, ws[tap * C + q * 8 + 2 * e], acc);
-          acc = fmaf(hi, ws[tap * C + q * 8 + 2 * e + 1], acc);
-        }
-      }
+    unsigned char* st = smem_raw + (size_t)s * kB3Stage;
+    load_cells32_async<kTX, kTY>(a2, g, b, x0, y0, reinterpret_cast<bf16*>(st));
+    for (int i = threadIdx.x; i < kTX * kTY * 8; i += kB3Threads) {
+      const int chunk = i & 7, p = i >> 3;
+      const int64_t x = x0 + p / kTY, yv = y0 + p % kTY;
+      const bool in = x < g.nx && yv < g.ny;
+      cp_async16(st + kB3OffZ + p * 128 + ((chunk ^ (2 * (p & 3))) * 16),
+                 in ? z2 + g.cell(b, x, yv) * C + chunk * 4 : z2, in);
     }
-    y[g.cell(b, xx, yy)] = acc + b3[0];
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Layer 3 backward, CUDA cores. Per tile:
-//   dz2[q][ci] = BF16( GELU'(z2[q][ci]) sum_tap w3[tap][ci] dy[q - tap] )
-//   dW3[tap][ci] += sum_p a2[p + tap][ci] dy[p],  db3 += sum_p dy[p],  db2[ci] += sum_q dz2[q][ci]
-
-constexpr size_t kConv3BwdSmem =
-    (size_t)kHX * kHY * kCS * sizeof(bf16) + (size_t)kTX * kTY * (C + 1) * sizeof(float);
-
-__global__ void __launch_bounds__(256)
-    conv3_bwd_kernel(Grid g, const bf16* __restrict__ a2, const float* __restrict__ z2,
-                     const bf16* __restrict__ w3, const float* __restrict__ dy,
-                     bf16* __restrict__ dz2, float* __restrict__ partial) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* as = reinterpret_cast<bf16*>(smem_raw);                           // [kHX*kHY][kCS]
-  float* dzs = reinterpret_cast<float*>(smem_raw + kHX * kHY * kCS * 2);  // [256][C + 1]
-  __shared__ float ws[9 * C];
-  __shared__ float dys[kHX * kHY];
-  for (int i = threadIdx.x; i < 9 * C; i += blockDim.x) ws[i] = bf(w3[i]);
-  const int ti = threadIdx.x / kTY, tj = threadIdx.x % kTY;
-  float wacc[2] = {0.0f, 0.0f};  // outputs k = threadIdx.x and threadIdx.x + 256 of [dW3, db3]
-  float bsum = 0.0f;             // threads < 32: db2[threadIdx.x]
-
-  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
-    int64_t b, x0, y0;
-    g.tile(t, b, x0, y0);
-    __syncthreads();
-    load_cells32<kHX, kHY>(a2, g, b, x0 - 1, y0 - 1, as);
-    for (int i = threadIdx.x; i < kHX * kHY; i += blockDim.x) {
+#pragma unroll
+    for (int k = 0; k < kDyN; ++k) {
+      const int i = threadIdx.x + k * kB3Threads;
       const int r = i / kHY, c = i - r * kHY;
       const int64_t x = x0 - 1 + r, yv = y0 - 1 + c;
-      dys[i] = (x >= 0 && x < g.nx && yv >= 0 && yv < g.ny) ? dy[g.cell(b, x, yv)] : 0.0f;
+      dyv[k] = (i < kHX * kHY && x >= 0 && x < g.nx && yv >= 0 && yv < g.ny)
+                   ? dy[g.cell(b, x, yv)]
+                   : 0.0f;
     }
+  };
+  int stage = 0;
+  if ((int64_t)blockIdx.x < g.tiles) fetch(blockIdx.x, 0);
+  cp_async_commit();
+  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, stage ^= 1) {
+    int64_t b, x0, y0;
+    g.tile(t, b, x0, y0);
+    __syncthreads();  // the previous tile is done with dy2, dyp and its stage
+    const bf16* as = reinterpret_cast<const bf16*>(smem_raw + (size_t)stage * kB3Stage);
+    const unsigned char* zs = smem_raw + (size_t)stage * kB3Stage + kB3OffZ;
+#pragma unroll
+    for (int k3 = 0; k3 < kDyN; ++k3) {
+      const int i = threadIdx.x + k3 * kB3Threads;
+      if (i >= kHX * kHY) break;
+      const int r = i / kHY, c = i - r * kHY;
+      const float v = dyv[k3];
+      dy2[i] = make_float2(v, v);
+      // v = h + m + l exactly (a non-finite v stays in h)
+      const bool fin = fabsf(v) <= 3.0e38f;
+      const bf16 h = to_bf(v);
+      const float vm = fin ? __fsub_rn(v, bf(h)) : 0.0f;
+      const bf16 m = to_bf(vm);
+      const bf16 l = to_bf(__fsub_rn(vm, bf(m)));
+      const bf16 part[3] = {h, m, l};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        dyp[((k * 2) * kHX + r) * kDyS + c] = part[k];
+        if (c > 0) dyp[((k * 2 + 1) * kHX + r) * kDyS + c - 1] = part[k];
+      }
+    }
+    if (t + gridDim.x < g.tiles) fetch(t + gridDim.x, stage ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
     __syncthreads();
 
-    const int64_t xx = x0 + ti, yy = y0 + tj;
-    float* drow = dzs + threadIdx.x * (C + 1);
-    if (xx < g.nx && yy < g.ny) {
-      const int64_t cell = g.cell(b, xx, yy);
-      float d[C];
+    const int64_t xx = x0 + ti;
+    float2 d[2][8];
 #pragma unroll
-      for (int ci = 0; ci < C; ++ci) d[ci] = 0.0f;
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-      for (int tap = 0; tap < 9; ++tap) {
-        const int dx = tap / 3 - 1, dyy = tap % 3 - 1;
-        const float v = dys[(ti + 1 - dx) * kHY + tj + 1 - dyy];
+      for (int q = 0; q < 8; ++q) d[p][q] = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int ci = 0; ci < C; ++ci) d[ci] = fmaf(ws[tap * C + ci], v, d[ci]);
+    for (int tap = 0; tap < 9; ++tap) {
+      const int dx = tap / 3 - 1, dyy = tap % 3 - 1;
+      const float2* vp = dy2 + (ti + 1 - dx) * kHY + tj + lc + 1 - dyy;
+      const float2 v0 = vp[0], v1 = vp[16];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + tap * C + 8 * k + 4 * g2);
+        d[0][2 * k] = ffma2(make_float2(w.x, w.y), v0, d[0][2 * k]);
+        d[0][2 * k + 1] = ffma2(make_float2(w.z, w.w), v0, d[0][2 * k + 1]);
+        d[1][2 * k] = ffma2(make_float2(w.x, w.y), v1, d[1][2 * k]);
+        d[1][2 * k + 1] = ffma2(make_float2(w.z, w.w), v1, d[1][2 * k + 1]);
       }
-      uint32_t packed[C / 2];
-#pragma unroll
-      for (int ci = 0; ci < C; ci += 4) {
-        const float4 z = *reinterpret_cast<const float4*>(z2 + cell * C + ci);
-        const bf16 h0 = to_bf(d[ci] * gelu_grad(z.x)), h1 = to_bf(d[ci + 1] * gelu_grad(z.y));
-        const bf16 h2 = to_bf(d[ci + 2] * gelu_grad(z.z)), h3 = to_bf(d[ci + 3] * gelu_grad(z.w));
-        drow[ci] = bf(h0);
-        drow[ci + 1] = bf(h1);
-        drow[ci + 2] = bf(h2);
-        drow[ci + 3] = bf(h3);
-        packed[ci / 2] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        packed[ci / 2 + 1] =
-            (uint32_t)__bfloat16_as_ushort(h2) | ((uint32_t)__bfloat16_as_ushort(h3) << 16);
-      }
-      uint4* op = reinterpret_cast<uint4*>(dz2 + cell * C);
-#pragma unroll
-      for (int q = 0; q < C / 8; ++q)
-        op[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-    } else {
-#pragma unroll
-      for (int ci = 0; ci < C; ++ci) drow[ci] = 0.0f;
     }
-    __syncthreads();
-
-    // Weight and bias sums over the tile's cells, each output owned by one thread.
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int k = threadIdx.x + 256 * e;
-      if (k > 9 * C) continue;
-      float s = 0.0f;
-      if (k == 9 * C) {
-        for (int p = 0; p < kTX * kTY; ++p) s += dys[(p / kTY + 1) * kHY + p % kTY + 1];
-      } else {
-        const int tap = k / C, ci = k % C;
-        const int dx = tap / 3 - 1, dyy = tap % 3 - 1;
-        for (int p = 0; p < kTX * kTY; ++p) {
-          const int pi = p / kTY, pj = p % kTY;
-          s = fmaf(bf(as[((pi + 1 + dx) * kHY + pj + 1 + dyy) * kCS + ci]),
-                   dys[(pi + 1) * kHY + pj + 1], s);
+    for (int p = 0; p < 2; ++p) {
+      const int64_t yy = y0 + tj + lc + 16 * p;
+      const bool valid = xx < g.nx && yy < g.ny;
+      const int64_t cell = valid ? g.cell(b, xx, yy) : 0;
+      uint32_t w[4][2];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int q = ti * kTY + tj + lc + 16 * p;
+        const float4 z = *reinterpret_cast<const float4*>(
+            zs + q * 128 + (((2 * k + g2) ^ (2 * (q & 3))) * 16));
+        w[k][0] = pack_bf2(d[p][2 * k].x * gelu_grad(z.x), d[p][2 * k].y * gelu_grad(z.y));
+        w[k][1] = pack_bf2(d[p][2 * k + 1].x * gelu_grad(z.z), d[p][2 * k + 1].y * gelu_grad(z.w));
+        if (valid) {
+          bsum[4 * k] += bf_lo(w[k][0]);
+          bsum[4 * k + 1] += bf_hi(w[k][0]);
+          bsum[4 * k + 2] += bf_lo(w[k][1]);
+          bsum[4 * k + 3] += bf_hi(w[k][1]);
         }
       }
-      wacc[e] += s;
+      store_bf16_row(dz2 + cell * C, w, g2, valid);
     }
-    if (threadIdx.x < C) {
-      float s = 0.0f;
-      for (int p = 0; p < kTX * kTY; ++p) s += dzs[p * (C + 1) + threadIdx.x];
-      bsum += s;
+    dsum += dy2[(ti + 1) * kHY + tj + 1 + lane].x;  // zero outside the domain
+
+    // dW3: two k-steps of 16 cells.
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      uint32_t af[2][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(dyp + aoff[e] + ks * 16);
+        af[e >> 1][e & 1] = aoff[e] >= 0 ? p[0] : 0u;
+        af[e >> 1][(e & 1) + 2] = aoff[e] >= 0 ? p[4] : 0u;
+      }
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        uint32_t r[4];
+        const int cell = ti * kTY + tj + ks * 16 + (mi & 1) * 8 + rr;
+        ldsm_x4_t(r, as + cell * kCS + (2 * np + (mi >> 1)) * 8);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          mma_bf16(acc[mt][2 * np], af[mt], r[0], r[1]);
+          mma_bf16(acc[mt][2 * np + 1], af[mt], r[2], r[3]);
+        }
+      }
     }
   }
 
-  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS;
+  // Warp sums into shared memory, then the warps in order.
+  cp_async_wait<0>();
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(smem_raw) + warp * kB3Sums;
 #pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int k = threadIdx.x + 256 * e;
-    if (k <= 9 * C) row[LBM_CLOSURE_OFF_W3 + k] = wacc[e];  // k == 288 is b3
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = mt * 16 + gq + 8 * (e >> 1);
+        if (m < 27) sums[m * C + nt * 8 + 2 * tq + (e & 1)] = acc[mt][nt][e];
+      }
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    float v = bsum[k];
+#pragma unroll
+    for (int o = 2; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lc == 0) sums[27 * C + 8 * (k >> 2) + 4 * g2 + (k & 3)] = v;
   }
-  if (threadIdx.x < C) row[LBM_CLOSURE_OFF_B2 + threadIdx.x] = bsum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+  if (lane == 0) sums[28 * C] = dsum;
+  __syncthreads();
+  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS;
+  const float* all = reinterpret_cast<const float*>(smem_raw);
+  for (int k = threadIdx.x; k < 10 * C + 1; k += blockDim.x) {
+    float v = 0.0f;
+    for (int w = 0; w < kB3Threads / 32; ++w) {
+      const float* sw = all + w * kB3Sums;
+      if (k < 9 * C)
+        v += sw[18 * C + k] + sw[9 * C + k] + sw[k];  // smallest part first
+      else
+        v += sw[18 * C + k];  // db2, then db3
+    }
+    if (k < 9 * C)
+      row[LBM_CLOSURE_OFF_W3 + k] = v;
+    else if (k < 10 * C)
+      row[LBM_CLOSURE_OFF_B2 + k - 9 * C] = v;
+    else
+      row[LBM_CLOSURE_OFF_B3] = v;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Layer-1 weight gradient, CUDA cores: dW1[co][tap][ci] = sum_p dz1[p][co] x[p + tap][ci].
-// Thread (co, tap) owns the 4 input channels.
+// Layer-1 weight gradient on tensor cores: dW1[co][tap][ci] = sum_p dz1[p][co] x[p + tap][ci].
+// M = 32 output channels (2 m-tiles), N = 36 (tap, ci) columns (5 n-tiles, the last half empty),
+// K = cells. dz1 comes through ldmatrix; the features lie in shared memory as one plane a channel,
+// twice (the second copy shifted by one cell), so that two consecutive cells of any tap are one
+// aligned 32-bit word. Bound by reading dz1 and x. Batch 8 x 1024 x 512: 870 -> 93 us.
 
-__global__ void __launch_bounds__(288)
+constexpr int kW1Threads = 256;
+constexpr int kXS = kHY + 2;  // BF16 elements of a row of a feature plane
+constexpr size_t kW1Stage0 = (size_t)kTX * kTY * kCS * 2;  // dz1 of a tile
+constexpr size_t kW1OffX = 2 * kW1Stage0;
+constexpr size_t kW1Stage = kW1OffX + (size_t)4 * 2 * kHX * kXS * 2;
+constexpr size_t kW1Smem = (size_t)(kW1Threads / 32) * 36 * C * 4 > kW1Stage
+                               ? (size_t)(kW1Threads / 32) * 36 * C * 4
+                               : kW1Stage;
+
+__global__ void __launch_bounds__(kW1Threads, 3)
     conv1_wgrad_kernel(Grid g, const bf16* __restrict__ x, const bf16* __restrict__ dz1,
                        float* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* dzs = reinterpret_cast<bf16*>(smem_raw);  // [kTX * kTY][kCS]
-  __shared__ __align__(16) bf16 xs[kHX * kHY * 4];
-  const int co = threadIdx.x / 9, tap = threadIdx.x % 9;
-  const int dx = tap / 3 - 1, dy = tap % 3 - 1;
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
-    int64_t b, x0, y0;
-    g.tile(t, b, x0, y0);
-    __syncthreads();
-    load_cells32<kTX, kTY>(dz1, g, b, x0, y0, dzs);
-    load_cells4(x, g, b, x0, y0, xs);
-    __syncthreads();
-    for (int p = 0; p < kTX * kTY; ++p) {
-      const int pi = p / kTY, pj = p % kTY;
-      const float d = bf(dzs[p * kCS + co]);
-      const uint2 v = *reinterpret_cast<const uint2*>(xs + ((pi + 1 + dx) * kHY + pj + 1 + dy) * 4);
-      acc[0] = fmaf(d, __uint_as_float(v.x << 16), acc[0]);
-      acc[1] = fmaf(d, __uint_as_float(v.x & 0xffff0000u), acc[1]);
-      acc[2] = fmaf(d, __uint_as_float(v.y << 16), acc[2]);
-      acc[3] = fmaf(d, __uint_as_float(v.y & 0xffff0000u), acc[3]);
+  bf16* xp = reinterpret_cast<bf16*>(smem_raw + kW1OffX);  // [ci][shift][kHX][kXS]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gq = lane >> 2, tq = lane & 3, mi = lane >> 3, rr = lane & 7;
+  const int ti = warp >> 1, tj = (warp & 1) * 32;
+  // B fragments: column n = gq of n-tile nt is (tap, ci) = (n / 4, n % 4) of 8 nt + gq.
+  int boff[5];
+#pragma unroll
+  for (int nt = 0; nt < 5; ++nt) {
+    const int n = nt * 8 + gq, tap = n >> 2, ci = n & 3;
+    boff[nt] = -1;
+    if (tap < 9) {
+      const int col = tj + 1 + tap % 3 - 1, r = ti + 1 + tap / 3 - 1, odd = col & 1;
+      boff[nt] = ((ci * 2 + odd) * kHX + r) * kXS + col - odd + 2 * tq;
     }
   }
-  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W1;
+  float acc[2][5][4];
 #pragma unroll
-  for (int ci = 0; ci < 4; ++ci) row[co * 36 + tap * 4 + ci] = acc[ci];
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 5; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[mt][nt][e] = 0.0f;
+  for (int i = threadIdx.x; i < 4 * 2 * kHX * kXS; i += blockDim.x) xp[i] = to_bf(0.0f);
+  // The next tile's operands are in flight while this one is multiplied.
+  FeatureTile<kW1Threads> in;
+  auto fetch = [&](int64_t t, int s) {
+    int64_t b, x0, y0;
+    g.tile(t, b, x0, y0);
+    load_cells32_async<kTX, kTY>(dz1, g, b, x0, y0,
+                                 reinterpret_cast<bf16*>(smem_raw + (size_t)s * kW1Stage0));
+    in.load(x, g, t);
+  };
+  int stage = 0;
+  if ((int64_t)blockIdx.x < g.tiles) fetch(blockIdx.x, 0);
+  cp_async_commit();
+  for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, stage ^= 1) {
+    __syncthreads();  // the previous tile is done with the planes and its stage
+    in.each([&](int i, uint2 v) {
+      const int r = i / kHY, c = i - r * kHY;
+      const uint32_t h[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
+#pragma unroll
+      for (int ci = 0; ci < 4; ++ci) {
+        const bf16 e = __ushort_as_bfloat16((unsigned short)h[ci]);
+        xp[((ci * 2) * kHX + r) * kXS + c] = e;
+        if (c > 0) xp[((ci * 2 + 1) * kHX + r) * kXS + c - 1] = e;
+      }
+    });
+    if (t + gridDim.x < g.tiles) fetch(t + gridDim.x, stage ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    const bf16* dzs = reinterpret_cast<const bf16*>(smem_raw + (size_t)stage * kW1Stage0);
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      uint32_t af[2][4];
+      const int cell = ti * kTY + tj + ks * 16 + (mi >> 1) * 8 + rr;
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) ldsm_x4_t(af[mt], dzs + cell * kCS + mt * 16 + (mi & 1) * 8);
+#pragma unroll
+      for (int nt = 0; nt < 5; ++nt) {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(xp + boff[nt] + ks * 16);
+        const uint32_t b0 = boff[nt] >= 0 ? p[0] : 0u, b1 = boff[nt] >= 0 ? p[4] : 0u;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) mma_bf16(acc[mt][nt], af[mt], b0, b1);
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(smem_raw);  // [warp][co][36]
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 5; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int co = mt * 16 + gq + 8 * (e >> 1), n = nt * 8 + 2 * tq + (e & 1);
+        if (n < 36) sums[(warp * C + co) * 36 + n] = acc[mt][nt][e];
+      }
+  __syncthreads();
+  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W1;
+  for (int i = threadIdx.x; i < 36 * C; i += blockDim.x) {
+    float v = 0.0f;
+    for (int w = 0; w < kW1Threads / 32; ++w) v += sums[w * 36 * C + i];
+    row[i] = v;
+  }
 }
 
-// Column sums of the partial rows, in row order (double accumulation).
-__global__ void reduce_rows_kernel(const float* __restrict__ partial, int rows,
-                                   float* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= LBM_CLOSURE_PARAMS) return;
-  double s = 0.0;
-  for (int r = 0; r < rows; ++r) s += partial[(int64_t)r * LBM_CLOSURE_PARAMS + j];
-  out[j] = (float)s;
+// Column sums of the partial rows (double accumulation in a fixed order); the layer-2 weight
+// gradient has rows_w2 of them, the rest `rows`. Eight threads a column, so that the rows are read
+// by enough of the chip.
+__global__ void __launch_bounds__(256)
+    reduce_rows_kernel(const float* __restrict__ partial, int rows, int rows_w2,
+                       float* __restrict__ out) {
+  __shared__ double s[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + tx;
+  double v = 0.0;
+  if (j < LBM_CLOSURE_PARAMS) {
+    const bool w2 = j >= LBM_CLOSURE_OFF_W2 && j < LBM_CLOSURE_OFF_W2 + C * 288;
+    const int n = w2 ? rows_w2 : rows;
+    for (int r = ty; r < n; r += 8) v += partial[(int64_t)r * LBM_CLOSURE_PARAMS + j];
+  }
+  s[ty][tx] = v;
+  __syncthreads();
+  if (ty == 0 && j < LBM_CLOSURE_PARAMS) {
+    for (int k = 1; k < 8; ++k) v += s[k][tx];
+    out[j] = (float)v;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
 // Loss
 
-__global__ void count_kernel(const int32_t* __restrict__ flags, int64_t n,
-                             unsigned long long* __restrict__ count) {
+// Fluid cells, as kCountBlocks partial counts (one block alone took 77 us on 1024 x 512).
+constexpr int kCountBlocks = 32;
+
+__global__ void __launch_bounds__(1024)
+    count_kernel(const int32_t* __restrict__ flags, int64_t n,
+                 unsigned long long* __restrict__ counts) {
   __shared__ unsigned long long s[32];
   unsigned long long c = 0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) c += fluid_cell(flags[i]) ? 1 : 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    c += fluid_cell(flags[i]) ? 1 : 0;
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long t = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
-    *count = t;
+    counts[blockIdx.x] = t;
   }
 }
 
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ target,
-                            const int32_t* __restrict__ flags, int64_t n, int64_t batch,
-                            const unsigned long long* __restrict__ count, float* __restrict__ dy,
-                            double* __restrict__ partial) {
+__device__ __forceinline__ double total_count(const unsigned long long* counts, int64_t batch) {
+  unsigned long long c = 0;
+  for (int k = 0; k < kCountBlocks; ++k) c += counts[k];
+  return (double)c * (double)batch;
+}
+
+// Each thread takes a cell through the whole batch: its flag is read once, and no index needs a
+// division.
+__global__ void __launch_bounds__(256)
+    loss_kernel(const float* __restrict__ y, const float* __restrict__ target,
+                const int32_t* __restrict__ flags, int64_t n, int64_t batch,
+                const unsigned long long* __restrict__ counts, float* __restrict__ dy,
+                double* __restrict__ partial) {
   __shared__ double s[32];
-  const double total = (double)(*count) * (double)batch;
+  const double total = total_count(counts, batch);
   const float scale = total > 0 ? (float)(2.0 / total) : 0.0f;
   double acc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * batch;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const bool m = fluid_cell(flags[i % n]);
-    const float d = y[i] - target[i];
-    dy[i] = m ? scale * d : 0.0f;
-    if (m) acc += (double)d * (double)d;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    const bool m = fluid_cell(flags[c]);
+#pragma unroll 4
+    for (int64_t b = 0; b < batch; ++b) {
+      const int64_t i = b * n + c;
+      const float d = y[i] - target[i];
+      dy[i] = m ? scale * d : 0.0f;
+      if (m) acc += (double)d * (double)d;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
@@ -787,13 +1217,18 @@ __global__ void loss_kernel(const float* __restrict__ y, const float* __restrict
   }
 }
 
-__global__ void loss_final_kernel(const double* __restrict__ partial, int blocks,
-                                  const unsigned long long* __restrict__ count, int64_t batch,
-                                  double* __restrict__ loss) {
+// One warp: the partial sums by lanes, then across them (a fixed order).
+__global__ void __launch_bounds__(32)
+    loss_final_kernel(const double* __restrict__ partial, int blocks,
+                      const unsigned long long* __restrict__ counts, int64_t batch,
+                      double* __restrict__ loss) {
   double t = 0.0;
-  for (int i = 0; i < blocks; ++i) t += partial[i];
-  const double total = (double)(*count) * (double)batch;
-  *loss = total > 0 ? t / total : 0.0;
+  for (int i = threadIdx.x; i < blocks; i += 32) t += partial[i];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) {
+    const double total = total_count(counts, batch);
+    *loss = total > 0 ? t / total : 0.0;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1281,6 +1716,8 @@ constexpr size_t kTOffW = (size_t)4 * kTPad * 16;
 constexpr size_t kTOffBias = kTOffW + (size_t)36 * C * 16;
 constexpr size_t kTOffBar = kTOffBias + (size_t)C * 4;  // MMA mbarrier, load mbarrier, TMEM addr
 constexpr size_t kTSmem = kTOffBar + 24;
+constexpr int kTStageBytes = 2 * 32 * 128;  // a warp's rows in the epilogue
+static_assert((size_t)(kTThreads / 32) * kTStageBytes <= kTOffW, "the epilogue's rows must fit");
 constexpr unsigned kTLoadBytes = 4u * kTRegR * kTRegC * 16;  // the four plane boxes of a tile
 static_assert((size_t)kTThreads * (C + 1) * 4 <= kTOffW, "bias partial sums must fit the region");
 static_assert(kTBlocks * 32 <= kTTmemCols, "accumulators exceed the TMEM allocation");
@@ -1341,11 +1778,8 @@ __global__ void __launch_bounds__(kTThreads, 2)
     }
   }
   if (!BWD && threadIdx.x < C) bs[threadIdx.x] = bias[threadIdx.x];
-  // Plane cells past the region feed only discarded rows; keep them finite.
-  for (int i = threadIdx.x; i < 4 * kTPad; i += blockDim.x)
-    if (i % kTPad >= kTRegR * kTRegC)
-      *reinterpret_cast<uint4*>(ac + (size_t)i * 16) = make_uint4(0, 0, 0, 0);
-  // The weights and the zeroed plane tails, written here, are read by the MMAs (async proxy).
+  // (Plane cells past the region, whatever they hold, feed only discarded rows.)
+  // The weights, written here, are read by the MMAs (async proxy).
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (threadIdx.x == 0) {
     cl_mbar_init(mma_done, 1);
@@ -1424,55 +1858,112 @@ __global__ void __launch_bounds__(kTThreads, 2)
     }
     tc_fence_after();
     // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition) of blocks
-    // w / 4, w / 4 + 2, ...; one thread per cell, its 32 channels in registers.
-    for (int m = warp >> 2; m < kTBlocks; m += kWarps / 4) {
-      const int sp = warp & 3;
-      uint32_t r32[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
+    // w / 4, w / 4 + 2, ...; one thread per cell, its 32 channels in registers. Rows of cells pass
+    // through shared memory (the region's, whose operands the MMAs have read), so that global
+    // accesses are whole 128-byte lines: a lane's own row of 128 bytes at a time is a quarter of
+    // that. Chunk c of the row of lane l lies at chunk c ^ (l % 8).
+    const int sp = warp & 3;
+    unsigned char* own = ac + warp * kTStageBytes;  // this warp's: two slots of 32 rows x 128 bytes
+    auto cell_of = [&](int m, int64_t& cell) {      // block m's cell of this lane, if it has one
       const int q = kTFirst + 128 * m + 32 * sp + lane;  // region index of this row
       const int r = q / kTRegC - 1, c = q % kTRegC - 1;   // output tile coordinates
-      if (r < 0 || r >= kTR || c < 0 || c >= kTC) continue;
       const int64_t x = x0 + r, y = y0 + c;
-      if (x >= g.nx || y >= g.ny) continue;
-      const int64_t cell = g.cell(b, x, y);
+      const bool ok = r >= 0 && r < kTR && c >= 0 && c < kTC && x < g.nx && y < g.ny;
+      cell = ok ? g.cell(b, x, y) : -1;
+      return ok;
+    };
+    auto fetch_z = [&](int m, int slot) {  // BWD: block m's rows of z1 into a slot
+      int64_t cell;
+      cell_of(m, cell);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int l = 4 * k + (lane >> 3), ch = lane & 7;
+        const int64_t cl = __shfl_sync(0xffffffffu, cell, l);
+        cp_async16(own + slot * 4096 + l * 128 + ((ch ^ (l & 7)) * 16),
+                   cl >= 0 ? zin + cl * C + ch * 4 : zin, cl >= 0);
+      }
+      cp_async_commit();
+    };
+    constexpr int kStep = kWarps / 4;
+    if (BWD) fetch_z(warp >> 2, 0);
+    int slot = 0;
+    for (int m = warp >> 2; m < kTBlocks; m += kStep) {
+      if (BWD) {
+        if (m + kStep < kTBlocks) {
+          fetch_z(m + kStep, slot ^ 1);
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
+        }
+        __syncwarp();
+      }
+      uint32_t r32[32];
+      tmem_ld32(tmem + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
+      int64_t cell;
+      const bool valid = cell_of(m, cell);
+      unsigned char* buf = own + slot * 4096;
+      uint4* mine = reinterpret_cast<uint4*>(buf + lane * 128);
       uint32_t packed[C / 2];
       if (!BWD) {
-        float z[C];
-#pragma unroll
-        for (int ch = 0; ch < C; ++ch) z[ch] = __uint_as_float(r32[ch]) + bs[ch];
-        if (zout != nullptr) {
-          float4* zp = reinterpret_cast<float4*>(zout + cell * C);
-#pragma unroll
-          for (int k = 0; k < C / 4; ++k)
-            zp[k] = make_float4(z[4 * k], z[4 * k + 1], z[4 * k + 2], z[4 * k + 3]);
-        }
-#pragma unroll
-        for (int ch = 0; ch < C; ch += 2)
-          packed[ch / 2] = (uint32_t)__bfloat16_as_ushort(to_bf(gelu(z[ch]))) |
-                           ((uint32_t)__bfloat16_as_ushort(to_bf(gelu(z[ch + 1]))) << 16);
-      } else {
-        const float4* zp = reinterpret_cast<const float4*>(zin + cell * C);
 #pragma unroll
         for (int k = 0; k < C / 4; ++k) {
-          const float4 zz = zp[k];
-          const float zv[4] = {zz.x, zz.y, zz.z, zz.w};
+          float z[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) z[e] = __uint_as_float(r32[4 * k + e]) + bs[4 * k + e];
+          if (zout != nullptr)
+            mine[k ^ (lane & 7)] = make_uint4(__float_as_uint(z[0]), __float_as_uint(z[1]),
+                                              __float_as_uint(z[2]), __float_as_uint(z[3]));
+          packed[2 * k] = pack_bf2(gelu2(make_float2(z[0], z[1])));
+          packed[2 * k + 1] = pack_bf2(gelu2(make_float2(z[2], z[3])));
+        }
+        if (zout != nullptr) {
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int l = 4 * k + (lane >> 3), ch = lane & 7;
+            const int64_t cl = __shfl_sync(0xffffffffu, cell, l);
+            const uint4 v = *reinterpret_cast<const uint4*>(buf + l * 128 + ((ch ^ (l & 7)) * 16));
+            if (cl >= 0) reinterpret_cast<uint4*>(zout + cl * C)[ch] = v;
+          }
+          __syncwarp();
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < C / 4; ++k) {
+          const uint4 zz = mine[k ^ (lane & 7)];
+          const float zv[4] = {__uint_as_float(zz.x), __uint_as_float(zz.y), __uint_as_float(zz.z),
+                               __uint_as_float(zz.w)};
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
             const int ch = 4 * k + e;
-            const bf16 o0 = to_bf(__uint_as_float(r32[ch]) * gelu_grad(zv[e]));
-            const bf16 o1 = to_bf(__uint_as_float(r32[ch + 1]) * gelu_grad(zv[e + 1]));
-            bias_sum[ch] += bf(o0);
-            bias_sum[ch + 1] += bf(o1);
-            packed[ch / 2] =
-                (uint32_t)__bfloat16_as_ushort(o0) | ((uint32_t)__bfloat16_as_ushort(o1) << 16);
+            packed[ch / 2] = pack_bf2(__uint_as_float(r32[ch]) * gelu_grad(zv[e]),
+                                      __uint_as_float(r32[ch + 1]) * gelu_grad(zv[e + 1]));
+            if (valid) {
+              bias_sum[ch] += bf_lo(packed[ch / 2]);
+              bias_sum[ch + 1] += bf_hi(packed[ch / 2]);
+            }
           }
         }
+        __syncwarp();
       }
-      uint4* op = reinterpret_cast<uint4*>(out + cell * C);
+      // BF16 rows of 64 bytes, eight cells an access.
+      const int swz = (lane >> 1) & 3;
 #pragma unroll
       for (int k = 0; k < C / 8; ++k)
-        op[k] = make_uint4(packed[4 * k], packed[4 * k + 1], packed[4 * k + 2], packed[4 * k + 3]);
+        reinterpret_cast<uint4*>(buf + lane * 64)[k ^ swz] =
+            make_uint4(packed[4 * k], packed[4 * k + 1], packed[4 * k + 2], packed[4 * k + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int l = 8 * k + (lane >> 2), ch = lane & 3;
+        const int64_t cl = __shfl_sync(0xffffffffu, cell, l);
+        const uint4 v = *reinterpret_cast<const uint4*>(buf + l * 64 + ((ch ^ ((l >> 1) & 3)) * 16));
+        if (cl >= 0) reinterpret_cast<uint4*>(out + cl * C)[ch] = v;
+      }
+      __syncwarp();
+      slot ^= 1;
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next tile's copies
     tc_fence_before();
     __syncthreads();  // the region and every TMEM column are free for the next tile
   }
@@ -1532,11 +2023,7 @@ bool tc_input_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, in
 }
 
 // Tiles of kTR x kTC cells for conv32_tc_kernel.
-Grid tc_grid(int64_t nx, int64_t ny, int64_t batch) {
-  Grid g{nx, ny, batch, (nx + kTR - 1) / kTR, (ny + kTC - 1) / kTC, 0};
-  g.tiles = g.tx * g.ty * batch;
-  return g;
-}
+Grid tc_grid(int64_t nx, int64_t ny, int64_t batch) { return tiles_of(nx, ny, batch, kTR, kTC); }
 
 // Which kernel runs layer 2 of the training path (lbm_closure_set_layer2_kernel).
 int g_layer2_kernel = LBM_CLOSURE_LAYER2_TCGEN05;
@@ -1631,10 +2118,11 @@ int set_smem(const void* fn, size_t bytes) {
   return LBM_OK;
 }
 
-// Workspace: [count (8 B, padded to 256)][loss partials (kLossBlocks doubles, padded)]
+// Workspace: [kCountBlocks counts (256 B)][loss partials (kLossBlocks doubles, padded)]
 //            [dz2 BF16 [cells][32]][dz1 BF16 [cells][32]][partial rows FP32 [kPartialRows][P]]
 constexpr int64_t kWsCount = 0;
 constexpr int64_t kWsLoss = 256;
+static_assert(kCountBlocks * 8 <= kWsLoss, "the counts must fit");
 constexpr int64_t kWsDz = kWsLoss + ((kLossBlocks * 8 + 255) / 256) * 256;
 
 int64_t round256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -1704,8 +2192,8 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
   const cudaStream_t s = (cudaStream_t)stream;
   const int sms = device_sms();
   const auto* wb = reinterpret_cast<const bf16*>(params_bf16);
-  const int grid_small = (int)std::min<int64_t>(g.tiles, (int64_t)sms * 4);
-  conv1_fwd_kernel<<<grid_small, 256, 0, s>>>(g, reinterpret_cast<const bf16*>(x),
+  const int grid1 = (int)std::min<int64_t>(g.tiles, (int64_t)sms * kC1PerSm);
+  conv1_fwd_kernel<<<grid1, kC1Threads, 0, s>>>(g, reinterpret_cast<const bf16*>(x),
                                               wb + LBM_CLOSURE_OFF_W1, params + LBM_CLOSURE_OFF_B1,
                                               z1, reinterpret_cast<bf16*>(a1));
   CL_CUDA(cudaGetLastError());
@@ -1723,9 +2211,11 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
         params + LBM_CLOSURE_OFF_B2, nullptr, z2, reinterpret_cast<bf16*>(a2), nullptr);
   }
   CL_CUDA(cudaGetLastError());
-  conv3_fwd_kernel<<<grid_small, 256, kConv3Smem, s>>>(g, reinterpret_cast<const bf16*>(a2),
-                                                       wb + LBM_CLOSURE_OFF_W3,
-                                                       params + LBM_CLOSURE_OFF_B3, y);
+  const Grid g3 = tiles_of(nx, ny, batch, kC3R, kTY);
+  const int grid3 = (int)std::min<int64_t>(g3.tiles, (int64_t)sms * 2);
+  conv3_fwd_kernel<<<grid3, kC3Threads, kConv3Smem, s>>>(g3, reinterpret_cast<const bf16*>(a2),
+                                                         wb + LBM_CLOSURE_OFF_W3,
+                                                         params + LBM_CLOSURE_OFF_B3, y);
   CL_CUDA(cudaGetLastError());
   return LBM_OK;
 }
@@ -1746,11 +2236,11 @@ int lbm_closure_loss(const float* y, const float* target, const int32_t* flags, 
   auto* count = reinterpret_cast<unsigned long long*>(base + kWsCount);
   auto* partial = reinterpret_cast<double*>(base + kWsLoss);
   const int64_t n = nx * ny;
-  count_kernel<<<1, 1024, 0, s>>>(flags, n, count);
+  count_kernel<<<kCountBlocks, 1024, 0, s>>>(flags, n, count);
   CL_CUDA(cudaGetLastError());
   loss_kernel<<<kLossBlocks, 256, 0, s>>>(y, target, flags, n, batch, count, dy, partial);
   CL_CUDA(cudaGetLastError());
-  loss_final_kernel<<<1, 1, 0, s>>>(partial, kLossBlocks, count, batch, loss);
+  loss_final_kernel<<<1, 32, 0, s>>>(partial, kLossBlocks, count, batch, loss);
   CL_CUDA(cudaGetLastError());
   return LBM_OK;
 }
@@ -1772,6 +2262,7 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
     if (int rc = set_smem((const void*)conv32_tc_kernel<true>, kTSmem)) return rc;
     if (int rc = set_smem((const void*)conv32_wgrad_kernel, kDw2Smem)) return rc;
     if (int rc = set_smem((const void*)conv3_bwd_kernel, kConv3BwdSmem)) return rc;
+    if (int rc = set_smem((const void*)conv1_wgrad_kernel, kW1Smem)) return rc;
     configured = true;
   }
   const Grid g = make_grid(nx, ny, batch);
@@ -1783,11 +2274,12 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   auto* partial = reinterpret_cast<float*>(base + kWsDz + 2 * dzb);
   const auto* wb = reinterpret_cast<const bf16*>(params_bf16);
   const int rows = (int)std::min<int64_t>(g.tiles, kPartialRows);
+  const int rows_w2 = (int)std::min<int64_t>(rows, device_sms());
 
-  conv3_bwd_kernel<<<rows, 256, kConv3BwdSmem, s>>>(g, reinterpret_cast<const bf16*>(a2), z2,
+  conv3_bwd_kernel<<<rows, kB3Threads, kConv3BwdSmem, s>>>(g, reinterpret_cast<const bf16*>(a2), z2,
                                                     wb + LBM_CLOSURE_OFF_W3, dy, dz2, partial);
   CL_CUDA(cudaGetLastError());
-  conv32_wgrad_kernel<<<rows, kDw2Threads, kDw2Smem, s>>>(g, reinterpret_cast<const bf16*>(a1),
+  conv32_wgrad_kernel<<<rows_w2, kDw2Threads, kDw2Smem, s>>>(g, reinterpret_cast<const bf16*>(a1),
                                                           dz2, partial);
   CL_CUDA(cudaGetLastError());
   CUtensorMap dz2_map;
@@ -1802,10 +2294,10 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
         g, dz2, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1, partial);
   }
   CL_CUDA(cudaGetLastError());
-  conv1_wgrad_kernel<<<rows, 288, kTX * kTY * kCS * sizeof(bf16), s>>>(
+  conv1_wgrad_kernel<<<rows, kW1Threads, kW1Smem, s>>>(
       g, reinterpret_cast<const bf16*>(x), dz1, partial);
   CL_CUDA(cudaGetLastError());
-  reduce_rows_kernel<<<blocks_for(LBM_CLOSURE_PARAMS, 256), 256, 0, s>>>(partial, rows, grad);
+  reduce_rows_kernel<<<blocks_for(LBM_CLOSURE_PARAMS, 32), 256, 0, s>>>(partial, rows, rows_w2, grad);
   CL_CUDA(cudaGetLastError());
   return LBM_OK;
 }
