@@ -36,8 +36,8 @@ NVCC_FLAGS = [
     f"-I{INCLUDE}",
 ]
 
-CUDA_SOURCES = ["aa_d2q9.cu", "aa_d3q27.cu", "fields.cu", "capi.cu", "noalloc.cu", "ensemble.cu", "closure.cu"]
-HEADERS = ["aa_step.cuh", "aa_tma.cuh", "aa_pair.cuh", "aa_launch.cuh", "lattice.cuh",
+CUDA_SOURCES = ["aa_d2q9.cu", "aa_d3q27.cu", "aa_resident.cu", "fields.cu", "capi.cu", "noalloc.cu", "ensemble.cu", "closure.cu"]
+HEADERS = ["aa_step.cuh", "aa_tma.cuh", "aa_pair.cuh", "aa_resident.cuh", "aa_launch.cuh", "lattice.cuh",
            "storage.cuh", "sim.h"]
 
 

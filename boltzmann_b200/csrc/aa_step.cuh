@@ -50,7 +50,7 @@ struct TracerArgs {
 struct FastDiv {
   unsigned d = 1, mul = 1, sh1 = 0, sh2 = 0;
   FastDiv() = default;
-  explicit FastDiv(unsigned divisor) : d(divisor) {
+  __host__ __device__ explicit FastDiv(unsigned divisor) : d(divisor) {
     unsigned l = 0;
     while (l < 32 && (1ull << l) < d) ++l;
     mul = (unsigned)((((1ull << l) - d) << 32) / d) + 1;

@@ -86,6 +86,8 @@ int download_reals(lbm_sim* s, float* dst, const void* src, int64_t count) {
   return LBM_OK;
 }
 
+size_t pad256(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
 // Reads the device status word after a synchronisation: bit 1 means a kernel gave up waiting for
 // its own asynchronous copies (it then stopped early and the state is not valid).
 int check_status(lbm_sim* s) {
@@ -112,15 +114,8 @@ void drop_graph(lbm_sim* s) {
 
 void release(lbm_sim* s) {
   drop_graph(s);
-  for (lbm_sim::Tracer& t : s->tracers) {
-    cudaFree(t.g);
-    cudaFree(t.val);
-  }
-  cudaFree(s->f);
-  cudaFree(s->rho);
-  cudaFree(s->vel);
-  cudaFree(s->flags);
-  cudaFree(s->status);
+  for (lbm_sim::Tracer& t : s->tracers) cudaFree(t.g);
+  cudaFree(s->arena);
   if (s->stream) cudaStreamDestroy(s->stream);
 }
 
@@ -234,18 +229,23 @@ int lbm_create(int dim, const int64_t* counts, int q, int collision, float omega
   if (e != cudaSuccess) return bail(e, "cudaGetDevice");
   e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return bail(e, "cudaStreamCreate");
-  const size_t rb = s->real_bytes();
-  if ((e = cudaMalloc(&s->f, (size_t)n * q * lbm::pop_bytes(storage))) != cudaSuccess)
-    return bail(e, "cudaMalloc(f)");
-  if ((e = cudaMalloc(&s->rho, (size_t)n * rb)) != cudaSuccess) return bail(e, "cudaMalloc(rho)");
-  if ((e = cudaMalloc(&s->vel, (size_t)n * dim * rb)) != cudaSuccess)
-    return bail(e, "cudaMalloc(vel)");
-  // Flags are padded to whole 256-byte blocks: kernels read them as aligned 4-byte words.
-  const size_t flag_bytes = ((size_t)n + 255) / 256 * 256;
-  if ((e = cudaMalloc((void**)&s->flags, flag_bytes)) != cudaSuccess)
-    return bail(e, "cudaMalloc(flags)");
-  if ((e = cudaMalloc((void**)&s->status, 64 * sizeof(double))) != cudaSuccess)
-    return bail(e, "cudaMalloc(status)");
+  // One allocation for everything: its parts start on 256 bytes. Flags are padded to whole 256-byte
+  // blocks: kernels read them as aligned 4-byte words.
+  const size_t rb = s->real_bytes(), mail = lbm::resident_mail_bytes(*s, 0);
+  const size_t flag_bytes = pad256((size_t)n), status_bytes = 64 * sizeof(double);
+  const size_t parts[] = {pad256((size_t)n * q * lbm::pop_bytes(storage)), pad256((size_t)n * rb),
+                          pad256((size_t)n * dim * rb), flag_bytes, pad256(status_bytes), mail};
+  size_t total = 0;
+  for (size_t b : parts) total += b;
+  if ((e = cudaMalloc(&s->arena, total)) != cudaSuccess) return bail(e, "cudaMalloc(fields)");
+  unsigned char* at = static_cast<unsigned char*>(s->arena);
+  s->f = at;
+  s->rho = at += parts[0];
+  s->vel = at += parts[1];
+  s->flags = at += parts[2];
+  s->status = reinterpret_cast<int*>(at += parts[3]);
+  at += parts[4];
+  if (mail) s->mail = at;
   s->sums = reinterpret_cast<double*>(s->status) + 1;  // 63 doubles after the status word
   s->sums_len = 63;
   // Reference defaults (src/fields.rs:75-77, src/simulation.rs:35): f = 0, rho = 1, vel = 0,
@@ -254,7 +254,7 @@ int lbm_create(int dim, const int64_t* counts, int q, int collision, float omega
       (e = lbm::fill_value(s->rho, n, 1.0, storage == LBM_STORAGE_F64, s->stream)) ||
       (e = cudaMemsetAsync(s->vel, 0, (size_t)n * dim * rb, s->stream)) ||
       (e = cudaMemsetAsync(s->flags, 0, flag_bytes, s->stream)) ||
-      (e = cudaMemsetAsync(s->status, 0, 64 * sizeof(double), s->stream)) ||
+      (e = cudaMemsetAsync(s->status, 0, pad256(status_bytes) + mail, s->stream)) ||
       (e = cudaStreamSynchronize(s->stream)))
     return bail(e, "initialise fields");
   *out = s;
@@ -304,15 +304,18 @@ int lbm_add_tracer(lbm_sim* sim, int q, int collision, float omega_pos, float om
   t.omega_neg = omega_neg;
   if (sim->tracer_storage >= 0 && !sim->tracers.empty())
     return fail(LBM_ERR_UNSUPPORTED, "16-bit tracer storage takes one tracer");
+  // One allocation for the populations, the values and, with a first tracer, the resident kernel's
+  // message words (which the simulation without one no longer uses).
   const size_t rb = sim->real_bytes(), gb = sim->tracer_pop_bytes();
-  LBM_CUDA(cudaMalloc(&t.g, (size_t)sim->n * q * gb));
-  cudaError_t e = cudaMalloc(&t.val, (size_t)sim->n * rb);
-  if (e != cudaSuccess) {
-    cudaFree(t.g);
-    return cuda_fail(e, "cudaMalloc(tracer val)");
-  }
-  LBM_CUDA(cudaMemsetAsync(t.g, 0, (size_t)sim->n * q * gb, sim->stream));
-  LBM_CUDA(cudaMemsetAsync(t.val, 0, (size_t)sim->n * rb, sim->stream));
+  const size_t pops = pad256((size_t)sim->n * q * gb), vals = pad256((size_t)sim->n * rb);
+  const size_t mail =
+      sim->tracers.empty() && tracer_kernel(sim->dim, q, collision) ? lbm::resident_mail_bytes(*sim, 1) : 0;
+  LBM_CUDA(cudaMalloc(&t.g, pops + vals + mail));
+  t.val = static_cast<unsigned char*>(t.g) + pops;
+  LBM_CUDA(cudaMemsetAsync(t.g, 0, pops + vals + mail, sim->stream));
+  sim->mail = mail ? static_cast<unsigned char*>(t.g) + pops + vals : nullptr;
+  sim->mail_tracers = 1;
+  sim->mail_seq = 1;
   sim->tracers.push_back(t);
   drop_graph(sim);
   if (out_index) *out_index = (int)sim->tracers.size() - 1;
@@ -467,6 +470,11 @@ int lbm_iterate(lbm_sim* sim, int64_t iters) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const bool outer = cudaStreamIsCapturing(sim->stream, &cs) == cudaSuccess &&
                      cs != cudaStreamCaptureStatusNone;
+  if (!outer) {
+    // (Not into a caller's graph: its replays would repeat the sequence numbers.)
+    const cudaError_t e = lbm::iterate_resident(*sim, iters);
+    if (e != cudaErrorNotSupported) return e == cudaSuccess ? LBM_OK : step_launch_fail(e);
+  }
   if (!outer && !sim->graph_failed && left >= kMinGraphPairs + 2) {
     if (!sim->graph_warm) {
       if (cudaError_t e = launch_pair(sim, false)) return step_launch_fail(e);

@@ -16,7 +16,7 @@ CSRC = Path(__file__).resolve().parent / "csrc"
 # The files each kernel family is compiled from (its own translation units and headers).
 GROUPS = {
     "stencil": ["aa_step.cuh", "aa_tma.cuh", "aa_pair.cuh", "aa_launch.cuh", "lattice.cuh",
-                "storage.cuh", "aa_d2q9.cu", "aa_d3q27.cu"],
+                "storage.cuh", "aa_d2q9.cu", "aa_d3q27.cu", "aa_resident.cuh", "aa_resident.cu"],
     "ensemble": ["ensemble.cu", "aa_step.cuh", "aa_tma.cuh", "aa_pair.cuh", "lattice.cuh",
                  "storage.cuh"],
     "closure": ["closure.cu"],
