@@ -32,9 +32,9 @@ bool layout(int ny, int nz, int gy, int gz, size_t limit, ResidentPlan& p) {
   ResidentArgs& d = p.args;
   d.gy = gy;
   d.gz = gz;
-  // The smaller tiles' frames: no larger (see frame_cells), down to one row or column less.
-  d.frame = std::max(std::max(frame_cells(h, w), frame_cells(h - 1, w)),
-                     std::max(frame_cells(h, w - 1), frame_cells(h - 1, w - 1)));
+  // Over the tiles of one row or column less, too (a thin one has no interior to leave out).
+  d.published = std::max(std::max(rim_cells(h, w), rim_cells(h - 1, w)),
+                         std::max(rim_cells(h, w - 1), rim_cells(h - 1, w - 1)));
   d.messages = resident_slots<K, NT>() * halo_entries(h, w);
   p.smem = ResidentStage<K, NT, KT>::off_table + (size_t)2 * d.messages * 8;
   // A thread per cell, or per message where those are more.
@@ -53,10 +53,12 @@ bool plan_for(lbm_sim& s, int sms, size_t limit, ResidentPlan& best) {
   if (s.n > (int64_t)sms * resident_stride<K, NT, KT>() || s.n >= (1 << 22)) return false;
   if (s.resident_key == NT)  // the search's result for this number of tracers
     return s.resident_gy > 0 && layout<K, NT, KT>(ny, nz, s.resident_gy, s.resident_gz, limit, best);
+  // Tiles of some 64 cells at least: smaller ones send more words than they update cells.
+  const int ctas = (int)std::min<int64_t>(sms, std::max<int64_t>(1, s.n / 64));
   double least = 0;
   bool found = false;
-  for (int gy = 1; gy <= std::min(ny, sms); ++gy)
-    for (int gz = 1; gz <= std::min(nz, sms / gy); ++gz) {
+  for (int gy = 1; gy <= std::min(ny, ctas); ++gy)
+    for (int gz = 1; gz <= std::min(nz, ctas / gy); ++gz) {
       const int h = (ny + gy - 1) / gy, w = (nz + gz - 1) / gz;
       const double cost = (double)h * w + 2.5 * (h + w);
       if (found && cost >= least) continue;
@@ -92,7 +94,7 @@ cudaError_t run(lbm_sim& s, const ResidentPlan& plan, int64_t steps) {
     ResidentArgs d = plan.args;
     d.steps = now;
     d.seq = s.mail_seq;
-    d.mail = static_cast<unsigned long long*>(s.mail);
+    for (int k = 0; k < 2; ++k) d.mail[k] = static_cast<unsigned long long*>(s.mail[k]);
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
@@ -127,14 +129,14 @@ template <int K, int NT, int KT>
 size_t mail_bytes(lbm_sim& s) {
   ResidentPlan plan;
   if (!plan_here<K, NT, KT>(s, plan)) return 0;
-  return (size_t)2 * mail_words<typename Pop<K>::type>() * plan.args.gy * plan.args.gz *
-         resident_slots<K, NT>() * plan.args.frame * 8;
+  return (size_t)mail_words<typename Pop<K>::type>() * plan.args.gy * plan.args.gz *
+         resident_slots<K, NT>() * plan.args.published * 8;
 }
 
 template <int K, int NT, int KT>
 cudaError_t iterate(lbm_sim& s, int64_t steps) {
   ResidentPlan plan;
-  if (s.mail == nullptr || s.mail_tracers != NT || !plan_here<K, NT, KT>(s, plan))
+  if (s.mail[1] == nullptr || s.mail_tracers != NT || !plan_here<K, NT, KT>(s, plan))
     return cudaErrorNotSupported;
   return s.collision == 1 ? run<true, K, NT, KT>(s, plan, steps)
                           : run<false, K, NT, KT>(s, plan, steps);

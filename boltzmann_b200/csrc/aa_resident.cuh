@@ -62,10 +62,10 @@ __host__ __device__ constexpr int resident_stride() {
 struct ResidentArgs {
   int gy, gz;      // tiles along the two axes; CTA = ty * gz + tz
   int steps;       // even
-  int frame;       // published cells of a CTA at most
+  int published;   // cells a CTA publishes of a slot at most
   int messages;    // table entries for receiving (and for sending) at most
   unsigned seq;    // sequence number of the first pair
-  unsigned long long* mail;  // [2 sets][words][CTAs][slots][frame]
+  unsigned long long* mail[2];  // two sets of [words][CTAs][slots][published]
 };
 
 // Shared-memory layout of a variant (bytes).
@@ -103,17 +103,6 @@ __device__ __forceinline__ void fetch_pop(T* dst, const T* src) {
     *dst = *src;
 }
 
-// Published cells: those within two of the tile's edge, row by row.
-__host__ __device__ __forceinline__ int frame_cells(int h, int w) {
-  return h <= 4 ? h * w : 4 * w + (h - 4) * (w < 4 ? w : 4);
-}
-__host__ __device__ __forceinline__ int frame_index(int r, int c, int h, int w) {
-  if (h <= 4 || r < 2) return r * w + c;
-  if (r >= h - 2) return 2 * w + (r - (h - 2)) * w + c;
-  if (w < 4) return 4 * w + (r - 2) * w + c;
-  return 4 * w + (r - 2) * 4 + (c < 2 ? c : c - w + 4);
-}
-
 // Halo cells whose slot with velocity (cy, cz) is read by a cell of the tile or of the ring around
 // it: the (h + 2) x (w + 2) rectangle shifted against the velocity, without the tile. Their number
 // is the same for every slot; entry k of them.
@@ -149,20 +138,29 @@ __host__ __device__ __forceinline__ void rim_cell(int k, int h, int w, int& r, i
 
 // Cells of the tile whose slot with velocity (cy, cz) is read by a cell that some other tile updates
 // too (on the rim, or outside): the tile without its interior shifted against the velocity. As many
-// as rim_cells for every slot; entry k of them.
-__host__ __device__ __forceinline__ void tx_cell(int k, int cy, int cz, int h, int w, int& r, int& c) {
+// as rim_cells for every slot; entry k of them, and the entry of cell (r, c) that is one of them.
+__host__ __device__ __forceinline__ void published_cell(int k, int cy, int cz, int h, int w, int& r,
+                                                        int& c) {
   if (h <= 2 || w <= 2) {
     r = k / w;
     c = k - r * w;
-  } else if (k < 2 * w) {
+  } else if (k < 2 * w) {  // two rows
     const int j = k >= w;
     r = cy == 0 ? (j ? h - 1 : 0) : (cy > 0 ? h - 2 + j : j);
     c = k - j * w;
-  } else {
+  } else {  // two cells of every other row
     const int e = k - 2 * w, j = e & 1;
     r = (e >> 1) + 1 - cy;
     c = cz == 0 ? (j ? w - 1 : 0) : (cz > 0 ? w - 2 + j : j);
   }
+}
+__host__ __device__ __forceinline__ int published_index(int r, int c, int cy, int cz, int h, int w) {
+  if (h <= 2 || w <= 2) return r * w + c;
+  const int row = cy == 0 ? (r == 0 ? 0 : (r == h - 1 ? 1 : -1))
+                          : (cy > 0 ? r - (h - 2) : (r < 2 ? r : -1));
+  if (row >= 0) return row * w + c;
+  const int col = cz == 0 ? (c == 0 ? 0 : 1) : (cz > 0 ? c - (w - 2) : c);
+  return 2 * w + 2 * (r - 1 + cy) + col;
 }
 
 __device__ __forceinline__ void mail_put(unsigned long long* p, unsigned v, unsigned seq) {
@@ -284,9 +282,8 @@ __global__ void __launch_bounds__(resident_threads<K, NT>())
     const int s = e / rim_cells(h, w), k = e - s * rim_cells(h, w);
     int cy, cz, r, c;
     velocity(s, cy, cz);
-    tx_cell(k, cy, cz, h, w, r, c);
-    tx[e] = make_uint2(slot_at(s, region(r, c)),
-                       (unsigned)((blockIdx.x * NS + s) * d.frame + frame_index(r, c, h, w)));
+    published_cell(k, cy, cz, h, w, r, c);
+    tx[e] = make_uint2(slot_at(s, region(r, c)), (unsigned)((blockIdx.x * NS + s) * d.published + k));
   }
   for (int e = tid; e < nrx; e += nthreads) {
     const int s = e / halo_entries(h, w), k = e - s * halo_entries(h, w);
@@ -299,8 +296,8 @@ __global__ void __launch_bounds__(resident_threads<K, NT>())
     const int fy = tile_first(oy, d.gy, a.ny), fz = tile_first(oz, d.gz, a.nz);
     const int oh = tile_first(oy + 1, d.gy, a.ny) - fy, ow = tile_first(oz + 1, d.gz, a.nz) - fz;
     rx[e] = make_uint2(slot_at(s, region(r, c)),
-                       (unsigned)(((oy * d.gz + oz) * NS + s) * d.frame +
-                                  frame_index(y - fy, z - fz, oh, ow)));
+                       (unsigned)(((oy * d.gz + oz) * NS + s) * d.published +
+                                  published_index(y - fy, z - fz, cy, cz, oh, ow)));
   }
 
   // The tile into the region, and the flags of the tile and its ring (the other halo slots come as
@@ -382,10 +379,10 @@ __global__ void __launch_bounds__(resident_threads<K, NT>())
 
   StepArgs<Real> now = a;  // only the last step of a call writes moments
   unsigned seq = d.seq;
-  const size_t set_words = (size_t)gridDim.x * NS * d.frame;
+  const size_t set_words = (size_t)gridDim.x * NS * d.published;
   bool ok = true;
   for (int s = 0; s < d.steps; s += 2, ++seq) {
-    unsigned long long* box = d.mail + (size_t)(seq & 1u) * W * set_words;
+    unsigned long long* box = d.mail[seq & 1u];
     for (int e = tid; e < ntx; e += nthreads) {
       const uint2 m = tx[e];
       const bool value = NT == 1 && e >= (NS - 1) * rim_cells(h, w);

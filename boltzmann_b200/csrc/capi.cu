@@ -1,6 +1,7 @@
 // C ABI of include/lbm_cuda.h: simulation lifetime, transfers and the per-step launch loop.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -58,17 +59,15 @@ int check_tracer(lbm_sim* s, int t) {
   return LBM_OK;
 }
 
-// Host float -> device real (float, or double through a temporary for F64).
+// Host float -> device real (float; for F64 double through the simulation's scratch array, whose users
+// follow one another on the stream).
 int upload_reals(lbm_sim* s, void* dst, const float* src, int64_t count) {
   if (s->storage != LBM_STORAGE_F64) {
     LBM_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     return LBM_OK;
   }
-  float* tmp = nullptr;
-  LBM_CUDA(cudaMallocAsync((void**)&tmp, count * sizeof(float), s->stream));
-  LBM_CUDA(cudaMemcpyAsync(tmp, src, count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-  LBM_CUDA(lbm::widen_to_double(tmp, static_cast<double*>(dst), count, s->stream));
-  LBM_CUDA(cudaFreeAsync(tmp, s->stream));
+  LBM_CUDA(cudaMemcpyAsync(s->scratch, src, count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
+  LBM_CUDA(lbm::widen_to_double(static_cast<float*>(s->scratch), static_cast<double*>(dst), count, s->stream));
   return LBM_OK;
 }
 
@@ -78,15 +77,47 @@ int download_reals(lbm_sim* s, float* dst, const void* src, int64_t count) {
     LBM_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
     return LBM_OK;
   }
-  float* tmp = nullptr;
-  LBM_CUDA(cudaMallocAsync((void**)&tmp, count * sizeof(float), s->stream));
-  LBM_CUDA(lbm::narrow_to_float(static_cast<const double*>(src), tmp, count, s->stream));
-  LBM_CUDA(cudaMemcpyAsync(dst, tmp, count * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-  LBM_CUDA(cudaFreeAsync(tmp, s->stream));
+  LBM_CUDA(lbm::narrow_to_float(static_cast<const double*>(src), static_cast<float*>(s->scratch), count, s->stream));
+  LBM_CUDA(cudaMemcpyAsync(dst, s->scratch, count * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
   return LBM_OK;
 }
 
 size_t pad256(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// Device memory for several arrays (out[k]: bytes[k], null for 0). The driver carves allocations below
+// 512 KB out of blocks it has (about 1 us each) and maps new memory for larger ones (350 us and
+// more, and as much to free them), so these share one allocation.
+cudaError_t allocate(lbm_sim* s, const size_t* bytes, void** out, int count) {
+  constexpr size_t kSmall = 512 << 10;
+  const size_t had = s->owned.size();
+  size_t total = 0;
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < count && e == cudaSuccess; ++k) {
+    out[k] = nullptr;
+    if (bytes[k] >= kSmall) {
+      total += pad256(bytes[k]);
+    } else if (bytes[k] > 0) {
+      e = cudaMalloc(&out[k], bytes[k]);
+      if (e == cudaSuccess) s->owned.push_back(out[k]);
+    }
+  }
+  void* block = nullptr;
+  if (e == cudaSuccess && total > 0) {
+    e = cudaMalloc(&block, total);
+    if (e == cudaSuccess) s->owned.push_back(block);
+  }
+  if (e != cudaSuccess) {
+    for (; s->owned.size() > had; s->owned.pop_back()) cudaFree(s->owned.back());
+    return e;
+  }
+  auto* at = static_cast<unsigned char*>(block);
+  for (int k = 0; k < count; ++k)
+    if (bytes[k] >= kSmall) {
+      out[k] = at;
+      at += pad256(bytes[k]);
+    }
+  return cudaSuccess;
+}
 
 // Reads the device status word after a synchronisation: bit 1 means a kernel gave up waiting for
 // its own asynchronous copies (it then stopped early and the state is not valid).
@@ -114,8 +145,7 @@ void drop_graph(lbm_sim* s) {
 
 void release(lbm_sim* s) {
   drop_graph(s);
-  for (lbm_sim::Tracer& t : s->tracers) cudaFree(t.g);
-  cudaFree(s->arena);
+  for (void* p : s->owned) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
 }
 
@@ -229,23 +259,23 @@ int lbm_create(int dim, const int64_t* counts, int q, int collision, float omega
   if (e != cudaSuccess) return bail(e, "cudaGetDevice");
   e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return bail(e, "cudaStreamCreate");
-  // One allocation for everything: its parts start on 256 bytes. Flags are padded to whole 256-byte
-  // blocks: kernels read them as aligned 4-byte words.
+  // Flags are padded to whole 256-byte blocks: kernels read them as aligned 4-byte words.
   const size_t rb = s->real_bytes(), mail = lbm::resident_mail_bytes(*s, 0);
   const size_t flag_bytes = pad256((size_t)n), status_bytes = 64 * sizeof(double);
-  const size_t parts[] = {pad256((size_t)n * q * lbm::pop_bytes(storage)), pad256((size_t)n * rb),
-                          pad256((size_t)n * dim * rb), flag_bytes, pad256(status_bytes), mail};
-  size_t total = 0;
-  for (size_t b : parts) total += b;
-  if ((e = cudaMalloc(&s->arena, total)) != cudaSuccess) return bail(e, "cudaMalloc(fields)");
-  unsigned char* at = static_cast<unsigned char*>(s->arena);
-  s->f = at;
-  s->rho = at += parts[0];
-  s->vel = at += parts[1];
-  s->flags = at += parts[2];
-  s->status = reinterpret_cast<int*>(at += parts[3]);
-  at += parts[4];
-  if (mail) s->mail = at;
+  s->scratch_bytes = std::min((size_t)n * sizeof(int32_t), lbm::kFlagPiece);
+  if (rb == 8) s->scratch_bytes = std::max(s->scratch_bytes, (size_t)n * dim * sizeof(float));
+  const size_t bytes[] = {(size_t)n * q * lbm::pop_bytes(storage), (size_t)n * rb,
+                          (size_t)n * dim * rb, flag_bytes, status_bytes, s->scratch_bytes, mail, mail};
+  void* at[8];
+  if ((e = allocate(s, bytes, at, 8)) != cudaSuccess) return bail(e, "cudaMalloc(fields)");
+  s->f = at[0];
+  s->rho = at[1];
+  s->vel = at[2];
+  s->flags = static_cast<uint8_t*>(at[3]);
+  s->status = static_cast<int*>(at[4]);
+  s->scratch = at[5];
+  s->mail[0] = at[6];
+  s->mail[1] = at[7];
   s->sums = reinterpret_cast<double*>(s->status) + 1;  // 63 doubles after the status word
   s->sums_len = 63;
   // Reference defaults (src/fields.rs:75-77, src/simulation.rs:35): f = 0, rho = 1, vel = 0,
@@ -254,7 +284,9 @@ int lbm_create(int dim, const int64_t* counts, int q, int collision, float omega
       (e = lbm::fill_value(s->rho, n, 1.0, storage == LBM_STORAGE_F64, s->stream)) ||
       (e = cudaMemsetAsync(s->vel, 0, (size_t)n * dim * rb, s->stream)) ||
       (e = cudaMemsetAsync(s->flags, 0, flag_bytes, s->stream)) ||
-      (e = cudaMemsetAsync(s->status, 0, pad256(status_bytes) + mail, s->stream)) ||
+      (e = cudaMemsetAsync(s->status, 0, status_bytes, s->stream)) ||
+      (mail && (e = cudaMemsetAsync(s->mail[0], 0, mail, s->stream))) ||
+      (mail && (e = cudaMemsetAsync(s->mail[1], 0, mail, s->stream))) ||
       (e = cudaStreamSynchronize(s->stream)))
     return bail(e, "initialise fields");
   *out = s;
@@ -304,16 +336,22 @@ int lbm_add_tracer(lbm_sim* sim, int q, int collision, float omega_pos, float om
   t.omega_neg = omega_neg;
   if (sim->tracer_storage >= 0 && !sim->tracers.empty())
     return fail(LBM_ERR_UNSUPPORTED, "16-bit tracer storage takes one tracer");
-  // One allocation for the populations, the values and, with a first tracer, the resident kernel's
-  // message words (which the simulation without one no longer uses).
+  // With a first tracer new message words for the resident kernel, too (those of the simulation without
+  // one are no longer used).
   const size_t rb = sim->real_bytes(), gb = sim->tracer_pop_bytes();
-  const size_t pops = pad256((size_t)sim->n * q * gb), vals = pad256((size_t)sim->n * rb);
   const size_t mail =
       sim->tracers.empty() && tracer_kernel(sim->dim, q, collision) ? lbm::resident_mail_bytes(*sim, 1) : 0;
-  LBM_CUDA(cudaMalloc(&t.g, pops + vals + mail));
-  t.val = static_cast<unsigned char*>(t.g) + pops;
-  LBM_CUDA(cudaMemsetAsync(t.g, 0, pops + vals + mail, sim->stream));
-  sim->mail = mail ? static_cast<unsigned char*>(t.g) + pops + vals : nullptr;
+  const size_t bytes[] = {(size_t)sim->n * q * gb, (size_t)sim->n * rb, mail, mail};
+  void* at[4];
+  if (cudaError_t e = allocate(sim, bytes, at, 4)) return cuda_fail(e, "cudaMalloc(tracer)");
+  t.g = at[0];
+  t.val = at[1];
+  LBM_CUDA(cudaMemsetAsync(t.g, 0, bytes[0], sim->stream));
+  LBM_CUDA(cudaMemsetAsync(t.val, 0, bytes[1], sim->stream));
+  for (int k = 0; k < 2; ++k) {
+    sim->mail[k] = at[2 + k];
+    if (mail) LBM_CUDA(cudaMemsetAsync(at[2 + k], 0, mail, sim->stream));
+  }
   sim->mail_tracers = 1;
   sim->mail_seq = 1;
   sim->tracers.push_back(t);
@@ -367,13 +405,15 @@ int lbm_upload_flags(lbm_sim* sim, const int32_t* flags) {
   if (int rc = activate(sim)) return rc;
   if (flags == nullptr) return fail(LBM_ERR_ARGUMENT, "null flags");
   // Only bits 0-3 are read by the kernels (WALL, FIXED_FLUID_*, FIXED_SCALAR_VALUE): the int32
-  // array goes over as it is (one DMA from the caller's buffer) and is narrowed on the device.
-  int32_t* tmp = nullptr;
-  LBM_CUDA(cudaMallocAsync((void**)&tmp, (size_t)sim->n * sizeof(int32_t), sim->stream));
-  LBM_CUDA(cudaMemcpyAsync(tmp, flags, (size_t)sim->n * sizeof(int32_t), cudaMemcpyHostToDevice,
-                           sim->stream));
-  LBM_CUDA(lbm::flags_to_u8(tmp, static_cast<uint8_t*>(sim->flags), sim->n, sim->stream));
-  LBM_CUDA(cudaFreeAsync(tmp, sim->stream));
+  // array goes over as it is and is narrowed on the device, a piece of the scratch array at a time.
+  const int64_t piece = (int64_t)(sim->scratch_bytes / sizeof(int32_t));
+  for (int64_t at = 0; at < sim->n; at += piece) {
+    const int64_t count = std::min(piece, sim->n - at);
+    LBM_CUDA(cudaMemcpyAsync(sim->scratch, flags + at, (size_t)count * sizeof(int32_t),
+                             cudaMemcpyHostToDevice, sim->stream));
+    LBM_CUDA(lbm::flags_to_u8(static_cast<const int32_t*>(sim->scratch), sim->flags + at, count,
+                              sim->stream));
+  }
   LBM_CUDA(cudaStreamSynchronize(sim->stream));
   return LBM_OK;
 }
@@ -508,8 +548,7 @@ int lbm_download_fluid(lbm_sim* sim, float* rho, float* vel) {
   if (vel) {
     if (int rc = download_reals(sim, vel, sim->vel, sim->n * sim->dim)) return rc;
   }
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return check_status(sim);
+  return check_status(sim);  // waits for the stream
 }
 
 int lbm_download_tracer(lbm_sim* sim, int tracer, float* val) {

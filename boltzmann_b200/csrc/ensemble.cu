@@ -613,6 +613,7 @@ void release(lbm_ensemble* e) {
   cudaFree(e->shell.vel);
   cudaFree(e->shell.flags);
   cudaFree(e->shell.status);
+  cudaFree(e->shell.scratch);
   cudaFree(e->d_domains);
   cudaFree(e->d_tiles);
   cudaFree(e->d_rows);
@@ -678,6 +679,8 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
   // Rows longer than the staged kernel's stages go through the tile kernel.
   e->tile = e->max_row <= kRowMax ? 0 : 256;
   const size_t flag_bytes = ((size_t)n + 255) / 256 * 256;
+  const size_t scratch = std::min((size_t)n * sizeof(int32_t), lbm::kFlagPiece);
+  s.scratch_bytes = scratch;
   // 256 bytes of padding after the populations: the staged kernel's aligned row copies may
   // reach up to 15 bytes past the last slot's last row.
   if ((r = cudaMalloc(&s.f, (size_t)n * 9 * lbm::pop_bytes(storage) + 256)) != cudaSuccess ||
@@ -685,6 +688,7 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
       (r = cudaMalloc(&s.vel, (size_t)n * 2 * sizeof(float))) != cudaSuccess ||
       (r = cudaMalloc((void**)&s.flags, flag_bytes)) != cudaSuccess ||
       (r = cudaMalloc((void**)&s.status, 64 * sizeof(double))) != cudaSuccess ||
+      (r = cudaMalloc(&s.scratch, scratch)) != cudaSuccess ||
       (r = cudaMalloc((void**)&e->d_domains, ndomains * sizeof(DomainDesc))) != cudaSuccess)
     return bail(r, "cudaMalloc");
   s.sums = reinterpret_cast<double*>(s.status) + 1;

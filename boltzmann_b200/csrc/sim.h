@@ -14,7 +14,7 @@ struct lbm_sim {
     float omega = 0;      // omega (BGK) or omega+ (TRT)
     float omega_neg = 0;  // omega- (TRT)
     void* g = nullptr;    // [q][N], float (double for F64 storage)
-    void* val = nullptr;  // [N], in g's allocation
+    void* val = nullptr;  // [N]
   };
   struct Coupling {
     int tracer = 0;
@@ -47,7 +47,11 @@ struct lbm_sim {
   bool graph_warm = false, graph_failed = false;
   const float* omega_field = nullptr;  // caller-owned per-cell om_pos, or null
 
-  void* arena = nullptr;  // one allocation for f, rho, vel, flags, status and mail
+  std::vector<void*> owned;  // the device allocations behind the arrays below and the tracers'
+  // Fields on their way to or from the host: flags as int32 (in pieces where they do not fit), and
+  // FP64 fields as floats. Its users follow one another on the stream.
+  void* scratch = nullptr;
+  size_t scratch_bytes = 0;
   void* f = nullptr;    // [q][N] populations in the storage type
   void* rho = nullptr;  // [N], float (double for F64)
   void* vel = nullptr;  // [N][dim]
@@ -56,10 +60,9 @@ struct lbm_sim {
   double* sums = nullptr;     // device scratch of the conservation reduction
   int sums_len = 0;
 
-  // Message words of the resident kernel (zero at first, part of `arena` or of the tracer's
-  // allocation; null where it does not apply), the number of tracers they are laid out for, and the
-  // next sequence number.
-  void* mail = nullptr;
+  // The two sets of message words of the resident kernel (zero at first; null where it does not apply),
+  // the number of tracers they are laid out for, and the next sequence number.
+  void* mail[2] = {nullptr, nullptr};
   int mail_tracers = 0;
   unsigned mail_seq = 1;
   // The resident kernel's tiling for `resident_key` tracers (0 x 0: it does not fit).
@@ -84,6 +87,9 @@ void set_last_error(const std::string& msg);
 // Bytes of one stored population for a storage kind.
 inline size_t pop_bytes(int storage) { return storage == 3 ? 8 : (storage == 0 ? 4 : 2); }
 
+// Bytes of int32 flags that go to the device at a time (lbm_sim::scratch).
+constexpr size_t kFlagPiece = 8 << 20;
+
 // Enqueues one AA step of the whole simulation (fluid, tracers, sources) on sim.stream.
 cudaError_t launch_step_d2q9(const lbm_sim& sim, bool even, bool write_moments);
 cudaError_t launch_step_d3q27(const lbm_sim& sim, bool even, bool write_moments);
@@ -91,7 +97,7 @@ cudaError_t launch_step_d3q27(const lbm_sim& sim, bool even, bool write_moments)
 // The whole call of `steps` steps (even, moments at the end) in one launch that keeps the domain on the
 // chip (aa_resident.cu). cudaErrorNotSupported, with nothing enqueued, when it does not apply.
 cudaError_t iterate_resident(lbm_sim& sim, int64_t steps);
-// Bytes of its message words for a simulation with `tracers` tracers; 0 when it does not apply.
+// Bytes of one set of its message words for a simulation with `tracers` tracers; 0 when it does not apply.
 size_t resident_mail_bytes(lbm_sim& sim, int tracers);
 
 // Field kernels (fields.cu), all on sim.stream.
