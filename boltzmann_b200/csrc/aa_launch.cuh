@@ -69,24 +69,6 @@ StepArgs<Real> make_step_args(const lbm_sim& s, bool write_moments) {
   return a;
 }
 
-// Launches a step kernel as a programmatic dependent of the previous one on the stream (the kernels
-// wait for it on the device before they touch memory).
-template <class... Params, class... Args>
-cudaError_t launch_step_kernel(void (*kern)(Params...), unsigned grid, unsigned threads,
-                               size_t smem, cudaStream_t stream, const Args&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 // Ring depth of the TMA kernel: as many stages as fit in ~50 KB per CTA (2-4), so that three or
 // four CTAs (24-32 consumer warps) share an SM and each keeps one or more tiles of copies in
 // flight while it computes another.
@@ -197,17 +179,41 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
   return launch_step_kernel(kern, (unsigned)grid, threads, smem, stream, a, maps);
 }
 
+// Whether the TMA-staged kernel is the faster one for rows of whole 256-cell tiles (fused tracers: none
+// or one). It keeps more loads in flight per SM with fewer instructions, the direct kernel more warps
+// at work: domains that sit in L2, and cells with more arithmetic per byte, are better off direct. us a
+// step, direct / staged, after a second under load (cold, at full clocks, the direct kernel looks up
+// to 5% better), by which the lines are drawn:
+//   D2Q9  FP32         2048x1024 21.7 / 25.7, 3000x1536 64.1 / 63.8, 4096x2048 115.9 / 111.6
+//         with tracer  1024x512 8.3 / 11.0, 2048x1024 44.3 / 43.7, 4096x2048 TRT 176.4 / 171.0
+//         FP64         1500x1024 41.3 / 40.4; with a tracer 4096x1024 168 / 187
+//         FP16         4096x2048 76 / 87, TRT 79.4 / 79.0; with an FP16 tracer 118 / 143
+//   D3Q27 FP32 BGK     48x64x256 24.3 / 23.7, 200x200x256 390 / 356, 128x100x512 251 / 242
+//         FP32 TRT     48x64x256 25.3 / 31.0, 200x200x256 407 / 409, 128x100x512 260 / 354;
+//                      with a tracer 200x200x256 494 / 501 (BGK), 497 / 506
+//         FP16 BGK     32x48x256 9.9 / 10.0, 48x64x256 17.4 / 15.4, 128x100x512 165 / 161
+//         FP16 TRT     48x64x256 18.4 / 17.7, 128x100x512 184 / 233
+//         FP16 tracer  48x64x256 22.5 / 22.7, 100x100x256 90.7 / 70.5, 128x100x512 227 / 289
+//         FP64         48x64x256 61.3 / 57.8; with a tracer 77.4 / 73.6
+template <class L, bool TRT, int K, int NT>
+bool staged_pays(const StepArgs<typename Pop<K>::real>& a) {
+  const long long cells = (long long)a.nx * a.ny * a.nz;
+  if (L::D == 2) {
+    if (K == kF32) return cells >= (NT == 0 ? 6000000 : 2000000);
+    return K == kF64 && NT == 0 && cells >= 1500000;
+  }
+  if (dev_in<K>() && (TRT || NT != 0))
+    return a.nz == kTmaTile && cells >= (NT == 0 ? 700000 : 1500000);
+  if (K == kF32 && (TRT || NT != 0)) return false;
+  return cells >= 700000;
+}
+
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
 cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t stream,
                        int64_t* launches) {
-  // Rows that split into whole 256-cell tiles go through the TMA-staged kernel (fused tracers:
-  // none or one); everything else through the direct kernel.
-  // Small domains (under ~8 tiles per SM; they sit in L2 anyway) stay on the direct kernel,
-  // whose launch has no ring to fill and drain.
   if constexpr (NT >= 0) {
-    const long long tiles = (long long)a.nx * a.ny * (a.nz / kTmaTile);
     const bool fits = a.nz % kTmaTile == 0;
-    const bool staged = a.path == 2 || (a.path == 0 && tiles >= 8LL * 148);
+    const bool staged = a.path == 2 || (a.path == 0 && staged_pays<L, TRT, K, NT>(a));
     if (fits && staged) {
       cudaError_t e;
       if (EVEN && a.nz == kTmaTile)

@@ -648,6 +648,24 @@ __device__ __forceinline__ void grid_wait_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Launches a step kernel as a programmatic dependent of the previous one on the stream (the kernels
+// wait for it on the device before they touch memory).
+template <class... Params, class... Args>
+cudaError_t launch_step_kernel(void (*kern)(Params...), unsigned grid, unsigned threads,
+                               size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 constexpr int kDirectThreads = 128;
 // How the direct kernel of a lattice, storage and tracer form addresses populations, and the CTAs
 // an SM its registers must allow. A D3Q27 cell has 54 addresses; kept from the loads to the stores
