@@ -39,7 +39,8 @@ def size_class(ens) -> str:
 def key(ens, storage: str) -> str:
     coll = "trt" if ens.collision else "bgk"
     rows = "rows" if max(b for _, b in ens.counts) <= ROW_MAX else "tiles-only"
-    return f"D2Q9/{coll}/{storage}/{size_class(ens)}/{KERNELS}/{rows}"
+    flat = "/flat" if getattr(ens, "flat", False) else ""  # entries made before the flat kernel
+    return f"D2Q9/{coll}/{storage}/{size_class(ens)}/{KERNELS}/{rows}{flat}"
 
 
 def _load() -> dict:
@@ -89,7 +90,9 @@ def tune(ens, storage: str = "f32", use_cache: bool = True, pairs: int = 4) -> d
     saved = ens.populations()
     saved_iteration = ens.iteration
     timings = {}
-    shapes = [(0, b) for b in ROW_BLOCKS] if max(b for _, b in ens.counts) <= ROW_MAX else []
+    # A small ensemble's shapes 0, 0 and 128, 0 are one kernel: timed once, as the latter.
+    rows = [b for b in ROW_BLOCKS if b or not getattr(ens, "flat", False)]
+    shapes = [(0, b) for b in rows] if max(b for _, b in ens.counts) <= ROW_MAX else []
     shapes += [(t, b) for t in TILES for b in BLOCKS]
     for tile, blocks in shapes:
         timings[f"{tile}x{blocks}"] = time_shape(ens, tile, blocks, pairs)

@@ -10,7 +10,7 @@
 // domain is periodic in itself (its own rows wrap), exactly as a separate simulation of that size
 // would be, and the cell update is the same device function the single-domain kernels use.
 //
-// Two kernels walk the domains:
+// Three kernels walk the domains (small ensembles: flat, one cell a thread, see below):
 //   rows (default whenever every row has at most 512 cells): one domain row per work item. A
 //     producer warp copies, with one TMA bulk copy per population slot, the 16-byte-aligned
 //     superset of the row that slot is read from (on even steps rows x-1, x, x+1 of the domain,
@@ -107,6 +107,63 @@ __global__ void __launch_bounds__(512)
       update_cell<D2Q9, TRT, K, EVEN, 0>(a, c[1], flagB, fb, g, Real(0), (Real)dom.om_pos,
                                          (Real)dom.om_neg);
   }
+}
+
+// ---- The flat kernel: all domains' cells in order, one a thread, as dependent launches (aa_step.cuh).
+// For ensembles whose populations sit in L2, where the row-staged kernel's ring (a row a stage, its
+// fill and drain every step, whole SMs waiting on a launch) is longer than the work. us a step, row-
+// staged and flat: 9 domains of 210,371 cells in all 5.6 / 3.3, 72 of 369,358 11.2 / 5.1, 64 of
+// 1,574,641 25.2 / 16.5, FP16 32 of 3,734,984 38.2 / 34.7; past L2 32 of 3,734,984 52.4 / 58.6, FP16
+// 128 of 13,045,701 130 / 168.
+constexpr size_t kFlatBytes = 90u << 20;  // of populations
+
+// A domain for threads that hold a cell index.
+struct FlatDomain {
+  unsigned base, next;   // first cell, first cell of the next domain
+  unsigned nx, ny;
+  lbm::FastDiv by_ny;
+  float om_pos, om_neg;
+};
+
+struct FlatArgs {
+  const FlatDomain* domains;
+  const int* first;  // domain of each CTA's first cell
+  unsigned cells;
+};
+
+template <bool TRT, int K, bool EVEN>
+__global__ void __launch_bounds__(lbm::kDirectThreads, 8)
+    ensemble_flat_kernel(const __grid_constant__ lbm::StepArgs<typename lbm::Pop<K>::real> a,
+                         const FlatArgs e) {
+  using namespace lbm;
+  using P = Pop<K>;
+  using Real = typename P::real;
+  grid_trigger_next();
+  const unsigned cell = blockIdx.x * (unsigned)kDirectThreads + threadIdx.x;
+  if (cell >= e.cells) return;
+  // The tables never change, so they are read before the previous step has ended.
+  int k = e.first[blockIdx.x];
+  while (cell >= e.domains[k].next) ++k;
+  const FlatDomain dom = e.domains[k];
+  const unsigned local = cell - dom.base, x = dom.by_ny.div(local), z = local - x * dom.ny;
+  CellPos c;
+  c.cell = cell;
+  c.ox[0] = c.ox[1] = c.ox[2] = dom.base;
+  c.oy[1] = x * dom.ny;
+  c.oz[1] = z;
+  if (EVEN) {
+    c.oy[0] = (x == 0 ? dom.nx - 1 : x - 1) * dom.ny;
+    c.oy[2] = (x == dom.nx - 1 ? 0 : x + 1) * dom.ny;
+    c.oz[0] = z == 0 ? dom.ny - 1 : z - 1;
+    c.oz[2] = z == dom.ny - 1 ? 0 : z + 1;
+  }
+  grid_wait_previous();
+  const int flag = a.flags[cell];
+  Real f[D2Q9::Q];
+  aa_load<D2Q9, P, EVEN, dev_in<K>()>(a.f, nullptr, a.n, c, f);
+  Real g[1];
+  update_cell<D2Q9, TRT, K, EVEN, 0, GlobalSink<>, default_tracer_kind<K>(), true>(
+      a, c, flag, f, g, Real(0), (Real)dom.om_pos, (Real)dom.om_neg);
 }
 
 // ---- The row-staged kernel.
@@ -388,6 +445,8 @@ struct lbm_ensemble {
   RowDesc* d_rows = nullptr;       // the row table of the row-staged kernel (tile == 0)
   long long nrows = 0;
   int max_row = 0;                 // longest row (cells)
+  FlatDomain* d_flat = nullptr;    // the flat kernel's tables (null for large ensembles)
+  int* d_first = nullptr;
   // Captured graph of `graph_pairs` step pairs in persistent mode.
   cudaGraphExec_t graph = nullptr;
   int graph_pairs = 0, graph_tile = 0, graph_blocks = 0;
@@ -495,6 +554,41 @@ cudaError_t launch_persistent(lbm_ensemble* e, bool even, bool write_moments) {
   return cudaGetLastError();
 }
 
+template <bool TRT, int K>
+cudaError_t launch_flat(lbm_ensemble* e, bool even, bool write_moments) {
+  using Real = typename lbm::Pop<K>::real;
+  const lbm::StepArgs<Real> a = base_args<Real>(e, write_moments);
+  const FlatArgs args{e->d_flat, e->d_first, (unsigned)e->n};
+  auto kern = even ? ensemble_flat_kernel<TRT, K, true> : ensemble_flat_kernel<TRT, K, false>;
+  const unsigned grid = (unsigned)((e->n + lbm::kDirectThreads - 1) / lbm::kDirectThreads);
+  return lbm::launch_step_kernel(kern, grid, lbm::kDirectThreads, 0, e->stream, a, args);
+}
+
+// The flat kernel's tables, in one allocation.
+cudaError_t build_flat(lbm_ensemble* e) {
+  std::vector<FlatDomain> flat;
+  for (const DomainDesc& d : e->domains)
+    flat.push_back(FlatDomain{(unsigned)d.base, (unsigned)(d.base + (long long)d.nx * d.ny),
+                              (unsigned)d.nx, (unsigned)d.ny, lbm::FastDiv((unsigned)d.ny), d.om_pos,
+                              d.om_neg});
+  std::vector<int> first;
+  int k = 0;
+  for (long long c = 0; c < e->n; c += lbm::kDirectThreads) {
+    while (c >= flat[k].next) ++k;
+    first.push_back(k);
+  }
+  const size_t bytes = flat.size() * sizeof(FlatDomain);
+  cudaError_t r = cudaMalloc((void**)&e->d_flat, bytes + first.size() * sizeof(int));
+  if (r != cudaSuccess) return r;
+  e->d_first = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(e->d_flat) + bytes);
+  if ((r = cudaMemcpyAsync(e->d_flat, flat.data(), bytes, cudaMemcpyHostToDevice, e->stream)))
+    return r;
+  if ((r = cudaMemcpyAsync(e->d_first, first.data(), first.size() * sizeof(int),
+                           cudaMemcpyHostToDevice, e->stream)))
+    return r;
+  return cudaStreamSynchronize(e->stream);
+}
+
 template <bool TRT, int K, bool EVEN>
 cudaError_t launch_rows_parity(lbm_ensemble* e, bool write_moments) {
   using Real = typename lbm::Pop<K>::real;
@@ -556,6 +650,9 @@ cudaError_t launch_per_domain(lbm_ensemble* e, bool even, bool write_moments) {
 template <bool TRT, int K>
 cudaError_t launch_step(lbm_ensemble* e, bool even, bool write_moments, int mode) {
   if (mode == 2) return launch_per_domain<TRT, K>(e, even, write_moments);
+  if ((e->tile == 0 || e->tile == lbm::kDirectThreads) && e->blocks_per_sm == 0 &&
+      e->d_flat != nullptr)
+    return launch_flat<TRT, K>(e, even, write_moments);
   if (e->tile == 0)
     return even ? launch_rows_parity<TRT, K, true>(e, write_moments)
                 : launch_rows_parity<TRT, K, false>(e, write_moments);
@@ -617,6 +714,7 @@ void release(lbm_ensemble* e) {
   cudaFree(e->d_domains);
   cudaFree(e->d_tiles);
   cudaFree(e->d_rows);
+  cudaFree(e->d_flat);
   if (e->stream) cudaStreamDestroy(e->stream);
 }
 
@@ -677,7 +775,8 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
   s.device = e->device;
   s.stream = e->stream;
   // Rows longer than the staged kernel's stages go through the tile kernel.
-  e->tile = e->max_row <= kRowMax ? 0 : 256;
+  const bool flat = (size_t)n * 9 * lbm::pop_bytes(storage) <= kFlatBytes;
+  e->tile = e->max_row <= kRowMax ? 0 : (flat ? lbm::kDirectThreads : 256);
   const size_t flag_bytes = ((size_t)n + 255) / 256 * 256;
   const size_t scratch = std::min((size_t)n * sizeof(int32_t), lbm::kFlagPiece);
   s.scratch_bytes = scratch;
@@ -703,6 +802,8 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
     delete e;
     return rc;
   }
+  if (flat)
+    if ((r = build_flat(e)) != cudaSuccess) return bail(r, "ensemble tables");
   *out = e;
   return LBM_OK;
 }

@@ -23,6 +23,7 @@ _lib.lbm_last_error.restype = C.c_char_p
 
 MODES = {"persistent": 0, "graph": 1, "per_domain": 2}
 STORAGE = {"f32": 0, "f16": 1, "bf16": 2}
+FLAT_BYTES = 90 << 20  # populations of the largest ensemble that takes the flat kernel
 
 
 def _check(rc: int) -> None:
@@ -62,8 +63,10 @@ class Ensemble:
         self.vel = np.zeros((self.n, 2), np.float32)
         self.iteration = 0
         # The library's default: the row-staged kernel (tile 0) when every row has at most 512
-        # cells, else tiles of 256 cells; CTAs per SM as many as fit.
-        self.shape = (0 if max(b for _, b in self.counts) <= 512 else 256, 0)
+        # cells, else tiles of 256 cells, CTAs per SM as many as fit; for a small ensemble the flat
+        # kernel (tiles 0 and 128).
+        self.flat = self.n * 9 * (4 if storage == "f32" else 2) <= FLAT_BYTES
+        self.shape = (0 if max(b for _, b in self.counts) <= 512 else 128 if self.flat else 256, 0)
 
     def __del__(self):
         if getattr(self, "h", None):

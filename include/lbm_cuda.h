@@ -173,8 +173,8 @@ LBM_API int lbm_set_kernel_path(lbm_sim* sim, int path);
  * path. No reference counterpart. */
 LBM_API int lbm_set_spin_limit(lbm_sim* sim, int64_t polls);
 
-/* AA step launches since lbm_create, per kernel variant: the direct kernel (aa_step_kernel) and
- * the TMA-staged one (aa_tma_kernel). Host-side counters, no synchronisation. No reference
+/* AA step launches since lbm_create, per kernel variant: the direct kernel (aa_step_kernel; the
+ * steps of resident launches count here, one each) and the TMA-staged one (aa_tma_kernel). Host-side counters, no synchronisation. No reference
  * counterpart (instrumentation: which kernel a workload actually ran). */
 LBM_API int lbm_launch_counts(lbm_sim* sim, int64_t* direct, int64_t* staged);
 
@@ -234,7 +234,9 @@ LBM_API int lbm_ensemble_cells(lbm_ensemble* ens, int64_t* total);
  * when every domain row has at most 512 cells; LBM_ERR_UNSUPPORTED otherwise): one domain row
  * per work item, loaded by TMA bulk copies into a shared-memory ring. A multiple of 32 in
  * [32, 512] selects the tile kernel with that many cells per tile (two per thread), loads straight
- * into registers. blocks_per_sm: CTAs per SM of the persistent grid (0 = as many as fit).
+ * into registers. blocks_per_sm: CTAs per SM of the persistent grid (0 = as many as fit). Small
+ * ensembles (at most 90 MB of populations) take a flat kernel with the shapes 0, 0 and 128, 0: one
+ * cell a thread over all domains' cells in order, rows of any length; it is their default.
  * Chosen by the autotuner (boltzmann_b200.autotune); every shape gives the same bits. */
 LBM_API int lbm_ensemble_set_shape(lbm_ensemble* ens, int tile_cells, int blocks_per_sm);
 LBM_API int lbm_ensemble_upload(lbm_ensemble* ens, const int32_t* flags, const float* rho,
