@@ -144,6 +144,19 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// d += A * B with the running sum d kept by rounded FP32 additions. The tensor cores truncate what
+// they add to, so a sum chained through them drifts with its length: over 4 M cells the gradients
+// of layers 1 and 3 were 1.0e-6 and 2.4e-6 off, against 1.0e-7 and 2.6e-8 in FP32 on the CUDA
+// cores. The 16 products of one instruction lose next to nothing.
+__device__ __forceinline__ void mma_bf16_add(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                             uint32_t b1) {
+  float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  mma_bf16(t, a, b0, b1);
+  const float2 lo = __fadd2_rn(make_float2(d[0], d[1]), make_float2(t[0], t[1]));
+  const float2 hi = __fadd2_rn(make_float2(d[2], d[3]), make_float2(t[2], t[3]));
+  d[0] = lo.x, d[1] = lo.y, d[2] = hi.x, d[3] = hi.y;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Shared-memory tile loads (zero outside the domain).
 
@@ -794,7 +807,7 @@ __global__ void __launch_bounds__(kC3Threads, 2)
 // lane. The weight gradient on tensor cores: M = (part, tap), N = ci, K = cells, where dy enters as
 // the exact sum of three BF16 parts (8 + 8 + 8 significant bits), so that every product is that of
 // the FP32 value; the parts' sums are added at the end. (One thread an output over the tile's 256
-// cells was the kernel's longest part by far.) Bound by 260 bytes a cell. Batch 8 x 1024 x 512: 978 -> 332 us.
+// cells was the kernel's longest part by far.) Bound by 260 bytes a cell. Batch 8 x 1024 x 512: 978 -> 325 us.
 
 constexpr int kB3Threads = 256;
 constexpr int kDyS = kHY + 2;  // BF16 elements of a row of a dy part (a multiple of 2)
@@ -973,8 +986,13 @@ __global__ void __launch_bounds__(kB3Threads, 2)
         ldsm_x4_t(r, as + cell * kCS + (2 * np + (mi >> 1)) * 8);
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
-          mma_bf16(acc[mt][2 * np], af[mt], r[0], r[1]);
-          mma_bf16(acc[mt][2 * np + 1], af[mt], r[2], r[3]);
+          if (mt == 0) {  // rows of the first part, h; the others are below 2^-8 of it
+            mma_bf16_add(acc[mt][2 * np], af[mt], r[0], r[1]);
+            mma_bf16_add(acc[mt][2 * np + 1], af[mt], r[2], r[3]);
+          } else {
+            mma_bf16(acc[mt][2 * np], af[mt], r[0], r[1]);
+            mma_bf16(acc[mt][2 * np + 1], af[mt], r[2], r[3]);
+          }
         }
       }
     }
@@ -1029,7 +1047,8 @@ __global__ void __launch_bounds__(kB3Threads, 2)
 // M = 32 output channels (2 m-tiles), N = 36 (tap, ci) columns (5 n-tiles, the last half empty),
 // K = cells. dz1 comes through ldmatrix; the features lie in shared memory as one plane a channel,
 // twice (the second copy shifted by one cell), so that two consecutive cells of any tap are one
-// aligned 32-bit word. Bound by reading dz1 and x. Batch 8 x 1024 x 512: 870 -> 93 us.
+// aligned 32-bit word. Bound by reading dz1 and x; two CTAs an SM. Batch 8 x 1024 x 512: 870 -> 98 us
+// (93 with the sums left in the tensor cores, which mma_bf16_add tells why not).
 
 constexpr int kW1Threads = 256;
 constexpr int kXS = kHY + 2;  // BF16 elements of a row of a feature plane
@@ -1040,7 +1059,7 @@ constexpr size_t kW1Smem = (size_t)(kW1Threads / 32) * 36 * C * 4 > kW1Stage
                                ? (size_t)(kW1Threads / 32) * 36 * C * 4
                                : kW1Stage;
 
-__global__ void __launch_bounds__(kW1Threads, 3)
+__global__ void __launch_bounds__(kW1Threads, 2)
     conv1_wgrad_kernel(Grid g, const bf16* __restrict__ x, const bf16* __restrict__ dz1,
                        float* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1107,7 +1126,7 @@ __global__ void __launch_bounds__(kW1Threads, 3)
         const uint32_t* p = reinterpret_cast<const uint32_t*>(xp + boff[nt] + ks * 16);
         const uint32_t b0 = boff[nt] >= 0 ? p[0] : 0u, b1 = boff[nt] >= 0 ? p[4] : 0u;
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) mma_bf16(acc[mt][nt], af[mt], b0, b1);
+        for (int mt = 0; mt < 2; ++mt) mma_bf16_add(acc[mt][nt], af[mt], b0, b1);
       }
     }
   }
