@@ -243,6 +243,18 @@ __device__ __forceinline__ float2 gelu2(float2 z) {
   return make_float2(__fdividef(z.x, d.x), __fdividef(z.y, d.y));
 }
 
+// gelu_grad of two values, likewise.
+__device__ __forceinline__ float2 gelu_grad2(float2 z) {
+  const float2 one = make_float2(1.0f, 1.0f), a = make_float2(kGeluA, kGeluA);
+  const float2 z2 = __fmul2_rn(z, z);
+  const float2 v = __fmul2_rn(z, ffma2(make_float2(kGeluB, kGeluB), z2, a));
+  const float2 d = __fadd2_rn(one, make_float2(__expf(-v.x), __expf(-v.y)));
+  const float2 sg = make_float2(__fdividef(1.0f, d.x), __fdividef(1.0f, d.y));
+  const float2 rest = __fadd2_rn(one, make_float2(-sg.x, -sg.y));
+  const float2 slope = ffma2(make_float2(3.0f * kGeluB, 3.0f * kGeluB), z2, a);
+  return __fmul2_rn(sg, ffma2(__fmul2_rn(z, rest), slope, one));
+}
+
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -468,8 +480,7 @@ __global__ void __launch_bounds__(kC1Threads, kC1PerSm)
 // of 16), N = 32 channels (4 n-tiles of 8), K = 9 taps x 32 channels (18 k-steps of 16).
 //
 // Forward:  z[p][co] = b[co] + sum_{tap,ci} W[co][tap][ci] a[p + tap][ci];  a2 = GELU(z) (BF16)
-// Backward: d[q][ci] = sum_{tap,co} W[co][tap][ci] dz[q - tap][co];  dz1 = d GELU'(z1) (BF16),
-//           plus the per-channel sums of dz1 (the layer-1 bias gradient) into partial rows.
+// Backward: d[q][ci] = sum_{tap,co} W[co][tap][ci] dz[q - tap][co];  dz1 = d GELU'(z1) (BF16).
 
 constexpr int kConv32Threads = 128;
 constexpr size_t kConv32Smem = (size_t)(kHX * kHY * kCS + C * kWS) * sizeof(bf16);
@@ -478,19 +489,14 @@ template <bool BWD>
 __global__ void __launch_bounds__(kConv32Threads)
     conv32_kernel(Grid g, const bf16* __restrict__ in, const bf16* __restrict__ w2,
                   const float* __restrict__ bias, const float* __restrict__ zin,
-                  float* __restrict__ zout, bf16* __restrict__ out, float* __restrict__ partial) {
+                  float* __restrict__ zout, bf16* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* ins = reinterpret_cast<bf16*>(smem_raw);
   bf16* wsm = ins + kHX * kHY * kCS;
-  __shared__ float colsum[kConv32Threads / 32][C];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
   load_w2(w2, wsm);
-
-  float bias_sum[4][2];  // BWD: this thread's running sums of dz1 for channels nt*8 + 2tq (+1)
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt) bias_sum[nt][0] = bias_sum[nt][1] = 0.0f;
 
   for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
     int64_t b, x0, y0;
@@ -567,32 +573,10 @@ __global__ void __launch_bounds__(kConv32Threads)
             const float2 z = *reinterpret_cast<const float2*>(zin + cell * C + ch);
             o.x = to_bf(v0 * gelu_grad(z.x));
             o.y = to_bf(v1 * gelu_grad(z.y));
-            bias_sum[nt][0] += bf(o.x);
-            bias_sum[nt][1] += bf(o.y);
           }
           *reinterpret_cast<__nv_bfloat162*>(out + cell * C + ch) = o;
         }
       }
-    }
-  }
-
-  if (BWD) {
-    // Sum over the 8 lanes sharing tq, then over warps, in a fixed order.
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float s = bias_sum[nt][e];
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        s += __shfl_xor_sync(0xffffffffu, s, 8);
-        s += __shfl_xor_sync(0xffffffffu, s, 16);
-        if (gq == 0) colsum[warp][nt * 8 + 2 * tq + e] = s;
-      }
-    __syncthreads();
-    if (threadIdx.x < C) {
-      float s = 0.0f;
-      for (int w = 0; w < kConv32Threads / 32; ++w) s += colsum[w][threadIdx.x];
-      partial[(int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_B1 + threadIdx.x] = s;
     }
   }
 }
@@ -1044,19 +1028,19 @@ __global__ void __launch_bounds__(kB3Threads, 2)
 
 // ---------------------------------------------------------------------------------------------
 // Layer-1 weight gradient on tensor cores: dW1[co][tap][ci] = sum_p dz1[p][co] x[p + tap][ci].
-// M = 32 output channels (2 m-tiles), N = 36 (tap, ci) columns (5 n-tiles, the last half empty),
-// K = cells. dz1 comes through ldmatrix; the features lie in shared memory as one plane a channel,
+// M = 32 output channels (2 m-tiles), N = 36 (tap, ci) columns and one of ones, whose sums are the
+// bias gradient (5 n-tiles, the last three columns empty), K = cells. dz1 comes through ldmatrix; the features lie in shared memory as one plane a channel,
 // twice (the second copy shifted by one cell), so that two consecutive cells of any tap are one
-// aligned 32-bit word. Bound by reading dz1 and x; two CTAs an SM. Batch 8 x 1024 x 512: 870 -> 98 us
-// (93 with the sums left in the tensor cores, which mma_bf16_add tells why not).
+// aligned 32-bit word. Bound by reading dz1 and x; two CTAs an SM. Batch
+// 8 x 1024 x 512: 870 -> 98 us (93 with the sums left in the tensor cores: mma_bf16_add).
 
 constexpr int kW1Threads = 256;
 constexpr int kXS = kHY + 2;  // BF16 elements of a row of a feature plane
 constexpr size_t kW1Stage0 = (size_t)kTX * kTY * kCS * 2;  // dz1 of a tile
 constexpr size_t kW1OffX = 2 * kW1Stage0;
 constexpr size_t kW1Stage = kW1OffX + (size_t)4 * 2 * kHX * kXS * 2;
-constexpr size_t kW1Smem = (size_t)(kW1Threads / 32) * 36 * C * 4 > kW1Stage
-                               ? (size_t)(kW1Threads / 32) * 36 * C * 4
+constexpr size_t kW1Smem = (size_t)(kW1Threads / 32) * 37 * C * 4 > kW1Stage
+                               ? (size_t)(kW1Threads / 32) * 37 * C * 4
                                : kW1Stage;
 
 __global__ void __launch_bounds__(kW1Threads, 2)
@@ -1078,6 +1062,8 @@ __global__ void __launch_bounds__(kW1Threads, 2)
       boff[nt] = ((ci * 2 + odd) * kHX + r) * kXS + col - odd + 2 * tq;
     }
   }
+  // Column 36 holds ones: the sums of dz1, the bias gradient.
+  const uint32_t none = gq == 4 ? 0x3f803f80u : 0u;
   float acc[2][5][4];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
@@ -1124,7 +1110,7 @@ __global__ void __launch_bounds__(kW1Threads, 2)
 #pragma unroll
       for (int nt = 0; nt < 5; ++nt) {
         const uint32_t* p = reinterpret_cast<const uint32_t*>(xp + boff[nt] + ks * 16);
-        const uint32_t b0 = boff[nt] >= 0 ? p[0] : 0u, b1 = boff[nt] >= 0 ? p[4] : 0u;
+        const uint32_t b0 = boff[nt] >= 0 ? p[0] : none, b1 = boff[nt] >= 0 ? p[4] : none;
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) mma_bf16_add(acc[mt][nt], af[mt], b0, b1);
       }
@@ -1132,7 +1118,7 @@ __global__ void __launch_bounds__(kW1Threads, 2)
   }
   cp_async_wait<0>();
   __syncthreads();
-  float* sums = reinterpret_cast<float*>(smem_raw);  // [warp][co][36]
+  float* sums = reinterpret_cast<float*>(smem_raw);  // [warp][co][37]
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
@@ -1140,14 +1126,15 @@ __global__ void __launch_bounds__(kW1Threads, 2)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int co = mt * 16 + gq + 8 * (e >> 1), n = nt * 8 + 2 * tq + (e & 1);
-        if (n < 36) sums[(warp * C + co) * 36 + n] = acc[mt][nt][e];
+        if (n < 37) sums[(warp * C + co) * 37 + n] = acc[mt][nt][e];
       }
   __syncthreads();
-  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W1;
-  for (int i = threadIdx.x; i < 36 * C; i += blockDim.x) {
+  float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS;
+  for (int i = threadIdx.x; i < 37 * C; i += blockDim.x) {
     float v = 0.0f;
-    for (int w = 0; w < kW1Threads / 32; ++w) v += sums[w * 36 * C + i];
-    row[i] = v;
+    for (int w = 0; w < kW1Threads / 32; ++w) v += sums[w * 37 * C + i];
+    const int co = i / 37, n = i - co * 37;
+    row[n < 36 ? LBM_CLOSURE_OFF_W1 + co * 36 + n : LBM_CLOSURE_OFF_B1 + co] = v;
   }
 }
 
@@ -1707,8 +1694,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 // ---------------------------------------------------------------------------------------------
 // Layer 2 of the training path on tcgen05: the forward conv (BWD = false: z2 = b2 + W * a1,
 // a2 = GELU(z2) in BF16) and the transposed conv of the backward pass (BWD = true:
-// d = W^T * dz2, dz1 = BF16(d GELU'(z1)), plus the per-channel sums of dz1 for the layer-1 bias
-// gradient in this CTA's partial row). Same products as conv32_kernel, on the fifth-generation
+// d = W^T * dz2, dz1 = BF16(d GELU'(z1))). Same products as conv32_kernel, on the fifth-generation
 // tensor cores with the layout of the fused inference kernel's layer 2:
 //   - a tile of kTR x kTC output cells reads a (kTR + 2) x (kTC + 2) input region, staged
 //     chunk-major: plane k (channels 8k .. 8k+7) holds 16 bytes a cell, cells in row-major order
@@ -1720,25 +1706,28 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 //   - the B operand is the weights as K-chunks of 8: [k chunk][n][8] with k = (tap, ci) and
 //     n = co for the forward conv, k = (tap, co) and n = ci for the transposed one.
 // One thread issues the MMAs and commits them to an mbarrier (bounded wait, as everywhere); the
-// epilogue reads each cell's 32 accumulators with tcgen05.ld. Two CTAs share an SM, so one stages
-// its next tile while the other's MMAs and epilogue run.
+// epilogue reads each cell's 32 accumulators with tcgen05.ld. Three CTAs share an SM, so one stages
+// its next tile while the others' MMAs and epilogues run: a chain of waits, longer than what the
+// memory (260 bytes a cell) takes. Tiles of 14 x 32 cells with one 4 KB slot a warp are what lets a
+// third CTA in; with 14 x 64, two slots and two CTAs, the two kernels took 308 and 300 us over
+// batch 8 x 1024 x 512, now 291 and 276.
 
-constexpr int kTR = 14, kTC = 64;                  // output tile
+constexpr int kTR = 14, kTC = 32;                  // output tile
 constexpr int kTRegR = kTR + 2, kTRegC = kTC + 2;  // input region
 constexpr int kTFirst = kTRegC + 1;                // region index of output cell (0, 0)
 constexpr int kTBlocks = (kTR * kTRegC + 127) / 128;  // 128-cell blocks covering the output rows
-constexpr int kTPad = 1168;  // cells per plane: >= kTFirst + 128 kTBlocks + kTRegC + 1, and a
-                             // multiple of 8 so that every plane starts on a 128-byte boundary
+constexpr int kTPad = 584;  // cells per plane: >= kTFirst + 128 kTBlocks + kTRegC + 1, and a
+                            // multiple of 8 so that every plane starts on a 128-byte boundary
 constexpr int kTThreads = 256;
-constexpr int kTTmemCols = 256;  // 8 accumulators of 32 FP32 columns
+constexpr int kTTmemCols = 128;  // 4 accumulators of 32 FP32 columns
+constexpr int kTPerSm = 3;
 constexpr size_t kTOffW = (size_t)4 * kTPad * 16;
 constexpr size_t kTOffBias = kTOffW + (size_t)36 * C * 16;
 constexpr size_t kTOffBar = kTOffBias + (size_t)C * 4;  // MMA mbarrier, load mbarrier, TMEM addr
 constexpr size_t kTSmem = kTOffBar + 24;
-constexpr int kTStageBytes = 2 * 32 * 128;  // a warp's rows in the epilogue
+constexpr int kTStageBytes = 32 * 128;  // a warp's rows in the epilogue
 static_assert((size_t)(kTThreads / 32) * kTStageBytes <= kTOffW, "the epilogue's rows must fit");
 constexpr unsigned kTLoadBytes = 4u * kTRegR * kTRegC * 16;  // the four plane boxes of a tile
-static_assert((size_t)kTThreads * (C + 1) * 4 <= kTOffW, "bias partial sums must fit the region");
 static_assert(kTBlocks * 32 <= kTTmemCols, "accumulators exceed the TMEM allocation");
 static_assert(kTFirst + kTBlocks * 128 + kTRegC + 1 <= kTPad, "planes too short for the shifts");
 static_assert(kTFirst + kTBlocks * 128 - 1 >= (kTR * kTRegC) + kTC, "blocks do not cover the tile");
@@ -1765,11 +1754,11 @@ __device__ __forceinline__ void tc_expect_tx(uint64_t* bar, unsigned bytes) {
 }
 
 template <bool BWD>
-__global__ void __launch_bounds__(kTThreads, 2)
+__global__ void __launch_bounds__(kTThreads, kTPerSm)
     conv32_tc_kernel(Grid g, const __grid_constant__ CUtensorMap in_map,
                      const bf16* __restrict__ w2, const float* __restrict__ bias,
                      const float* __restrict__ zin, float* __restrict__ zout,
-                     bf16* __restrict__ out, float* __restrict__ partial) {
+                     bf16* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* ac = smem_raw;                    // [4 planes][kTPad cells][16 B]
   unsigned char* wc = smem_raw + kTOffW;           // [36 K-chunks][32 n][16 B]
@@ -1821,9 +1810,6 @@ __global__ void __launch_bounds__(kTThreads, 2)
   const unsigned spin_limit = g_closure_spin_limit;
   bool healthy = true;
   unsigned phase = 0, load_phase = 0;
-  float bias_sum[C];  // BWD: this thread's running sums of dz1 per channel
-#pragma unroll
-  for (int c = 0; c < C; ++c) bias_sum[c] = 0.0f;
 
   for (int64_t t = blockIdx.x; t < g.tiles && healthy; t += gridDim.x) {
     int64_t b, x0, y0;
@@ -1882,45 +1868,33 @@ __global__ void __launch_bounds__(kTThreads, 2)
     // accesses are whole 128-byte lines: a lane's own row of 128 bytes at a time is a quarter of
     // that. Chunk c of the row of lane l lies at chunk c ^ (l % 8).
     const int sp = warp & 3;
-    unsigned char* own = ac + warp * kTStageBytes;  // this warp's: two slots of 32 rows x 128 bytes
-    auto cell_of = [&](int m, int64_t& cell) {      // block m's cell of this lane, if it has one
+    unsigned char* buf = ac + warp * kTStageBytes;  // this warp's 32 rows x 128 bytes
+    auto cell_of = [&](int m, int64_t& cell) {      // block m's cell of this lane, or -1
       const int q = kTFirst + 128 * m + 32 * sp + lane;  // region index of this row
       const int r = q / kTRegC - 1, c = q % kTRegC - 1;   // output tile coordinates
       const int64_t x = x0 + r, y = y0 + c;
       const bool ok = r >= 0 && r < kTR && c >= 0 && c < kTC && x < g.nx && y < g.ny;
       cell = ok ? g.cell(b, x, y) : -1;
-      return ok;
     };
-    auto fetch_z = [&](int m, int slot) {  // BWD: block m's rows of z1 into a slot
+    for (int m = warp >> 2; m < kTBlocks; m += kWarps / 4) {
       int64_t cell;
       cell_of(m, cell);
+      if (BWD) {  // this block's rows of z1
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int l = 4 * k + (lane >> 3), ch = lane & 7;
-        const int64_t cl = __shfl_sync(0xffffffffu, cell, l);
-        cp_async16(own + slot * 4096 + l * 128 + ((ch ^ (l & 7)) * 16),
-                   cl >= 0 ? zin + cl * C + ch * 4 : zin, cl >= 0);
-      }
-      cp_async_commit();
-    };
-    constexpr int kStep = kWarps / 4;
-    if (BWD) fetch_z(warp >> 2, 0);
-    int slot = 0;
-    for (int m = warp >> 2; m < kTBlocks; m += kStep) {
-      if (BWD) {
-        if (m + kStep < kTBlocks) {
-          fetch_z(m + kStep, slot ^ 1);
-          cp_async_wait<1>();
-        } else {
-          cp_async_wait<0>();
+        for (int k = 0; k < 8; ++k) {
+          const int l = 4 * k + (lane >> 3), ch = lane & 7;
+          const int64_t cl = __shfl_sync(0xffffffffu, cell, l);
+          cp_async16(buf + l * 128 + ((ch ^ (l & 7)) * 16), cl >= 0 ? zin + cl * C + ch * 4 : zin,
+                     cl >= 0);
         }
-        __syncwarp();
+        cp_async_commit();
       }
       uint32_t r32[32];
       tmem_ld32(tmem + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
-      int64_t cell;
-      const bool valid = cell_of(m, cell);
-      unsigned char* buf = own + slot * 4096;
+      if (BWD) {
+        cp_async_wait<0>();
+        __syncwarp();
+      }
       uint4* mine = reinterpret_cast<uint4*>(buf + lane * 128);
       uint32_t packed[C / 2];
       if (!BWD) {
@@ -1955,12 +1929,9 @@ __global__ void __launch_bounds__(kTThreads, 2)
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
             const int ch = 4 * k + e;
-            packed[ch / 2] = pack_bf2(__uint_as_float(r32[ch]) * gelu_grad(zv[e]),
-                                      __uint_as_float(r32[ch + 1]) * gelu_grad(zv[e + 1]));
-            if (valid) {
-              bias_sum[ch] += bf_lo(packed[ch / 2]);
-              bias_sum[ch + 1] += bf_hi(packed[ch / 2]);
-            }
+            packed[ch / 2] = pack_bf2(
+                __fmul2_rn(make_float2(__uint_as_float(r32[ch]), __uint_as_float(r32[ch + 1])),
+                           gelu_grad2(make_float2(zv[e], zv[e + 1]))));
           }
         }
         __syncwarp();
@@ -1980,7 +1951,6 @@ __global__ void __launch_bounds__(kTThreads, 2)
         if (cl >= 0) reinterpret_cast<uint4*>(out + cl * C)[ch] = v;
       }
       __syncwarp();
-      slot ^= 1;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next tile's copies
     tc_fence_before();
@@ -2001,20 +1971,6 @@ __global__ void __launch_bounds__(kTThreads, 2)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTTmemCols)
                  : "memory");
-  }
-  if (BWD) {
-    // Per-channel sums of this CTA's dz1 in a fixed order: thread sums in the region area (free
-    // now; rows padded to C + 1 against bank conflicts), then channel c adds the 256 threads'
-    // values in thread order.
-    float* sums = reinterpret_cast<float*>(ac);  // [kTThreads][C + 1]
-#pragma unroll
-    for (int c = 0; c < C; ++c) sums[threadIdx.x * (C + 1) + c] = bias_sum[c];
-    __syncthreads();
-    if (threadIdx.x < C) {
-      float s = 0.0f;
-      for (int k = 0; k < kTThreads; ++k) s += sums[k * (C + 1) + threadIdx.x];
-      partial[(int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_B1 + threadIdx.x] = s;
-    }
   }
 }
 
@@ -2219,15 +2175,15 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
   CUtensorMap a1_map;
   if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_input_map(&a1_map, a1, nx, ny, batch)) {
     const Grid gt = tc_grid(nx, ny, batch);
-    const int grid_tc = (int)std::min<int64_t>(gt.tiles, (int64_t)sms * 2);
+    const int grid_tc = (int)std::min<int64_t>(gt.tiles, (int64_t)sms * kTPerSm);
     conv32_tc_kernel<false><<<grid_tc, kTThreads, kTSmem, s>>>(
         gt, a1_map, wb + LBM_CLOSURE_OFF_W2, params + LBM_CLOSURE_OFF_B2, nullptr, z2,
-        reinterpret_cast<bf16*>(a2), nullptr);
+        reinterpret_cast<bf16*>(a2));
   } else {
     const int grid32 = (int)std::min<int64_t>(g.tiles, (int64_t)sms * 4);
     conv32_kernel<false><<<grid32, kConv32Threads, kConv32Smem, s>>>(
         g, reinterpret_cast<const bf16*>(a1), wb + LBM_CLOSURE_OFF_W2,
-        params + LBM_CLOSURE_OFF_B2, nullptr, z2, reinterpret_cast<bf16*>(a2), nullptr);
+        params + LBM_CLOSURE_OFF_B2, nullptr, z2, reinterpret_cast<bf16*>(a2));
   }
   CL_CUDA(cudaGetLastError());
   const Grid g3 = tiles_of(nx, ny, batch, kC3R, kTY);
@@ -2294,7 +2250,6 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   const auto* wb = reinterpret_cast<const bf16*>(params_bf16);
   const int rows = (int)std::min<int64_t>(g.tiles, kPartialRows);
   const int rows_w2 = (int)std::min<int64_t>(rows, device_sms());
-
   conv3_bwd_kernel<<<rows, kB3Threads, kConv3BwdSmem, s>>>(g, reinterpret_cast<const bf16*>(a2), z2,
                                                     wb + LBM_CLOSURE_OFF_W3, dy, dz2, partial);
   CL_CUDA(cudaGetLastError());
@@ -2303,14 +2258,13 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   CL_CUDA(cudaGetLastError());
   CUtensorMap dz2_map;
   if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_input_map(&dz2_map, dz2, nx, ny, batch)) {
-    // Same number of CTAs (partial rows) as the other reducing kernels: a CTA without a tile
-    // writes a zero row.
-    conv32_tc_kernel<true><<<rows, kTThreads, kTSmem, s>>>(
-        tc_grid(nx, ny, batch), dz2_map, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1,
-        partial);
+    const Grid gt = tc_grid(nx, ny, batch);
+    const int ctas = (int)std::min<int64_t>(gt.tiles, (int64_t)device_sms() * kTPerSm);
+    conv32_tc_kernel<true><<<ctas, kTThreads, kTSmem, s>>>(
+        gt, dz2_map, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1);
   } else {
     conv32_kernel<true><<<rows, kConv32Threads, kConv32Smem, s>>>(
-        g, dz2, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1, partial);
+        g, dz2, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1);
   }
   CL_CUDA(cudaGetLastError());
   conv1_wgrad_kernel<<<rows, kW1Threads, kW1Smem, s>>>(

@@ -1,4 +1,4 @@
-"""The closure's training kernels at the edges of their tiles (4 x 64, 14 x 64 and 30 x 64 cells):
+"""The closure's training kernels at the edges of their tiles (4 x 64, 14 x 32 and 30 x 64 cells):
 one cell short of a tile, one past it, smaller than any, several samples; the same checks and
 bounds against the float64 oracle as for the ordinary shapes."""
 
@@ -13,7 +13,8 @@ from tests.test_gpu_closure import cl, torch  # noqa: F401  (fixtures)
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(1, 2, 2), (2, 3, 63), (1, 29, 65), (1, 31, 64), (2, 13, 66), (1, 15, 129), (1, 61, 7)]
+SHAPES = [(1, 2, 2), (2, 3, 63), (1, 29, 65), (1, 31, 64), (2, 13, 66), (1, 15, 129), (1, 61, 7),
+          (1, 14, 33), (2, 29, 31)]
 
 
 @pytest.mark.parametrize("B,nx,ny", SHAPES)
