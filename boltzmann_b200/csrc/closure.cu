@@ -7,7 +7,7 @@
 //   layer   forward                       backward
 //   1 (4->32)   CUDA cores (36 MAC/out)    weights: mma.sync; no input gradient
 //   2 (32->32)  tcgen05 BF16, FP32 acc     data: tcgen05 (transposed conv, fused GELU');
-//               (TMEM accumulators)        weights: mma.sync (cells are the reduction axis)
+//               (TMEM accumulators)        weights: tcgen05 (cells are the reduction axis)
 //               mma.sync kept selectable (lbm_closure_set_layer2_kernel)
 //   3 (32->1)   CUDA cores                 data: CUDA cores (fused GELU'); weights: mma.sync, dy
 //                                          as the exact sum of three BF16 parts
@@ -587,7 +587,8 @@ __global__ void __launch_bounds__(kConv32Threads)
 // tiles, 16 per k-step. Warp (i, dx) takes tile row i and the three taps (dx, -1 .. 1): the dz
 // fragments it loads serve 24 MMAs (one warp a tap loaded them for eight). The next tile's operands
 // arrive (asynchronous copies) while this one's are multiplied. Bound by shared-memory reads (eight
-// ldmatrix a 24 MMAs). Batch 8 x 1024 x 512: 366 -> 311 us.
+// ldmatrix a 24 MMAs). Batch 8 x 1024 x 512: 366 -> 311 us. Runs with the warp-level layer-2 kernels,
+// and where conv32_wgrad_tc_kernel (118 us) has no tensor map.
 
 constexpr int kDw2Threads = 3 * kTX * 32;
 constexpr int kDw2Stage = (kTX * kTY + kHX * kHY) * kCS;  // BF16 elements of one stage
@@ -1974,9 +1975,190 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Layer-2 weight gradient on tcgen05: dW[co][tap][ci] = sum_p dz[p][co] a1[p + tap][ci], the products
+// of conv32_wgrad_kernel. The cells are the contraction (K), so both operands lie as they do in
+// memory, 32 channels (64 bytes, swizzled) a cell: M and N are the contiguous directions. One product
+// of 128 x 96 x 16 serves all nine taps of 16 cells of a1 row i:
+//   - M = (r, co): the rows i - 1 + r of dz, r = 0 .. 2, which lie one behind the other in shared
+//     memory (the stride between groups of 32 rows of A is a row of the tile). r = 3 is what M = 128
+//     adds; its results are dropped, so it may read anything;
+//   - N = (d, ci): three copies of the a1 row, shifted by d - 1 cells by the tensor engine.
+// Cells outside the domain read as zero. Warp 4 copies (a ring of kDtStages tiles), warp 3 issues,
+// warps 0 .. 2 (r) add each tile's accumulators to running sums in registers while the next tile's
+// products go to the other half of tensor memory: a chain in the truncating accumulators ends with
+// its tile.
+// Bound by the copies: 128 bytes a cell of DRAM traffic take 83 us over batch 8 x 1024 x 512, and
+// 288 bytes a cell come out of L2. 118 us, where conv32_wgrad_kernel, at the rate of mma.sync, takes
+// 311; the gradient is 2.1e-7 off its float64 sums at any batch, 6.8e-6 there.
+
+constexpr int kDtThreads = 160;
+constexpr int kDtStages = 3;
+constexpr unsigned kDtRow = kTY * C * 2;               // bytes of a tile row of 64 cells
+constexpr unsigned kDtDz = kHX * kDtRow;               // dz rows -1 .. kTX
+constexpr unsigned kDtCopy = kTX * kDtRow;             // one shifted copy of the a1 rows
+constexpr unsigned kDtStage = kDtDz + 3 * kDtCopy;
+constexpr size_t kDtOffBar = (size_t)kDtStages * kDtStage;
+constexpr int kDtBars = 2 * kDtStages + 5;             // full, empty; done[2], read[2]; drained
+constexpr size_t kDtSmem = kDtOffBar + kDtBars * 8 + 16 + 1024;  // the stages start on 1 KB
+constexpr int kDtTmemCols = 256;                       // two accumulators of 96 columns, 128 apart
+static_assert(kTX + 3 <= kHX + 3 * kTX, "the dropped rows stay inside the stage");
+
+__device__ __forceinline__ void tc_rows_copy(void* dst, const CUtensorMap* map, int y, int x, int b,
+                                             uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(x), "r"(b), "r"(smem_addr(bar))
+      : "memory");
+}
+
+__device__ __forceinline__ void cl_mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+__global__ void __launch_bounds__(kDtThreads, 1)
+    conv32_wgrad_tc_kernel(Grid g, const __grid_constant__ CUtensorMap dz_map,
+                           const __grid_constant__ CUtensorMap a1_map,
+                           float* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + kDtOffBar);
+  uint64_t* empty = full + kDtStages;
+  uint64_t* done = empty + kDtStages;
+  uint64_t* read = done + 2;
+  uint64_t* drained = read + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < kDtStages; ++k) cl_mbar_init(full + k, 1), cl_mbar_init(empty + k, 1);
+    for (int k = 0; k < 2; ++k) cl_mbar_init(done + k, 1), cl_mbar_init(read + k, 3);
+    cl_mbar_init(drained, 1);
+    *stop = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_addr(tmem_slot)),
+                 "r"(kDtTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const unsigned spin_limit = g_closure_spin_limit;
+  // Bounded wait that also ends when another warp has given up; whoever gives up stops the rest.
+  auto wait = [&](uint64_t* bar, unsigned parity, unsigned limit) {
+    constexpr unsigned kPolls = 64;
+    for (unsigned k = 0; k < limit; k += kPolls) {
+      if (cl_mbar_wait(bar, parity, kPolls)) return true;
+      if (*stop) return false;
+    }
+    *stop = 1;
+    return false;
+  };
+
+  float acc[3][C];  // warps 0 .. 2: row co = lane of tap row 2 - warp, columns (d, ci)
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int k = 0; k < C; ++k) acc[d][k] = 0.0f;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      unsigned n = 0;
+      for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
+        const unsigned s = n % kDtStages, lap = n / kDtStages;
+        if (lap > 0 && !wait(empty + s, (lap - 1) & 1u, kClosureSpinLimit)) break;
+        int64_t b, x0, y0;
+        g.tile(t, b, x0, y0);
+        unsigned char* st = base + (size_t)s * kDtStage;
+        tc_expect_tx(full + s, kDtStage);
+        tc_rows_copy(st, &dz_map, (int)y0, (int)x0 - 1, (int)b, full + s);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          tc_rows_copy(st + kDtDz + d * kDtCopy, &a1_map, (int)y0 + d - 1, (int)x0, (int)b, full + s);
+      }
+      // Every copy has landed before the CTA ends, whoever gave up.
+      for (unsigned k = n > kDtStages ? n - kDtStages : 0; k < n; ++k)
+        cl_mbar_wait(full + k % kDtStages, (k / kDtStages) & 1u);
+    }
+  } else if (warp == 3) {
+    if (lane == 0) {
+      // Both operands with M / N contiguous (bits 15 and 16) and rows of 64 bytes, swizzled (4 at
+      // bit 61): the descriptor's strides are between groups of 32 of M or N and between groups of
+      // eight cells.
+      const uint32_t idesc = umma_idesc_bf16(128, 96) | (1u << 15) | (1u << 16);
+      const uint64_t swizzle = 4ull << 61;
+      unsigned n = 0;
+      for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
+        const unsigned s = n % kDtStages, h = n & 1u;
+        if (!wait(full + s, (n / kDtStages) & 1u, kClosureSpinLimit)) break;
+        if (n >= 2 && !wait(read + h, (n / 2 - 1) & 1u, kClosureSpinLimit)) break;
+        tc_fence_after();
+        const unsigned dz = smem_addr(base) + s * kDtStage, a = dz + kDtDz;
+#pragma unroll
+        for (int i = 0; i < kTX; ++i)
+#pragma unroll
+          for (int k = 0; k < kTY / 16; ++k) {
+            const unsigned off = i * kDtRow + k * 16 * C * 2;
+            umma_bf16(tmem + h * 128, umma_desc(dz + off, kDtRow, 8 * C * 2) | swizzle,
+                      umma_desc(a + off, kDtCopy, 8 * C * 2) | swizzle, idesc, i + k != 0);
+          }
+        umma_commit(empty + s);
+        umma_commit(done + h);
+      }
+      umma_commit(drained);  // before tensor memory is given back
+      cl_mbar_wait(drained, 0);
+    }
+  } else {
+    unsigned n = 0;
+    for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
+      const unsigned h = n & 1u;
+      if (!__all_sync(0xffffffffu, wait(done + h, (n / 2) & 1u, spin_limit))) {
+        *stop = 1;
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        uint32_t v[32];
+        tmem_ld32(tmem + h * 128 + ((uint32_t)(warp * 32) << 16) + d * 32, v);
+#pragma unroll
+        for (int k = 0; k < C; ++k) acc[d][k] += __uint_as_float(v[k]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) cl_mbar_arrive(read + h);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kDtTmemCols)
+                 : "memory");
+  }
+  if (*stop && threadIdx.x == 0) atomicOr(&g_closure_status, 1);
+  if (warp < 3) {
+    float* row = partial + (int64_t)blockIdx.x * LBM_CLOSURE_PARAMS + LBM_CLOSURE_OFF_W2 +
+                 lane * 288 + (2 - warp) * 3 * C;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int k = 0; k < C; ++k) row[d * C + k] = acc[d][k];
+  }
+}
+
 // The [batch][nx][ny][32] BF16 activations as conv32_tc_kernel's 5D tensor map (through the
 // runtime's driver entry point: no link against libcuda). False when it cannot be encoded.
-bool tc_input_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch) {
+PFN_cuTensorMapEncodeTiled_v12000 tc_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q{};
@@ -1986,15 +2168,38 @@ bool tc_input_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, in
       return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
   }();
-  if (encode == nullptr || (reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
-  if (nx >= (1ll << 31) || ny >= (1ll << 31) || batch >= (1ll << 31)) return false;
+  return encode;
+}
+
+bool tc_mappable(const void* base, int64_t nx, int64_t ny, int64_t batch) {
+  return tc_encoder() != nullptr && (reinterpret_cast<uintptr_t>(base) & 15) == 0 &&
+         nx < (1ll << 31) && ny < (1ll << 31) && batch < (1ll << 31);
+}
+
+bool tc_input_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch) {
+  if (!tc_mappable(base, nx, ny, batch)) return false;
   const cuuint64_t dims[5] = {8, 4, (cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)batch};
   const cuuint64_t strides[4] = {16, 64, (cuuint64_t)ny * 64, (cuuint64_t)(nx * ny) * 64};
   const cuuint32_t box[5] = {8, 1, (cuuint32_t)kTRegC, (cuuint32_t)kTRegR, 1};
   const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides,
-                box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return tc_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims,
+                      strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same activations for conv32_wgrad_tc_kernel: boxes of `rows` x kTY whole cells.
+bool tc_rows_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch,
+                 int rows) {
+  if (!tc_mappable(base, nx, ny, batch)) return false;
+  const cuuint64_t dims[4] = {C, (cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {64, (cuuint64_t)ny * 64, (cuuint64_t)(nx * ny) * 64};
+  const cuuint32_t box[4] = {C, (cuuint32_t)kTY, (cuuint32_t)rows, 1};
+  const cuuint32_t elem[4] = {1, 1, 1, 1};
+  return tc_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims,
+                      strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Tiles of kTR x kTC cells for conv32_tc_kernel.
@@ -2236,6 +2441,7 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
     if (int rc = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return rc;
     if (int rc = set_smem((const void*)conv32_tc_kernel<true>, kTSmem)) return rc;
     if (int rc = set_smem((const void*)conv32_wgrad_kernel, kDw2Smem)) return rc;
+    if (int rc = set_smem((const void*)conv32_wgrad_tc_kernel, kDtSmem)) return rc;
     if (int rc = set_smem((const void*)conv3_bwd_kernel, kConv3BwdSmem)) return rc;
     if (int rc = set_smem((const void*)conv1_wgrad_kernel, kW1Smem)) return rc;
     configured = true;
@@ -2253,8 +2459,15 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   conv3_bwd_kernel<<<rows, kB3Threads, kConv3BwdSmem, s>>>(g, reinterpret_cast<const bf16*>(a2), z2,
                                                     wb + LBM_CLOSURE_OFF_W3, dy, dz2, partial);
   CL_CUDA(cudaGetLastError());
-  conv32_wgrad_kernel<<<rows_w2, kDw2Threads, kDw2Smem, s>>>(g, reinterpret_cast<const bf16*>(a1),
-                                                          dz2, partial);
+  CUtensorMap dz2_rows, a1_rows;
+  if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 &&
+      tc_rows_map(&dz2_rows, dz2, nx, ny, batch, kHX) &&
+      tc_rows_map(&a1_rows, a1, nx, ny, batch, kTX)) {
+    conv32_wgrad_tc_kernel<<<rows_w2, kDtThreads, kDtSmem, s>>>(g, dz2_rows, a1_rows, partial);
+  } else {
+    conv32_wgrad_kernel<<<rows_w2, kDw2Threads, kDw2Smem, s>>>(g, reinterpret_cast<const bf16*>(a1),
+                                                            dz2, partial);
+  }
   CL_CUDA(cudaGetLastError());
   CUtensorMap dz2_map;
   if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_input_map(&dz2_map, dz2, nx, ny, batch)) {
