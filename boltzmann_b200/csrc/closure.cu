@@ -1324,6 +1324,23 @@ __device__ __forceinline__ bool cl_mbar_wait(uint64_t* bar, unsigned parity,
   return false;
 }
 
+__device__ __forceinline__ void cl_mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// Bounded wait that also ends when another warp of the CTA has given up; whoever gives up stops the
+// rest.
+__device__ __forceinline__ bool cl_mbar_wait_or_stop(uint64_t* bar, unsigned parity, unsigned limit,
+                                                     volatile int* stop) {
+  constexpr unsigned kPolls = 64;
+  for (unsigned k = 0; k < limit; k += kPolls) {
+    if (cl_mbar_wait(bar, parity, kPolls)) return true;
+    if (*stop) return false;
+  }
+  *stop = 1;
+  return false;
+}
+
 // Set (bit 0) when a closure kernel gave up waiting for its tensor-core work; read and cleared
 // by lbm_closure_status.
 __device__ int g_closure_status;
@@ -1696,57 +1713,42 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 // Layer 2 of the training path on tcgen05: the forward conv (BWD = false: z2 = b2 + W * a1,
 // a2 = GELU(z2) in BF16) and the transposed conv of the backward pass (BWD = true:
 // d = W^T * dz2, dz1 = BF16(d GELU'(z1))). Same products as conv32_kernel, on the fifth-generation
-// tensor cores with the layout of the fused inference kernel's layer 2:
-//   - a tile of kTR x kTC output cells reads a (kTR + 2) x (kTC + 2) input region, staged
-//     chunk-major: plane k (channels 8k .. 8k+7) holds 16 bytes a cell, cells in row-major order
-//     of the region, so a tap shift (dx, dy) of the 3x3 stencil is an offset of the descriptor's
-//     start address, dx (kTC + 2) + dy cells (the negated shift for the transposed conv);
-//   - kTBlocks blocks of 128 consecutive region cells starting at output cell (0, 0), each an
-//     M = 128, N = 32, K = 288 product into its own 32 TMEM columns; rows that fall on the
-//     region's first or last column are computed and discarded;
+// tensor cores:
+//   - the input of a tile of kTR x kTC output cells is three copies of kTR + 2 rows of kTC cells,
+//     shifted by -1, 0 and 1 cells along the row by the tensor engine (zero outside the domain),
+//     64 bytes a cell, swizzled: a tap (dx, dy) of the 3x3 stencil reads copy dy + 1 from row
+//     1 + dx on (both negated for the transposed conv), and a row's 2 KB keep the swizzle's phase;
+//   - kTBlocks blocks of 128 consecutive cells, each an M = 128, N = 32, K = 288 product into its
+//     own 32 TMEM columns;
 //   - the B operand is the weights as K-chunks of 8: [k chunk][n][8] with k = (tap, ci) and
 //     n = co for the forward conv, k = (tap, co) and n = ci for the transposed one.
-// One thread issues the MMAs and commits them to an mbarrier (bounded wait, as everywhere); the
-// epilogue reads each cell's 32 accumulators with tcgen05.ld. Three CTAs share an SM, so one stages
-// its next tile while the others' MMAs and epilogues run: a chain of waits, longer than what the
-// memory (260 bytes a cell) takes. Tiles of 14 x 32 cells with one 4 KB slot a warp are what lets a
-// third CTA in; with 14 x 64, two slots and two CTAs, the two kernels took 308 and 300 us over
-// batch 8 x 1024 x 512, now 291 and 276.
+// One warp copies (a ring of kTStages tiles), one issues the products, and two groups of eight warps
+// take the tiles in turn in the epilogue, which reads each cell's 32 accumulators with tcgen05.ld.
+// Bound by shared memory (the products read A anew for each tap: 720 bytes a cell, of 1300 in all)
+// close to DRAM (256 bytes a cell, 166 us over batch 8 x 1024 x 512): 241 us forward and 232 us
+// backward there. Before, one region with a halo, 16 bytes a cell and plane, served all taps by the
+// start address: copies of 16-byte rows kept the tensor engine busy for 275 us whatever ran beside
+// them, and with copies, products and epilogue in turn in three CTAs an SM it took 290 and 278 us.
 
-constexpr int kTR = 14, kTC = 32;                  // output tile
-constexpr int kTRegR = kTR + 2, kTRegC = kTC + 2;  // input region
-constexpr int kTFirst = kTRegC + 1;                // region index of output cell (0, 0)
-constexpr int kTBlocks = (kTR * kTRegC + 127) / 128;  // 128-cell blocks covering the output rows
-constexpr int kTPad = 584;  // cells per plane: >= kTFirst + 128 kTBlocks + kTRegC + 1, and a
-                            // multiple of 8 so that every plane starts on a 128-byte boundary
-constexpr int kTThreads = 256;
-constexpr int kTTmemCols = 128;  // 4 accumulators of 32 FP32 columns
-constexpr int kTPerSm = 3;
-constexpr size_t kTOffW = (size_t)4 * kTPad * 16;
-constexpr size_t kTOffBias = kTOffW + (size_t)36 * C * 16;
-constexpr size_t kTOffBar = kTOffBias + (size_t)C * 4;  // MMA mbarrier, load mbarrier, TMEM addr
-constexpr size_t kTSmem = kTOffBar + 24;
-constexpr int kTStageBytes = 32 * 128;  // a warp's rows in the epilogue
-static_assert((size_t)(kTThreads / 32) * kTStageBytes <= kTOffW, "the epilogue's rows must fit");
-constexpr unsigned kTLoadBytes = 4u * kTRegR * kTRegC * 16;  // the four plane boxes of a tile
-static_assert(kTBlocks * 32 <= kTTmemCols, "accumulators exceed the TMEM allocation");
-static_assert(kTFirst + kTBlocks * 128 + kTRegC + 1 <= kTPad, "planes too short for the shifts");
-static_assert(kTFirst + kTBlocks * 128 - 1 >= (kTR * kTRegC) + kTC, "blocks do not cover the tile");
-static_assert(kTFirst - kTRegC - 1 >= 0, "a negative shift leaves the plane");
-
-// One plane of a tile's input region by the tensor engine: the activations as a 5D tensor
-// (8 channels, 4 channel chunks, y, x, batch), box {8, 1, kTRegC, kTRegR, 1} at (0, chunk,
-// y0 - 1, x0 - 1, b), which lands as kTRegR x kTRegC cells of 16 bytes in row-major order;
-// cells outside the domain read as zero (the box may start at -1).
-__device__ __forceinline__ void tc_plane_copy(void* dst, const CUtensorMap* map, int chunk, int y,
-                                              int x, int b, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], "
-      "[%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(chunk), "r"(y), "r"(x), "r"(b),
-      "r"(smem_addr(bar))
-      : "memory");
-}
+constexpr int kTR = 8, kTC = 32;                    // output tile
+constexpr int kTBlocks = kTR * kTC / 128;           // 128-cell blocks
+constexpr int kTGroup = 4 * kTBlocks;               // epilogue warps of a tile
+constexpr int kTEpilogue = 2 * kTGroup;             // warps of the epilogue
+constexpr int kTThreads = (kTEpilogue + 2) * 32;    // and one each for the copies and the products
+constexpr int kTStages = 2;
+constexpr int kTTmemCols = 2 * kTBlocks * 32;       // two tiles' accumulators of 32 FP32 columns
+constexpr unsigned kTRow = kTC * C * 2;             // bytes of a row of cells
+constexpr unsigned kTCopy = (kTR + 2) * kTRow;      // one shifted copy
+constexpr unsigned kTStage = 3 * kTCopy;
+constexpr size_t kTOffW = (size_t)kTStages * kTStage;
+constexpr size_t kTOffRows = kTOffW + (size_t)36 * C * 16;
+constexpr int kTStageBytes = 32 * 128;              // an epilogue warp's rows
+constexpr size_t kTOffBias = kTOffRows + (size_t)kTEpilogue * kTStageBytes;
+constexpr size_t kTOffBar = kTOffBias + (size_t)C * 4;
+constexpr int kTBars = 2 * kTStages + 5;            // full, empty; done[2], read[2]; drained
+constexpr size_t kTSmem = kTOffBar + kTBars * 8 + 8 + 1024;  // the stages start on 1 KB
+static_assert(kTR * kTC == kTBlocks * 128 && (kTTmemCols & (kTTmemCols - 1)) == 0, "whole blocks");
+static_assert(kTRow % 512 == 0, "a row keeps the swizzle's phase");
 
 __device__ __forceinline__ void tc_expect_tx(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
@@ -1754,21 +1756,38 @@ __device__ __forceinline__ void tc_expect_tx(uint64_t* bar, unsigned bytes) {
                : "memory");
 }
 
+// A box of whole cells of the activations (tc_rows_map) at row x, column y of sample b; cells outside
+// the domain read as zero.
+__device__ __forceinline__ void tc_rows_copy(void* dst, const CUtensorMap* map, int y, int x, int b,
+                                             uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(x), "r"(b), "r"(smem_addr(bar))
+      : "memory");
+}
+
+// For umma_desc: rows of 64 bytes, swizzled.
+constexpr uint64_t kSwizzle64 = 4ull << 61;
+
 template <bool BWD>
-__global__ void __launch_bounds__(kTThreads, kTPerSm)
+__global__ void __launch_bounds__(kTThreads, 1)
     conv32_tc_kernel(Grid g, const __grid_constant__ CUtensorMap in_map,
                      const bf16* __restrict__ w2, const float* __restrict__ bias,
                      const float* __restrict__ zin, float* __restrict__ zout,
                      bf16* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned char* ac = smem_raw;                    // [4 planes][kTPad cells][16 B]
-  unsigned char* wc = smem_raw + kTOffW;           // [36 K-chunks][32 n][16 B]
-  float* bs = reinterpret_cast<float*>(smem_raw + kTOffBias);  // forward: b2
-  uint64_t* mma_done = reinterpret_cast<uint64_t*>(smem_raw + kTOffBar);
-  uint64_t* loaded = reinterpret_cast<uint64_t*>(smem_raw + kTOffBar + 8);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + kTOffBar + 16);
+  unsigned char* base = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
+  unsigned char* wc = base + kTOffW;                // [36 K-chunks][32 n][16 B]
+  float* bs = reinterpret_cast<float*>(base + kTOffBias);  // forward: b2
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + kTOffBar);
+  uint64_t* empty = full + kTStages;
+  uint64_t* done = empty + kTStages;
+  uint64_t* read = done + 2;
+  uint64_t* drained = read + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kWarps = kTThreads / 32;
 
   // The B operand. Forward: chunk kk = (tap, ci chunk) of output channel co, 8 consecutive
   // weights of the [co][288] row. Transposed: chunk kk = (tap, co chunk) of input channel ci,
@@ -1787,12 +1806,13 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
     }
   }
   if (!BWD && threadIdx.x < C) bs[threadIdx.x] = bias[threadIdx.x];
-  // (Plane cells past the region, whatever they hold, feed only discarded rows.)
   // The weights, written here, are read by the MMAs (async proxy).
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (threadIdx.x == 0) {
-    cl_mbar_init(mma_done, 1);
-    cl_mbar_init(loaded, 1);
+    for (int k = 0; k < kTStages; ++k) cl_mbar_init(full + k, 1), cl_mbar_init(empty + k, 1);
+    for (int k = 0; k < 2; ++k) cl_mbar_init(done + k, 1), cl_mbar_init(read + k, kTGroup);
+    cl_mbar_init(drained, 1);
+    *stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -1806,81 +1826,84 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = umma_idesc_bf16(128, 32);
-  const unsigned ac_addr = smem_addr(ac), wc_addr = smem_addr(wc);
   const unsigned spin_limit = g_closure_spin_limit;
-  bool healthy = true;
-  unsigned phase = 0, load_phase = 0;
+  auto wait = [&](uint64_t* bar, unsigned parity, unsigned limit) {
+    return cl_mbar_wait_or_stop(bar, parity, limit, stop);
+  };
+  auto tile_of = [&](int64_t t, int64_t& b, int64_t& x0, int64_t& y0) {
+    const int64_t per = g.tx * g.ty;  // this kernel's tiles are kTR x kTC (see the launcher)
+    b = t / per;
+    const int64_t r = t - b * per;
+    x0 = (r / g.ty) * kTR;
+    y0 = (r % g.ty) * kTC;
+  };
 
-  for (int64_t t = blockIdx.x; t < g.tiles && healthy; t += gridDim.x) {
-    int64_t b, x0, y0;
-    {
-      const int64_t per = g.tx * g.ty;  // this kernel's tiles are kTR x kTC (see the launcher)
-      b = t / per;
-      const int64_t r = t - b * per;
-      x0 = (r / g.ty) * kTR;
-      y0 = (r % g.ty) * kTC;
-    }
-    // The input region, chunk-major, by four tensor copies (zero outside the domain).
-    if (threadIdx.x == 0) {
-      tc_expect_tx(loaded, kTLoadBytes);
+  if (warp == kTEpilogue) {
+    if (lane == 0) {
+      unsigned n = 0;
+      for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
+        const unsigned s = n % kTStages, lap = n / kTStages;
+        if (lap > 0 && !wait(empty + s, (lap - 1) & 1u, kClosureSpinLimit)) break;
+        int64_t b, x0, y0;
+        tile_of(t, b, x0, y0);
+        tc_expect_tx(full + s, kTStage);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        tc_plane_copy(ac + (size_t)k * kTPad * 16, &in_map, k, (int)y0 - 1, (int)x0 - 1, (int)b,
-                      loaded);
-    }
-    const bool have = cl_mbar_wait(loaded, load_phase);  // the copies take no spin limit: the
-    load_phase ^= 1u;                                     // tile's MMAs need them
-    if (!__syncthreads_and(have)) {
-      healthy = false;
-      break;
-    }
-    if (threadIdx.x == 0) {
-      tc_fence_after();
-      // K-slice outer, block inner: consecutive MMAs accumulate into different TMEM columns.
-#pragma unroll 1
-      for (int tap = 0; tap < 9; ++tap) {
-        const int sh = (tap / 3 - 1) * kTRegC + (tap % 3 - 1);
-        const int off = BWD ? -sh : sh;
-#pragma unroll
-        for (int kc = 0; kc < 2; ++kc) {
-          const int sidx = tap * 2 + kc;
-          const uint64_t bdesc = umma_desc(wc_addr + (unsigned)(sidx * 1024), C * 16, 128);
-          const unsigned a_base = ac_addr + (unsigned)((2 * kc * kTPad + kTFirst + off) * 16);
-#pragma unroll
-          for (int m = 0; m < kTBlocks; ++m)
-            umma_bf16(tmem + (uint32_t)(m * 32),
-                      umma_desc(a_base + (unsigned)(m * 128 * 16), kTPad * 16, 128), bdesc, idesc,
-                      sidx != 0);
-        }
+        for (int d = 0; d < 3; ++d)
+          tc_rows_copy(base + s * kTStage + d * kTCopy, &in_map, (int)y0 + d - 1, (int)x0 - 1, (int)b,
+                       full + s);
       }
-      umma_commit(mma_done);
+      // Every copy has landed before the CTA ends, whoever gave up.
+      for (unsigned k = n > kTStages ? n - kTStages : 0; k < n; ++k)
+        cl_mbar_wait(full + k % kTStages, (k / kTStages) & 1u);
     }
-    const bool got = cl_mbar_wait(mma_done, phase, spin_limit);
-    phase ^= 1u;
-    if (!__syncthreads_and(got)) {
-      healthy = false;
-      break;
+  } else if (warp == kTEpilogue + 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16(128, 32);
+      const unsigned wc_addr = smem_addr(wc);
+      unsigned n = 0;
+      for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
+        const unsigned s = n % kTStages, h = n & 1u;
+        if (!wait(full + s, (n / kTStages) & 1u, kClosureSpinLimit)) break;
+        if (n >= 2 && !wait(read + h, (n / 2 - 1) & 1u, kClosureSpinLimit)) break;
+        tc_fence_after();
+        const unsigned in_addr = smem_addr(base) + s * kTStage;
+        // K-slice outer, block inner: consecutive MMAs accumulate into different TMEM columns.
+#pragma unroll 1
+        for (int tap = 0; tap < 9; ++tap) {
+          const int dx = BWD ? 1 - tap / 3 : tap / 3 - 1, d = BWD ? 2 - tap % 3 : tap % 3;
+#pragma unroll
+          for (int kc = 0; kc < 2; ++kc) {
+            const int sidx = tap * 2 + kc;
+            const uint64_t bdesc = umma_desc(wc_addr + (unsigned)(sidx * 1024), C * 16, 128);
+            const unsigned a_base = in_addr + d * kTCopy + (1 + dx) * kTRow + kc * 32;
+#pragma unroll
+            for (int m = 0; m < kTBlocks; ++m)
+              umma_bf16(tmem + h * (kTBlocks * 32) + (uint32_t)(m * 32),
+                        umma_desc(a_base + (unsigned)(m * 128 * C * 2), 16, 8 * C * 2) | kSwizzle64,
+                        bdesc, idesc, sidx != 0);
+          }
+        }
+        umma_commit(empty + s);
+        umma_commit(done + h);
+      }
+      umma_commit(drained);  // before tensor memory is given back
+      cl_mbar_wait(drained, 0);
     }
-    tc_fence_after();
-    // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition) of blocks
-    // w / 4, w / 4 + 2, ...; one thread per cell, its 32 channels in registers. Rows of cells pass
-    // through shared memory (the region's, whose operands the MMAs have read), so that global
-    // accesses are whole 128-byte lines: a lane's own row of 128 bytes at a time is a quarter of
-    // that. Chunk c of the row of lane l lies at chunk c ^ (l % 8).
-    const int sp = warp & 3;
-    unsigned char* buf = ac + warp * kTStageBytes;  // this warp's 32 rows x 128 bytes
-    auto cell_of = [&](int m, int64_t& cell) {      // block m's cell of this lane, or -1
-      const int q = kTFirst + 128 * m + 32 * sp + lane;  // region index of this row
-      const int r = q / kTRegC - 1, c = q % kTRegC - 1;   // output tile coordinates
-      const int64_t x = x0 + r, y = y0 + c;
-      const bool ok = r >= 0 && r < kTR && c >= 0 && c < kTC && x < g.nx && y < g.ny;
-      cell = ok ? g.cell(b, x, y) : -1;
-    };
-    for (int m = warp >> 2; m < kTBlocks; m += kWarps / 4) {
-      int64_t cell;
-      cell_of(m, cell);
-      if (BWD) {  // this block's rows of z1
+  } else {
+    // Epilogue: warp w of a group reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition) of block
+    // w / 4; one thread per cell, its 32 channels in registers. Rows of cells pass through shared
+    // memory, so that global accesses are whole 128-byte lines: a lane's own row of 128 bytes at a
+    // time is a quarter of that. Chunk c of the row of lane l lies at chunk c ^ (l % 8).
+    const unsigned h = warp / kTGroup;  // tiles h, h + 2, ... of this CTA
+    const int sp = warp & 3, m = (warp % kTGroup) >> 2;
+    unsigned char* buf = base + kTOffRows + warp * kTStageBytes;  // 32 rows x 128 bytes
+    const int q = 128 * m + 32 * sp + lane, r = q / kTC, c = q % kTC;  // this lane's cell of a tile
+    unsigned n = h;
+    for (int64_t t = blockIdx.x + (int64_t)h * gridDim.x; t < g.tiles; t += 2 * gridDim.x, n += 2) {
+      int64_t b, x0, y0;
+      tile_of(t, b, x0, y0);
+      const int64_t cell = x0 + r < g.nx && y0 + c < g.ny ? g.cell(b, x0 + r, y0 + c) : -1;
+      if (BWD) {  // this block's rows of z1, while its products are computed
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int l = 4 * k + (lane >> 3), ch = lane & 7;
@@ -1890,8 +1913,16 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
         }
         cp_async_commit();
       }
+      if (!__all_sync(0xffffffffu, wait(done + h, (n / 2) & 1u, spin_limit))) {
+        *stop = 1;
+        break;
+      }
+      tc_fence_after();
       uint32_t r32[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
+      tmem_ld32(tmem + h * (kTBlocks * 32) + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) cl_mbar_arrive(read + h);
       if (BWD) {
         cp_async_wait<0>();
         __syncwarp();
@@ -1953,18 +1984,9 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
       }
       __syncwarp();
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next tile's copies
-    tc_fence_before();
-    __syncthreads();  // the region and every TMEM column are free for the next tile
+    if (BWD) cp_async_wait<0>();
   }
-  if (!healthy) {
-    if (threadIdx.x == 0) {
-      atomicOr(&g_closure_status, 1);
-      // Give the copies and MMAs still in flight a bounded chance to end.
-      cl_mbar_wait(loaded, load_phase ^ 1u);
-      cl_mbar_wait(mma_done, phase ^ 1u);
-    }
-  }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -1973,6 +1995,7 @@ __global__ void __launch_bounds__(kTThreads, kTPerSm)
                  "r"(kTTmemCols)
                  : "memory");
   }
+  if (*stop && threadIdx.x == 0) atomicOr(&g_closure_status, 1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2003,19 +2026,6 @@ constexpr int kDtBars = 2 * kDtStages + 5;             // full, empty; done[2], 
 constexpr size_t kDtSmem = kDtOffBar + kDtBars * 8 + 16 + 1024;  // the stages start on 1 KB
 constexpr int kDtTmemCols = 256;                       // two accumulators of 96 columns, 128 apart
 static_assert(kTX + 3 <= kHX + 3 * kTX, "the dropped rows stay inside the stage");
-
-__device__ __forceinline__ void tc_rows_copy(void* dst, const CUtensorMap* map, int y, int x, int b,
-                                             uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], "
-      "[%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(x), "r"(b), "r"(smem_addr(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ void cl_mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
 
 __global__ void __launch_bounds__(kDtThreads, 1)
     conv32_wgrad_tc_kernel(Grid g, const __grid_constant__ CUtensorMap dz_map,
@@ -2051,15 +2061,8 @@ __global__ void __launch_bounds__(kDtThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const unsigned spin_limit = g_closure_spin_limit;
-  // Bounded wait that also ends when another warp has given up; whoever gives up stops the rest.
   auto wait = [&](uint64_t* bar, unsigned parity, unsigned limit) {
-    constexpr unsigned kPolls = 64;
-    for (unsigned k = 0; k < limit; k += kPolls) {
-      if (cl_mbar_wait(bar, parity, kPolls)) return true;
-      if (*stop) return false;
-    }
-    *stop = 1;
-    return false;
+    return cl_mbar_wait_or_stop(bar, parity, limit, stop);
   };
 
   float acc[3][C];  // warps 0 .. 2: row co = lane of tap row 2 - warp, columns (d, ci)
@@ -2089,11 +2092,9 @@ __global__ void __launch_bounds__(kDtThreads, 1)
     }
   } else if (warp == 3) {
     if (lane == 0) {
-      // Both operands with M / N contiguous (bits 15 and 16) and rows of 64 bytes, swizzled (4 at
-      // bit 61): the descriptor's strides are between groups of 32 of M or N and between groups of
-      // eight cells.
+      // Both operands with M / N contiguous (bits 15 and 16): the descriptor's strides are between
+      // groups of 32 of M or N and between groups of eight cells.
       const uint32_t idesc = umma_idesc_bf16(128, 96) | (1u << 15) | (1u << 16);
-      const uint64_t swizzle = 4ull << 61;
       unsigned n = 0;
       for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
         const unsigned s = n % kDtStages, h = n & 1u;
@@ -2106,8 +2107,8 @@ __global__ void __launch_bounds__(kDtThreads, 1)
 #pragma unroll
           for (int k = 0; k < kTY / 16; ++k) {
             const unsigned off = i * kDtRow + k * 16 * C * 2;
-            umma_bf16(tmem + h * 128, umma_desc(dz + off, kDtRow, 8 * C * 2) | swizzle,
-                      umma_desc(a + off, kDtCopy, 8 * C * 2) | swizzle, idesc, i + k != 0);
+            umma_bf16(tmem + h * 128, umma_desc(dz + off, kDtRow, 8 * C * 2) | kSwizzle64,
+                      umma_desc(a + off, kDtCopy, 8 * C * 2) | kSwizzle64, idesc, i + k != 0);
           }
         umma_commit(empty + s);
         umma_commit(done + h);
@@ -2156,8 +2157,7 @@ __global__ void __launch_bounds__(kDtThreads, 1)
   }
 }
 
-// The [batch][nx][ny][32] BF16 activations as conv32_tc_kernel's 5D tensor map (through the
-// runtime's driver entry point: no link against libcuda). False when it cannot be encoded.
+// The runtime's driver entry point (no link against libcuda), or null.
 PFN_cuTensorMapEncodeTiled_v12000 tc_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
     void* p = nullptr;
@@ -2171,35 +2171,20 @@ PFN_cuTensorMapEncodeTiled_v12000 tc_encoder() {
   return encode;
 }
 
-bool tc_mappable(const void* base, int64_t nx, int64_t ny, int64_t batch) {
-  return tc_encoder() != nullptr && (reinterpret_cast<uintptr_t>(base) & 15) == 0 &&
-         nx < (1ll << 31) && ny < (1ll << 31) && batch < (1ll << 31);
-}
-
-bool tc_input_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch) {
-  if (!tc_mappable(base, nx, ny, batch)) return false;
-  const cuuint64_t dims[5] = {8, 4, (cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)batch};
-  const cuuint64_t strides[4] = {16, 64, (cuuint64_t)ny * 64, (cuuint64_t)(nx * ny) * 64};
-  const cuuint32_t box[5] = {8, 1, (cuuint32_t)kTRegC, (cuuint32_t)kTRegR, 1};
-  const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
-  return tc_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims,
-                      strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The same activations for conv32_wgrad_tc_kernel: boxes of `rows` x kTY whole cells.
-bool tc_rows_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch,
-                 int rows) {
-  if (!tc_mappable(base, nx, ny, batch)) return false;
+// The [batch][nx][ny][32] BF16 activations as a tensor map with boxes of rows x cols whole cells,
+// swizzled over 64 bytes. False when it cannot be encoded.
+bool tc_rows_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t batch, int rows,
+                 int cols) {
+  const auto encode = tc_encoder();
+  if (encode == nullptr || (reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
+  if (nx >= (1ll << 31) || ny >= (1ll << 31) || batch >= (1ll << 31)) return false;
   const cuuint64_t dims[4] = {C, (cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)batch};
   const cuuint64_t strides[3] = {64, (cuuint64_t)ny * 64, (cuuint64_t)(nx * ny) * 64};
-  const cuuint32_t box[4] = {C, (cuuint32_t)kTY, (cuuint32_t)rows, 1};
+  const cuuint32_t box[4] = {C, (cuuint32_t)cols, (cuuint32_t)rows, 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
-  return tc_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims,
-                      strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides,
+                box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Tiles of kTR x kTC cells for conv32_tc_kernel.
@@ -2378,9 +2363,9 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
                                               z1, reinterpret_cast<bf16*>(a1));
   CL_CUDA(cudaGetLastError());
   CUtensorMap a1_map;
-  if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_input_map(&a1_map, a1, nx, ny, batch)) {
+  if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_rows_map(&a1_map, a1, nx, ny, batch, kTR + 2, kTC)) {
     const Grid gt = tc_grid(nx, ny, batch);
-    const int grid_tc = (int)std::min<int64_t>(gt.tiles, (int64_t)sms * kTPerSm);
+    const int grid_tc = (int)std::min<int64_t>(gt.tiles, (int64_t)sms);
     conv32_tc_kernel<false><<<grid_tc, kTThreads, kTSmem, s>>>(
         gt, a1_map, wb + LBM_CLOSURE_OFF_W2, params + LBM_CLOSURE_OFF_B2, nullptr, z2,
         reinterpret_cast<bf16*>(a2));
@@ -2461,8 +2446,8 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   CL_CUDA(cudaGetLastError());
   CUtensorMap dz2_rows, a1_rows;
   if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 &&
-      tc_rows_map(&dz2_rows, dz2, nx, ny, batch, kHX) &&
-      tc_rows_map(&a1_rows, a1, nx, ny, batch, kTX)) {
+      tc_rows_map(&dz2_rows, dz2, nx, ny, batch, kHX, kTY) &&
+      tc_rows_map(&a1_rows, a1, nx, ny, batch, kTX, kTY)) {
     conv32_wgrad_tc_kernel<<<rows_w2, kDtThreads, kDtSmem, s>>>(g, dz2_rows, a1_rows, partial);
   } else {
     conv32_wgrad_kernel<<<rows_w2, kDw2Threads, kDw2Smem, s>>>(g, reinterpret_cast<const bf16*>(a1),
@@ -2470,9 +2455,9 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   }
   CL_CUDA(cudaGetLastError());
   CUtensorMap dz2_map;
-  if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_input_map(&dz2_map, dz2, nx, ny, batch)) {
+  if (g_layer2_kernel == LBM_CLOSURE_LAYER2_TCGEN05 && tc_rows_map(&dz2_map, dz2, nx, ny, batch, kTR + 2, kTC)) {
     const Grid gt = tc_grid(nx, ny, batch);
-    const int ctas = (int)std::min<int64_t>(gt.tiles, (int64_t)device_sms() * kTPerSm);
+    const int ctas = (int)std::min<int64_t>(gt.tiles, (int64_t)device_sms());
     conv32_tc_kernel<true><<<ctas, kTThreads, kTSmem, s>>>(
         gt, dz2_map, wb + LBM_CLOSURE_OFF_W2, nullptr, z1, nullptr, dz1);
   } else {

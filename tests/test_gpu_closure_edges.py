@@ -1,4 +1,4 @@
-"""The closure's training kernels at the edges of their tiles (4 x 64, 14 x 32 and 30 x 64 cells):
+"""The closure's training kernels at the edges of their tiles (4 x 64, 8 x 32 and 30 x 64 cells):
 one cell short of a tile, one past it, smaller than any, several samples; the same checks and
 bounds against the float64 oracle as for the ordinary shapes."""
 
