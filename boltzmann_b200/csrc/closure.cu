@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
 #include "../../include/lbm_closure.h"
 #include "sim.h"
@@ -1296,6 +1297,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Eight of them.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 constexpr unsigned kClosureSpinLimit = 1u << 22;
 
 __device__ __forceinline__ void cl_mbar_init(uint64_t* bar, unsigned count) {
@@ -1356,7 +1367,10 @@ __device__ int g_closure_status;
 // layer 1 with K = 48 (9 taps x 4 channels, zero-padded from 36), layer 2 with K = 288, layer 3
 // with K = 288 and N = 8 (one real output column). A warp's
 // 16-row MMA tile is any 16 consecutive cells of a region in row-major order (ldmatrix takes one
-// row address per lane), so the regions need not be multiples of 16 wide.
+// row address per lane), so the regions need not be multiples of 16 wide. Bound by the instruction
+// stream of the two GELU epilogues and layer 1's fragments, with the MMAs' reads of A behind it.
+// 1024 x 512: 124 -> 105 us with GELU on packed pairs, the ninth block of layer 2 shared among the
+// warps of a sub-partition and layer 3's chains in pairs.
 
 constexpr int kFR = 14, kFC = 64;               // output tile
 constexpr int kA2R = kFR + 2, kA2C = kFC + 2;  // layer-2 region
@@ -1582,10 +1596,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
           const int ch = nt * 8 + 2 * tq;
-          __nv_bfloat162 o;
-          o.x = to_bf(inside ? gelu(acc[nt][2 * h] + bs[ch]) : 0.0f);
-          o.y = to_bf(inside ? gelu(acc[nt][2 * h + 1] + bs[ch + 1]) : 0.0f);
-          *reinterpret_cast<__nv_bfloat162*>(a1c + ((size_t)nt * kA1Pad + q) * 16 + tq * 4) = o;
+          const float2 z = __fadd2_rn(make_float2(acc[nt][2 * h], acc[nt][2 * h + 1]),
+                                      *reinterpret_cast<const float2*>(bs + ch));
+          *reinterpret_cast<uint32_t*>(a1c + ((size_t)nt * kA1Pad + q) * 16 + tq * 4) =
+              inside ? pack_bf2(gelu2(z)) : 0u;
         }
       }
     }
@@ -1626,48 +1640,70 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       break;
     }
     tc_fence_after();
-    // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition) of blocks
-    // w / 4, w / 4 + 4, w / 4 + 8; one thread per cell, its 32 channels in registers.
-    for (int m = warp >> 2; m < kL2Blocks; m += kWarps / 4) {
-      const int sp = warp & 3;
-      uint32_t r32[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * sp) << 16) + (uint32_t)(m * 32), r32);
+    // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its sub-partition) of blocks w / 4 and
+    // w / 4 + 4, one thread per cell with its 32 channels, and channels 8 (w / 4) .. + 7 of the last
+    // block: a sub-partition's four warps, which share a scheduler, end together (with one of them
+    // on the whole last block they waited for it).
+    const int sp = warp & 3, part = warp >> 2;
+    auto activate = [&](int m, int ch0, const uint32_t* z, auto chunks) {
       const int p = kL2First + 128 * m + 32 * sp + lane;  // layer-1 flat index of this row
       const int r = p / kA1C - 1, c = p % kA1C - 1;      // layer-2 region coordinates
-      if (r < 0 || r >= kA2R || c < 0 || c >= kA2C) continue;
+      if (r < 0 || r >= kA2R || c < 0 || c >= kA2C) return;
       const int64_t x = x0 - 1 + r, y = y0 - 1 + c;
       const bool inside = x >= 0 && x < f.nx && y >= 0 && y < f.ny;
-      uint32_t packed[C / 2];
+      uint4* dst = reinterpret_cast<uint4*>(a2s + (r * kA2C + c) * kCS + ch0);
 #pragma unroll
-      for (int ch = 0; ch < C; ch += 2) {
-        const float v0 = inside ? gelu(__uint_as_float(r32[ch]) + bs[C + ch]) : 0.0f;
-        const float v1 = inside ? gelu(__uint_as_float(r32[ch + 1]) + bs[C + ch + 1]) : 0.0f;
-        packed[ch / 2] = (uint32_t)__bfloat16_as_ushort(to_bf(v0)) |
-                         ((uint32_t)__bfloat16_as_ushort(to_bf(v1)) << 16);
+      for (int q = 0; q < decltype(chunks)::value; ++q) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int ch = 8 * q + 2 * e;
+          const float2 v = __fadd2_rn(
+              make_float2(__uint_as_float(z[ch]), __uint_as_float(z[ch + 1])),
+              *reinterpret_cast<const float2*>(bs + C + ch0 + ch));
+          w[e] = inside ? pack_bf2(gelu2(v)) : 0u;
+        }
+        dst[q] = make_uint4(w[0], w[1], w[2], w[3]);
       }
-      uint4* dst = reinterpret_cast<uint4*>(a2s + (r * kA2C + c) * kCS);
-#pragma unroll
-      for (int q = 0; q < C / 8; ++q)
-        dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+    };
+    const uint32_t lanes = (uint32_t)(32 * sp) << 16;
+    static_assert(kL2Blocks == 9, "two blocks a warp and a quarter of the last");
+#pragma unroll 1
+    for (int m = part; m < 8; m += 4) {
+      uint32_t z[32];
+      __syncwarp();
+      tmem_ld32(tmem + lanes + (uint32_t)(m * 32), z);
+      activate(m, 0, z, std::integral_constant<int, 4>{});
+    }
+    {
+      uint32_t z[8];
+      __syncwarp();
+      tmem_ld8(tmem + lanes + (uint32_t)(8 * 32 + 8 * part), z);
+      activate(8, 8 * part, z, std::integral_constant<int, 1>{});
     }
     __syncthreads();
 
     // Layer 3 on tensor cores (N = 8 with only column 0 carrying w3; K = 288) and the relaxation
     // rate (the mapping of omega_kernel) on the output tile: 16 cells of one tile row per MMA tile.
-    constexpr int n3 = kFR * kFC;
-    for (int mt = warp; mt * 16 < n3; mt += kWarps) {
+    // A warp takes two of them side by side: their chains of 18 products hide each other's latency.
+    constexpr int n3 = kFR * kFC, kTiles3 = n3 / 16;
+    static_assert(n3 % 16 == 0, "whole tiles");
+    for (int mt = warp; mt < kTiles3; mt += 2 * kWarps) {
       const int j = (lane & 7) + 8 * ((lane >> 3) & 1);
-      const int qa = mt * 16 + j;
-      const int ra = qa / kFC, ca = qa - ra * kFC;
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const bf16* arow[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int qa = min(mt + u * kWarps, kTiles3 - 1) * 16 + j;
+        const int ra = qa / kFC, ca = qa - ra * kFC;
+        arow[u] = a2s + ((ra + 1) * kA2C + ca + 1) * kCS + 8 * (lane >> 4);
+      }
+      float acc[2][4] = {};
 #pragma unroll 1
       for (int tap = 0; tap < 9; ++tap) {
         const int dx = tap / 3 - 1, dy = tap % 3 - 1;
-        const bf16* arow = a2s + ((ra + 1 + dx) * kA2C + ca + 1 + dy) * kCS + 8 * (lane >> 4);
+        const int off = (dx * kA2C + dy) * kCS;
 #pragma unroll
         for (int kc = 0; kc < 2; ++kc) {
-          uint32_t a[4];
-          ldsm_x4(a, arow + kc * 16);
           // B column 0 = w3[tap][kc*16 + k]; lanes of the other columns hold zeros.
           uint32_t b0 = 0u, b1 = 0u;
           if (gq == 0) {
@@ -1675,17 +1711,24 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             b0 = *reinterpret_cast<const uint32_t*>(w3b + k0);
             b1 = *reinterpret_cast<const uint32_t*>(w3b + k0 + 8);
           }
-          mma_bf16(acc, a, b0, b1);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            uint32_t a[4];
+            ldsm_x4(a, arow[u] + off + kc * 16);
+            mma_bf16(acc[u], a, b0, b1);
+          }
         }
       }
-      if (tq == 0) {  // column 0: rows gq and gq + 8 of this tile
+      if (tq == 0) {  // column 0: rows gq and gq + 8 of each tile
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int q = mt * 16 + gq + 8 * h;
+        for (int k = 0; k < 4; ++k) {
+          const int u = k >> 1, h = k & 1;
+          if (mt + u * kWarps >= kTiles3) continue;
+          const int q = (mt + u * kWarps) * 16 + gq + 8 * h;
           const int r = q / kFC, c = q - r * kFC;
           const int64_t x = x0 + r, y = y0 + c;
           if (x >= f.nx || y >= f.ny) continue;
-          const float yv = acc[2 * h] + b3;
+          const float yv = acc[u][2 * h] + b3;
           const int64_t cell = x * f.ny + y;
           float tau = f.tau0;
           if (fluid_cell(f.flags[cell])) tau += fminf(f.max_dtau, f.gain * fmaxf(yv, 0.0f));
