@@ -388,7 +388,7 @@ __global__ void features_kernel(const float* __restrict__ rho, const float* __re
 // each). Bound by the FMA pipe (1152 a cell) beside 200 bytes a cell of traffic. A warp takes one row
 // of the tile, two lanes a cell (store_bf16_row) and four cells a lane, so that each shared-memory
 // weight load feeds eight FMAs; the inputs lie in shared memory as (v, v) pairs, the packed
-// instruction's operand. Batch 8 x 1024 x 512: 635 -> 336 us.
+// instruction's operand. Batch 8 x 1024 x 512: 635 -> 327 us (336 with the taps not unrolled).
 
 constexpr int kC1Threads = 32 * kTX;
 constexpr int kC1Cells = kTY / 16;  // cells a lane
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kC1Threads, kC1PerSm)
     for (int p = 0; p < kC1Cells; ++p)
 #pragma unroll
       for (int q = 0; q < 8; ++q) acc[p][q] = make_float2(0.0f, 0.0f);
-#pragma unroll 1
+#pragma unroll 3
     for (int tap = 0; tap < 9; ++tap) {
       const int dx = tap / 3 - 1, dy = tap % 3 - 1;
       const float* xc = xs + ((ti + 1 + dx) * kHY + lc + 1 + dy) * 8;
