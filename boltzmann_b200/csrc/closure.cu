@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kConv32Threads)
 // fragments it loads serve 24 MMAs (one warp a tap loaded them for eight). The next tile's operands
 // arrive (asynchronous copies) while this one's are multiplied. Bound by shared-memory reads (eight
 // ldmatrix a 24 MMAs). Batch 8 x 1024 x 512: 366 -> 311 us. Runs with the warp-level layer-2 kernels,
-// and where conv32_wgrad_tc_kernel (118 us) has no tensor map.
+// and where conv32_wgrad_tc_kernel (111 us) has no tensor map.
 
 constexpr int kDw2Threads = 3 * kTX * 32;
 constexpr int kDw2Stage = (kTX * kTY + kHX * kHY) * kCS;  // BF16 elements of one stage
@@ -1255,6 +1255,12 @@ __device__ __forceinline__ uint64_t umma_desc(unsigned start, unsigned lbo, unsi
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The descriptor `bytes` (a multiple of 16) further on: one addition to its low word. One thread
+// issues all of a CTA's products, and building a descriptor anew took it longer than the product.
+__device__ __forceinline__ uint64_t umma_desc_at(uint64_t desc, unsigned bytes) {
+  return (desc & ~0xffffffffull) | ((uint32_t)desc + (bytes >> 4));
+}
+
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 accumulator, both K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -1370,7 +1376,8 @@ __device__ int g_closure_status;
 // row address per lane), so the regions need not be multiples of 16 wide. Bound by the instruction
 // stream of the two GELU epilogues and layer 1's fragments, with the MMAs' reads of A behind it.
 // 1024 x 512: 124 -> 105 us with GELU on packed pairs, the ninth block of layer 2 shared among the
-// warps of a sub-partition and layer 3's chains in pairs.
+// warps of a sub-partition and layer 3's chains in pairs; 99 us with descriptors advanced by one
+// addition.
 
 constexpr int kFR = 14, kFC = 64;               // output tile
 constexpr int kA2R = kFR + 2, kA2C = kFC + 2;  // layer-2 region
@@ -1464,7 +1471,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t idesc = umma_idesc_bf16(128, 32);
-  const unsigned a1c_addr = smem_addr(a1c), w2c_addr = smem_addr(w2c);
+  const uint64_t a1desc = umma_desc(smem_addr(a1c), kA1Pad * 16, 128);
+  const uint64_t w2desc = umma_desc(smem_addr(w2c), C * 16, 128);
   bool healthy = true;
   const unsigned spin_limit = g_closure_spin_limit;
   // Layer-1 A fragments: element e of k-step kk holds input k = 16 kk + 2 tq + 8 (e >> 1), that
@@ -1621,13 +1629,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 #pragma unroll
         for (int kc = 0; kc < 2; ++kc) {
           const int sidx = tap * 2 + kc;
-          const uint64_t bdesc = umma_desc(w2c_addr + (unsigned)(sidx * 1024), C * 16, 128);
-          const unsigned a_base = a1c_addr + (unsigned)((2 * kc * kA1Pad + kL2First + off) * 16);
+          const uint64_t bdesc = umma_desc_at(w2desc, (unsigned)(sidx * 1024));
+          const uint64_t adesc =
+              umma_desc_at(a1desc, (unsigned)((2 * kc * kA1Pad + kL2First + off) * 16));
 #pragma unroll
           for (int m = 0; m < kL2Blocks; ++m)
-            umma_bf16(tmem + (uint32_t)(m * 32),
-                      umma_desc(a_base + (unsigned)(m * 128 * 16), kA1Pad * 16, 128), bdesc,
-                      idesc, sidx != 0);
+            umma_bf16(tmem + (uint32_t)(m * 32), umma_desc_at(adesc, (unsigned)(m * 128 * 16)),
+                      bdesc, idesc, sidx != 0);
         }
       }
       umma_commit(mma_done);
@@ -1768,10 +1776,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 // One warp copies (a ring of kTStages tiles), one issues the products, and two groups of eight warps
 // take the tiles in turn in the epilogue, which reads each cell's 32 accumulators with tcgen05.ld.
 // Bound by shared memory (the products read A anew for each tap: 720 bytes a cell, of 1300 in all)
-// close to DRAM (256 bytes a cell, 166 us over batch 8 x 1024 x 512): 241 us forward and 232 us
-// backward there. Before, one region with a halo, 16 bytes a cell and plane, served all taps by the
-// start address: copies of 16-byte rows kept the tensor engine busy for 275 us whatever ran beside
-// them, and with copies, products and epilogue in turn in three CTAs an SM it took 290 and 278 us.
+// close to DRAM (256 bytes a cell, 166 us over batch 8 x 1024 x 512): 199 us forward and backward
+// there. With copies, products and epilogue in turn in three CTAs an SM, on regions with a halo whose
+// discarded rows are an eighth of the products, it took 290 and 278 us; side by side 279 and 276; on
+// whole rows 241 and 232, 120 cycles a product, most of them the issuing thread's descriptors.
 
 constexpr int kTR = 8, kTC = 32;                    // output tile
 constexpr int kTBlocks = kTR * kTC / 128;           // 128-cell blocks
@@ -1902,28 +1910,28 @@ __global__ void __launch_bounds__(kTThreads, 1)
   } else if (warp == kTEpilogue + 1) {
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_bf16(128, 32);
-      const unsigned wc_addr = smem_addr(wc);
+      const uint64_t bdesc = umma_desc(smem_addr(wc), C * 16, 128);
       unsigned n = 0;
       for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x, ++n) {
         const unsigned s = n % kTStages, h = n & 1u;
         if (!wait(full + s, (n / kTStages) & 1u, kClosureSpinLimit)) break;
         if (n >= 2 && !wait(read + h, (n / 2 - 1) & 1u, kClosureSpinLimit)) break;
         tc_fence_after();
-        const unsigned in_addr = smem_addr(base) + s * kTStage;
+        const uint64_t adesc =
+            umma_desc(smem_addr(base) + s * kTStage, 16, 8 * C * 2) | kSwizzle64;
         // K-slice outer, block inner: consecutive MMAs accumulate into different TMEM columns.
-#pragma unroll 1
+#pragma unroll
         for (int tap = 0; tap < 9; ++tap) {
           const int dx = BWD ? 1 - tap / 3 : tap / 3 - 1, d = BWD ? 2 - tap % 3 : tap % 3;
 #pragma unroll
           for (int kc = 0; kc < 2; ++kc) {
             const int sidx = tap * 2 + kc;
-            const uint64_t bdesc = umma_desc(wc_addr + (unsigned)(sidx * 1024), C * 16, 128);
-            const unsigned a_base = in_addr + d * kTCopy + (1 + dx) * kTRow + kc * 32;
 #pragma unroll
             for (int m = 0; m < kTBlocks; ++m)
               umma_bf16(tmem + h * (kTBlocks * 32) + (uint32_t)(m * 32),
-                        umma_desc(a_base + (unsigned)(m * 128 * C * 2), 16, 8 * C * 2) | kSwizzle64,
-                        bdesc, idesc, sidx != 0);
+                        umma_desc_at(adesc, d * kTCopy + (1 + dx) * kTRow + kc * 32 +
+                                                (unsigned)(m * 128 * C * 2)),
+                        umma_desc_at(bdesc, (unsigned)(sidx * 1024)), idesc, sidx != 0);
           }
         }
         umma_commit(empty + s);
@@ -2055,7 +2063,7 @@ __global__ void __launch_bounds__(kTThreads, 1)
 // products go to the other half of tensor memory: a chain in the truncating accumulators ends with
 // its tile.
 // Bound by the copies: 128 bytes a cell of DRAM traffic take 83 us over batch 8 x 1024 x 512, and
-// 288 bytes a cell come out of L2. 118 us, where conv32_wgrad_kernel, at the rate of mma.sync, takes
+// 288 bytes a cell come out of L2. 111 us, where conv32_wgrad_kernel, at the rate of mma.sync, takes
 // 311; the gradient is 2.1e-7 off its float64 sums at any batch, 6.8e-6 there.
 
 constexpr int kDtThreads = 160;
@@ -2144,14 +2152,16 @@ __global__ void __launch_bounds__(kDtThreads, 1)
         if (!wait(full + s, (n / kDtStages) & 1u, kClosureSpinLimit)) break;
         if (n >= 2 && !wait(read + h, (n / 2 - 1) & 1u, kClosureSpinLimit)) break;
         tc_fence_after();
-        const unsigned dz = smem_addr(base) + s * kDtStage, a = dz + kDtDz;
+        const unsigned dz = smem_addr(base) + s * kDtStage;
+        const uint64_t adesc = umma_desc(dz, kDtRow, 8 * C * 2) | kSwizzle64;
+        const uint64_t bdesc = umma_desc(dz + kDtDz, kDtCopy, 8 * C * 2) | kSwizzle64;
 #pragma unroll
         for (int i = 0; i < kTX; ++i)
 #pragma unroll
           for (int k = 0; k < kTY / 16; ++k) {
             const unsigned off = i * kDtRow + k * 16 * C * 2;
-            umma_bf16(tmem + h * 128, umma_desc(dz + off, kDtRow, 8 * C * 2) | kSwizzle64,
-                      umma_desc(a + off, kDtCopy, 8 * C * 2) | kSwizzle64, idesc, i + k != 0);
+            umma_bf16(tmem + h * 128, umma_desc_at(adesc, off), umma_desc_at(bdesc, off), idesc,
+                      i + k != 0);
           }
         umma_commit(empty + s);
         umma_commit(done + h);
