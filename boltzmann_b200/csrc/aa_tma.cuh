@@ -364,7 +364,6 @@ __global__ void __launch_bounds__(tma_threads<PAIR>(), tma_min_blocks<L, K, PAIR
   using TT = typename TP::type;
   constexpr int Q = L::Q;
 
-  grid_trigger_next();
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)S * St::bytes);
   uint64_t* empty = full + S;
@@ -425,7 +424,6 @@ __global__ void __launch_bounds__(tma_threads<PAIR>(), tma_min_blocks<L, K, PAIR
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
-  grid_wait_previous();
 
   if (warp == CW) {
     // ---- producer warp. Each lane owns up to two copy jobs (job = lane, lane + 32), fixed for
