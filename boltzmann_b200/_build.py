@@ -38,7 +38,7 @@ NVCC_FLAGS = [
 
 CUDA_SOURCES = ["aa_d2q9.cu", "aa_d3q27.cu", "aa_resident.cu", "fields.cu", "capi.cu", "noalloc.cu", "ensemble.cu", "closure.cu"]
 HEADERS = ["aa_step.cuh", "aa_tma.cuh", "aa_pair.cuh", "aa_resident.cuh", "aa_launch.cuh", "lattice.cuh",
-           "storage.cuh", "sim.h"]
+           "storage.cuh", "sim.h", "device_once.h"]
 
 
 def _run(cmd: list[str]) -> None:

@@ -5,11 +5,11 @@
 #include <cudaTypedefs.h>
 
 #include <atomic>
-#include <mutex>
 #include <type_traits>
 
 #include "aa_tma.cuh"
 #include "aa_step.cuh"
+#include "device_once.h"
 #include "sim.h"
 
 namespace lbm {
@@ -147,16 +147,17 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
   constexpr bool PAIR = pair_form<L, TRT, K, NT>() && (L::D == 2 || !EVEN || WR);
   constexpr int threads = tma_threads<PAIR>();
   auto kern = aa_tma_kernel<L, TRT, K, EVEN, NT, S, WR, PAIR, KT>;
-  static std::once_flag once;
-  static cudaError_t setup_err = cudaSuccess;
-  static int per_sm = 1;
-  std::call_once(once, [&] {
-    setup_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (setup_err == cudaSuccess)
-      setup_err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-    if (per_sm < 1) per_sm = 1;
+  static DeviceOnce once;
+  static std::atomic<int> occupancy{1};
+  const cudaError_t setup_err = once([&] {
+    int fit = 1;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem);
+    occupancy = fit < 1 ? 1 : fit;
+    return e;
   });
   if (setup_err != cudaSuccess) return setup_err;
+  const int per_sm = occupancy;
   int device = 0, sms = 148;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);

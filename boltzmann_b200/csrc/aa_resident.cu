@@ -2,9 +2,9 @@
 #include "aa_resident.cuh"
 
 #include <algorithm>
-#include <mutex>
 
 #include "aa_launch.cuh"
+#include "device_once.h"
 
 namespace lbm {
 namespace {
@@ -78,13 +78,11 @@ template <bool TRT, int K, int NT, int KT>
 cudaError_t run(lbm_sim& s, const ResidentPlan& plan, int64_t steps) {
   using Real = typename Pop<K>::real;
   auto kern = aa_resident_kernel<D2Q9, TRT, K, NT, KT>;
-  static std::once_flag once;
-  static cudaError_t setup_err = cudaSuccess;
-  std::call_once(once, [&] {
-    int device = 0, limit = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    setup_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+  static DeviceOnce once;
+  const cudaError_t setup_err = once([&] {
+    int limit = 0;
+    cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, s.device);
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   });
   if (setup_err != cudaSuccess) return setup_err;
   for (int64_t left = steps; left > 0;) {

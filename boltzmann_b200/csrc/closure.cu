@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "../../include/lbm_closure.h"
+#include "device_once.h"
 #include "sim.h"
 
 namespace {
@@ -2331,9 +2332,8 @@ bool shape_ok(int64_t nx, int64_t ny, int64_t batch) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-int set_smem(const void* fn, size_t bytes) {
-  CL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return LBM_OK;
+cudaError_t set_smem(const void* fn, size_t bytes) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // Workspace: [kCountBlocks counts (256 B)][loss partials (kLossBlocks doubles, padded)]
@@ -2398,14 +2398,15 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
   if (!aligned16(params_bf16) || !aligned16(x) || !aligned16(a1) || !aligned16(a2) ||
       (z1 && !aligned16(z1)) || (z2 && !aligned16(z2)))
     return fail(LBM_ERR_ARGUMENT, "closure forward: arrays must be 16-byte aligned");
-  static thread_local bool configured = false;
-  if (!configured) {
-    if (int rc = set_smem((const void*)conv32_kernel<false>, kConv32Smem)) return rc;
-    if (int rc = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return rc;
-    if (int rc = set_smem((const void*)conv32_tc_kernel<false>, kTSmem)) return rc;
-    if (int rc = set_smem((const void*)conv3_fwd_kernel, kConv3Smem)) return rc;
-    configured = true;
-  }
+  static lbm::DeviceOnce once;
+  const cudaError_t setup = once([] {
+    if (cudaError_t e = set_smem((const void*)conv32_kernel<false>, kConv32Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_tc_kernel<false>, kTSmem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv3_fwd_kernel, kConv3Smem)) return e;
+    return cudaSuccess;
+  });
+  CL_CUDA(setup);
   const Grid g = make_grid(nx, ny, batch);
   const cudaStream_t s = (cudaStream_t)stream;
   const int sms = device_sms();
@@ -2473,17 +2474,18 @@ int lbm_closure_backward(const float* params, const uint16_t* params_bf16, const
   if (!aligned16(workspace) || !aligned16(params_bf16) || !aligned16(x) || !aligned16(z1) ||
       !aligned16(a1) || !aligned16(z2) || !aligned16(a2))
     return fail(LBM_ERR_ARGUMENT, "closure backward: arrays must be 16-byte aligned");
-  static thread_local bool configured = false;
-  if (!configured) {
-    if (int rc = set_smem((const void*)conv32_kernel<false>, kConv32Smem)) return rc;
-    if (int rc = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return rc;
-    if (int rc = set_smem((const void*)conv32_tc_kernel<true>, kTSmem)) return rc;
-    if (int rc = set_smem((const void*)conv32_wgrad_kernel, kDw2Smem)) return rc;
-    if (int rc = set_smem((const void*)conv32_wgrad_tc_kernel, kDtSmem)) return rc;
-    if (int rc = set_smem((const void*)conv3_bwd_kernel, kConv3BwdSmem)) return rc;
-    if (int rc = set_smem((const void*)conv1_wgrad_kernel, kW1Smem)) return rc;
-    configured = true;
-  }
+  static lbm::DeviceOnce once;
+  const cudaError_t setup = once([] {
+    if (cudaError_t e = set_smem((const void*)conv32_kernel<false>, kConv32Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_tc_kernel<true>, kTSmem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_wgrad_kernel, kDw2Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv32_wgrad_tc_kernel, kDtSmem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv3_bwd_kernel, kConv3BwdSmem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv1_wgrad_kernel, kW1Smem)) return e;
+    return cudaSuccess;
+  });
+  CL_CUDA(setup);
   const Grid g = make_grid(nx, ny, batch);
   const cudaStream_t s = (cudaStream_t)stream;
   auto* base = static_cast<unsigned char*>(workspace);
@@ -2565,11 +2567,10 @@ int lbm_closure_relaxation(const float* params, const uint16_t* params_bf16, con
     return fail(LBM_ERR_ARGUMENT, "closure relaxation: bad arguments");
   if (!aligned16(params_bf16))
     return fail(LBM_ERR_ARGUMENT, "closure relaxation: params_bf16 must be 16-byte aligned");
-  static thread_local bool configured = false;
-  if (!configured) {
-    if (int rc = set_smem((const void*)closure_fused_kernel, kFusedSmem)) return rc;
-    configured = true;
-  }
+  static lbm::DeviceOnce once;
+  const cudaError_t setup =
+      once([] { return set_smem((const void*)closure_fused_kernel, kFusedSmem); });
+  CL_CUDA(setup);
   FusedArgs fa;
   fa.params = params;
   fa.wb = reinterpret_cast<const bf16*>(params_bf16);

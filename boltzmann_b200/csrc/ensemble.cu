@@ -30,8 +30,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
-#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -39,6 +39,7 @@
 #include "../../include/lbm_cuda.h"
 #include "aa_step.cuh"
 #include "aa_tma.cuh"
+#include "device_once.h"
 #include "sim.h"
 
 namespace {
@@ -594,18 +595,19 @@ cudaError_t launch_rows_parity(lbm_ensemble* e, bool write_moments) {
   using Real = typename lbm::Pop<K>::real;
   auto kern = ensemble_rows_kernel<TRT, K, EVEN>;
   constexpr size_t smem = row_smem_bytes<K>();
-  static std::once_flag once;
-  static cudaError_t setup_err = cudaSuccess;
-  static int occupancy = 1;
-  std::call_once(once, [&] {
-    setup_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (setup_err == cudaSuccess)
-      setup_err =
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, kern, kRowThreads, smem);
-    if (occupancy < 1) occupancy = 1;
+  static lbm::DeviceOnce once;
+  static std::atomic<int> occupancy{1};
+  const cudaError_t setup_err = once([&] {
+    int fit = 1;
+    cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (r == cudaSuccess)
+      r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kRowThreads, smem);
+    occupancy = fit < 1 ? 1 : fit;
+    return r;
   });
   if (setup_err != cudaSuccess) return setup_err;
-  const int per_sm = e->blocks_per_sm > 0 ? std::min(e->blocks_per_sm, occupancy) : occupancy;
+  const int fit = occupancy;
+  const int per_sm = e->blocks_per_sm > 0 ? std::min(e->blocks_per_sm, fit) : fit;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
   long long grid = (long long)sms * per_sm;

@@ -1,0 +1,52 @@
+"""The host side of lbm_iterate without a GPU: what it launches, and what it does when the runtime
+refuses."""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests.fake_runtime import FakeSim, load
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return load(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.mark.parametrize("counts,storage,kernel", [((64, 64), "f32", "aa_resident_kernel"),
+                                                   ((200, 150), "f16", "aa_resident_kernel"),
+                                                   ((64, 64, 256), "f32", "aa_tma_kernel")])
+def test_kernels_are_set_up_on_every_device(lib, counts, storage, kernel):
+    """Shared memory above 48 KB is opted into per device: a simulation on a second GPU of the
+    process runs as one on the first, in either order and again."""
+    for device in (1, 0, 1):
+        sim = FakeSim(lib, counts, storage=storage, device=device)
+        sim.check(sim.iterate(20))
+        launched = sim.launched()
+        assert launched and all(d == device and kernel in name for d, name in launched)
+        sim.close()
+
+
+def test_ensemble_and_closure_are_set_up_on_every_device(lib):
+    nx, ny = 40, 70
+    params = np.zeros(10752, np.float32)
+    fields = [np.zeros(nx * ny * 2, np.float32) for _ in range(4)]
+    p = lambda a: C.c_void_p(a.ctypes.data)  # noqa: E731
+    for device in (1, 0):
+        lib.fake_set_device(device)
+        h = C.c_void_p()
+        counts = (C.c_int64 * 2)(40000, 128)  # too large for the flat kernel: rows, staged
+        om = (C.c_float * 1)(1.6)
+        assert lib.lbm_ensemble_create(1, counts, 0, om, om, 0, C.byref(h)) == 0
+        assert lib.lbm_ensemble_iterate(h, C.c_int64(2), 0) == 0, lib.lbm_last_error()
+        lib.lbm_ensemble_destroy(h)
+        lib.fake_take_log()
+        rc = lib.lbm_closure_relaxation(p(params), p(params), p(fields[0]), p(fields[1]),
+                                        p(fields[2]), C.c_int64(nx), C.c_int64(ny), p(fields[3]),
+                                        C.c_float(0.6), C.c_float(0.1), C.c_float(0.1), p(fields[0]),
+                                        None)
+        assert rc == 0, lib.lbm_last_error()
+        assert lib.fake_take_log().decode().startswith(f"{device} ")
