@@ -50,3 +50,29 @@ def test_ensemble_and_closure_are_set_up_on_every_device(lib):
                                         None)
         assert rc == 0, lib.lbm_last_error()
         assert lib.fake_take_log().decode().startswith(f"{device} ")
+
+
+@pytest.mark.parametrize("steps", [20, 4000, 4002, 12000])
+def test_calls_of_any_length_fall_back_to_single_steps(lib, steps):
+    """Where a cooperative grid does not fit (a partition of the GPU), a call takes single steps,
+    however many launches the resident kernel would have made of it, and so do later calls."""
+    sim = FakeSim(lib, (256, 256))
+    try:
+        lib.fake_set_cooperative_limit(64)
+        sim.check(sim.iterate(steps))
+        assert set(sim.kernels()) == {"aa_step_kernel"}
+    finally:
+        lib.fake_set_cooperative_limit(-1)
+    sim.check(sim.iterate(steps))
+    assert set(sim.kernels()) <= {"aa_step_kernel"}
+    sim.close()
+
+
+def test_a_failure_after_the_first_launch_is_an_error(lib):
+    sim = FakeSim(lib, (64, 64))
+    lib.fake_fail_launch(1, 720)  # cudaErrorCooperativeLaunchTooLarge at the second launch
+    assert sim.iterate(8000) != 0
+    assert sim.kernels() == ["aa_resident_kernel"]
+    sim.check(sim.iterate(8000))
+    assert sim.kernels() == ["aa_resident_kernel"] * 2
+    sim.close()
