@@ -104,9 +104,10 @@ cudaError_t run(lbm_sim& s, const ResidentPlan& plan, int64_t steps) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     if (cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, d)) {
+      cudaGetLastError();  // reported here, not by the next launch's check too
       const bool first = left + now == steps;  // nothing enqueued yet
       if (e != cudaErrorCooperativeLaunchTooLarge || !first) return e;
-      cudaGetLastError();  // fewer SMs than the device has (a partition): single steps
+      // Fewer SMs than the device has (a partition): single steps.
       s.resident_gy = 0;
       return cudaErrorNotSupported;
     }

@@ -663,7 +663,9 @@ cudaError_t launch_step_kernel(void (*kern)(Params...), unsigned grid, unsigned 
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch's check too
+  return e;
 }
 
 constexpr int kDirectThreads = 128;

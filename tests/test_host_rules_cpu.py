@@ -76,3 +76,15 @@ def test_a_failure_after_the_first_launch_is_an_error(lib):
     sim.check(sim.iterate(8000))
     assert sim.kernels() == ["aa_resident_kernel"] * 2
     sim.close()
+
+
+@pytest.mark.parametrize("counts,steps", [((64, 64), 8000), ((64, 64), 2), ((30, 20, 10), 4),
+                                          ((64, 64, 256), 4)])
+def test_a_failed_launch_is_reported_once(lib, counts, steps):
+    """The error of a launch that fails is that call's; the next call does not meet it again."""
+    sim = FakeSim(lib, counts)
+    lib.fake_fail_launch(1, 701)  # cudaErrorLaunchOutOfResources at the second launch
+    assert sim.iterate(steps) != 0
+    sim.check(lib.lbm_equilibrate(sim.h))
+    sim.check(sim.iterate(2))
+    sim.close()
