@@ -92,6 +92,8 @@ cudaError_t run(lbm_sim& s, const ResidentPlan& plan, int64_t steps) {
     ResidentArgs d = plan.args;
     d.steps = now;
     d.seq = s.mail_seq;
+    d.polls = s.spin_limit < 0 ? kResidentPolls
+                               : (unsigned)std::min<int64_t>(s.spin_limit, kResidentPolls);
     for (int k = 0; k < 2; ++k) d.mail[k] = static_cast<unsigned long long*>(s.mail[k]);
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
@@ -190,8 +192,8 @@ cudaError_t iterate_resident(lbm_sim& s, int64_t steps) {
   // A launch costs the way of the domain into and out of shared memory (6 us for 64^2, 16 us for
   // 1000 x 501), which some steps have to earn: measured even with single steps at 4 of them for
   // 64^2, 6 for 256^2, 10 for 512 x 500, 14 for 700 x 451 in FP16.
-  if (s.dim != 2 || s.q != D2Q9::Q || s.kernel_path != 0 || s.spin_limit >= 0 ||
-      s.tracers.size() > 1 || steps < 4 + s.n / 32768)
+  if (s.dim != 2 || s.q != D2Q9::Q || s.kernel_path != 0 || s.tracers.size() > 1 ||
+      steps < 4 + s.n / 32768)
     return cudaErrorNotSupported;
   return with_variant(s, (int)s.tracers.size(), Iterate{s, steps});
 }

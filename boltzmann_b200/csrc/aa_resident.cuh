@@ -37,7 +37,8 @@
 
 namespace lbm {
 
-constexpr unsigned kResidentPolls = 1u << 20;  // about a second
+// Polls of a word before a thread gives up, unless the simulation sets a limit: about a second.
+constexpr unsigned kResidentPolls = 1u << 20;
 
 // Threads of a CTA at most: the registers of an SM over what a thread of the variant needs.
 template <int K, int NT>
@@ -65,6 +66,7 @@ struct ResidentArgs {
   int published;   // cells a CTA publishes of a slot at most
   int messages;    // table entries for receiving (and for sending) at most
   unsigned seq;    // sequence number of the first pair
+  unsigned polls;  // of the words that a thread waits for at a time, before it gives up
   unsigned long long* mail[2];  // two sets of [words][CTAs][slots][published]
 };
 
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(resident_threads<K, NT>())
   StepArgs<Real> now = a;  // only the last step of a call writes moments
   unsigned seq = d.seq;
   const size_t set_words = (size_t)gridDim.x * NS * d.published;
-  bool ok = true;
+  bool ok = d.polls > 0;
   for (int s = 0; s < d.steps; s += 2, ++seq) {
     unsigned long long* box = d.mail[seq & 1u];
     for (int e = tid; e < ntx; e += nthreads) {
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(resident_threads<K, NT>())
         for (int k = 0; k < W; ++k) {
           if (k >= nk) break;
           while ((unsigned)(v[k][j] >> 32) != seq) {
-            if (++polls > kResidentPolls) {
+            if (++polls > d.polls) {
               ok = false;
               break;
             }

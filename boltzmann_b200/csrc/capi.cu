@@ -120,7 +120,8 @@ cudaError_t allocate(lbm_sim* s, const size_t* bytes, void** out, int count) {
 }
 
 // Reads the device status word after a synchronisation: bit 1 means a kernel gave up waiting for
-// its own asynchronous copies (it then stopped early and the state is not valid).
+// its own asynchronous copies (staged) or for its neighbours' messages (resident); it then stopped
+// early and the state is not valid.
 int check_status(lbm_sim* s) {
   int word = 0;
   LBM_CUDA(cudaMemcpyAsync(&word, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -130,7 +131,8 @@ int check_status(lbm_sim* s) {
     const int rest = word & ~2;
     LBM_CUDA(cudaMemcpyAsync(s->status, &rest, sizeof(int), cudaMemcpyHostToDevice, s->stream));
     LBM_CUDA(cudaStreamSynchronize(s->stream));
-    return fail(LBM_ERR_CUDA, "an AA step gave up waiting for its staged copies (status bit 1)");
+    return fail(LBM_ERR_CUDA, "an AA step gave up waiting for its staged copies or its "
+                "neighbours' messages (status bit 1)");
   }
   return LBM_OK;
 }

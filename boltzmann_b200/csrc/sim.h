@@ -32,7 +32,7 @@ struct lbm_sim {
   int device = 0;
   cudaStream_t stream = nullptr;
   int kernel_path = 0;  // LBM_PATH_AUTO / _DIRECT / _STAGED
-  int64_t spin_limit = -1;  // polls of the staged kernel's pipeline waits; < 0: the default
+  int64_t spin_limit = -1;  // polls of the kernels' waits (lbm_set_spin_limit); < 0: the default
   // AA step launches since creation, per kernel variant: [0] direct, [1] TMA-staged.
   mutable int64_t launches[2] = {0, 0};
   // Step pairs captured as CUDA graphs and replayed by lbm_iterate, one per pair count (at most

@@ -164,13 +164,14 @@ LBM_API int lbm_nonfinite(lbm_sim* sim, int* out);
  * counterpart. */
 LBM_API int lbm_set_kernel_path(lbm_sim* sim, int path);
 
-/* Polls that each pipeline wait of the TMA-staged kernel makes before it gives up (the copies of
- * a stage, or its release by the consumer warps); polls < 0 restores the default (2^22). A kernel
- * that gives up sets bit 1 of the status word, still waits (with the default bound) for the
- * copies it issued, and returns; the next synchronising call (lbm_download_fluid,
- * lbm_synchronize) then fails with LBM_ERR_CUDA, once, and the populations are not valid until
- * they are uploaded again. 0 makes every pipeline wait give up at once: a way to exercise that
- * path. No reference counterpart. */
+/* Polls that each wait of a step kernel makes before it gives up: the pipeline waits of the
+ * TMA-staged kernel (the copies of a stage, or its release by the consumer warps) and the waits of
+ * the resident kernel, which takes whole calls of small 2D domains, for its neighbours' messages;
+ * polls < 0 restores the defaults (2^22 and 2^20). A kernel that gives up sets bit 1 of the status
+ * word, still waits (with the default bound) for the copies it issued, and returns; the next
+ * synchronising call (lbm_download_fluid, lbm_synchronize) then fails with LBM_ERR_CUDA, once, and
+ * the populations are not valid until they are uploaded again. 0 makes every wait give up at once:
+ * a way to exercise that path. No reference counterpart. */
 LBM_API int lbm_set_spin_limit(lbm_sim* sim, int64_t polls);
 
 /* AA step launches since lbm_create, per kernel variant: the direct kernel (aa_step_kernel; the

@@ -88,3 +88,12 @@ def test_a_failed_launch_is_reported_once(lib, counts, steps):
     sim.check(lib.lbm_equilibrate(sim.h))
     sim.check(sim.iterate(2))
     sim.close()
+
+
+def test_a_poll_limit_does_not_change_the_kernel(lib):
+    sim = FakeSim(lib, (64, 64))
+    for polls in (0, 1 << 20, -1):
+        sim.check(lib.lbm_set_spin_limit(sim.h, C.c_int64(polls)))
+        sim.check(sim.iterate(20))
+        assert sim.kernels() == ["aa_resident_kernel"]
+    sim.close()
