@@ -185,31 +185,48 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
 
 // Whether the TMA-staged kernel is the faster one for rows of whole 256-cell tiles (fused tracers: none
 // or one). It keeps more loads in flight per SM with fewer instructions, the direct kernel more warps
-// at work: domains that sit in L2, and cells with more arithmetic per byte, are better off direct. us a
-// step, direct / staged, after a second under load (cold, at full clocks, the direct kernel looks up
-// to 5% better), by which the lines are drawn:
-//   D2Q9  FP32         2048x1024 21.7 / 25.7, 3000x1536 64.1 / 63.8, 4096x2048 115.9 / 111.6
-//         with tracer  1024x512 8.3 / 11.0, 2048x1024 44.3 / 43.7, 4096x2048 TRT 176.4 / 171.0
-//         FP64         1500x1024 41.3 / 40.4; with a tracer 4096x1024 168 / 187
-//         FP16         4096x2048 76 / 87, TRT 79.4 / 79.0; with an FP16 tracer 118 / 143
-//   D3Q27 FP32 BGK     48x64x256 24.3 / 23.7, 200x200x256 390 / 356, 128x100x512 251 / 242
-//         FP32 TRT     48x64x256 25.3 / 31.0, 200x200x256 407 / 409, 128x100x512 260 / 354;
-//                      with a tracer 200x200x256 494 / 501 (BGK), 497 / 506
-//         FP16 BGK     32x48x256 9.9 / 10.0, 48x64x256 17.4 / 15.4, 128x100x512 165 / 161
-//         FP16 TRT     48x64x256 18.4 / 17.7, 128x100x512 184 / 233
-//         FP16 tracer  48x64x256 22.5 / 22.7, 100x100x256 90.7 / 70.5, 128x100x512 227 / 289
-//         FP64         48x64x256 61.3 / 57.8; with a tracer 77.4 / 73.6
-template <class L, bool TRT, int K, int NT>
+// at work: domains that sit in L2, and FP32 or FP64 cells with more arithmetic per byte, are better off
+// direct. In 16 bits rows of several tiles pay from some 95 MB of populations, of one tile, whose even
+// steps return by rows too, from half of that. us a step, direct / staged, each the median of a second
+// under its own load:
+//   D2Q9  FP32         2048x1024 20.8 / 26.1, 1500x2560 53.0 / 52.4 (TRT 53.4 / 54.0), 4096x2048
+//                      114 / 111 (TRT 115.2 / 114.9)
+//         with tracer  2048x512 14.6 / 18.7, 2048x1024 43.6 / 43.3; 4096x2048 166 / 174 in a periodic
+//                      box, 176 / 171 in a channel
+//         FP64         2048x512 22.8 / 26.9, 1500x2560 105 / 101; with a tracer, TRT, 164 / 179
+//         FP16         2048x1024 16.8 / 21.6, 4096x2048 73.4 / 77.4 (TRT 78.3 / 78.0)
+//         FP32 tracer  2048x512 12.8 / 15.4, 1500x1536 33.6 / 31.2, 8000x768 94.6 / 90.2
+//         FP16 tracer  1000x2560 31.5 / 33.1, 1500x2560 52.9 / 50.9, 4096x2048 113 / 111; TRT
+//                      1500x1536 29.4 / 30.2, 1000x2560 34.2 / 33.5, 4096x2048 121 / 111
+//   D3Q27 FP32 BGK     24x48x256 8.1 / 10.1, 48x64x256 24.4 / 24.0, 128x100x512 245 / 241
+//         FP32 TRT     48x64x256 25.4 / 31.8, 100x100x256 101 / 107, 128x100x512 255 / 356;
+//                      with a tracer 100x100x256 121 / 132, 128x100x512 307 / 436
+//         FP64         24x48x256 19.5 / 20.5, 48x64x256 64.3 / 60.8; with a tracer 82.4 / 74.9
+//         FP16 BGK     24x48x256 7.7 / 8.6, 48x64x256 17.4 / 15.9; 48x64x512 35.9 / 38.2, 40x90x512
+//                      44.3 / 43.7, 128x100x512 159 / 157
+//         FP16 TRT     24x48x256 7.9 / 9.4, 48x64x256 18.3 / 18.1, 100x100x256 73.4 / 53.8; 48x64x512
+//                      38.8 / 40.6, 40x90x512 50.2 / 46.9, 128x100x512 184 / 160, 100x100x1024 286 / 249
+//         FP32 tracer  24x48x256 9.7 / 11.4, 48x64x256 23.8 / 22.4; 32x48x512 23.7 / 26.4, 24x48x1024
+//                      43.3 / 41.4, 128x100x512 248 / 222 (TRT 272 / 234)
+//         FP16 tracer  24x48x256 9.7 / 11.3, 48x64x256 22.6 / 21.8; 24x48x1024 36.4 / 38.2, 48x64x512
+//                      54.5 / 51.3, 128x100x512 226 / 202; TRT 64x64x256 32.2 / 33.7, 64x90x256
+//                      52.9 / 48.0, 48x64x512 56.1 / 55.7, 128x100x512 230 / 215
+// KT: storage kind of the tracer's populations.
+template <class L, bool TRT, int K, int NT, int KT>
 bool staged_pays(const StepArgs<typename Pop<K>::real>& a) {
   const long long cells = (long long)a.nx * a.ny * a.nz;
+  constexpr bool wide_tracer = KT == kF32;
   if (L::D == 2) {
-    if (K == kF32) return cells >= (NT == 0 ? 6000000 : 2000000);
-    return K == kF64 && NT == 0 && cells >= 1500000;
+    if (K == kF64) return NT == 0 && cells >= 1500000;
+    if (K == kF32) return cells >= (NT == 0 ? (TRT ? 6000000 : 3500000) : 2000000);
+    return NT != 0 && cells >= (wide_tracer ? 2200000 : (TRT ? 2500000 : 3000000));
   }
-  if (dev_in<K>() && (TRT || NT != 0))
-    return a.nz == kTmaTile && cells >= (NT == 0 ? 700000 : 1500000);
   if (K == kF32 && (TRT || NT != 0)) return false;
-  return cells >= 700000;
+  if (!dev_in<K>()) return cells >= 700000;
+  const bool one_tile = a.nz == kTmaTile;
+  if (NT == 0) return cells >= (one_tile ? 700000 : 1700000);
+  if (wide_tracer) return cells >= (one_tile ? 750000 : 1100000);
+  return cells >= (one_tile ? (TRT ? 1200000 : 750000) : 1400000);
 }
 
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
@@ -217,7 +234,7 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
                        int64_t* launches) {
   if constexpr (NT >= 0) {
     const bool fits = a.nz % kTmaTile == 0;
-    const bool staged = a.path == 2 || (a.path == 0 && staged_pays<L, TRT, K, NT>(a));
+    const bool staged = a.path == 2 || (a.path == 0 && staged_pays<L, TRT, K, NT, KT>(a));
     if (fits && staged) {
       cudaError_t e;
       if (EVEN && a.nz == kTmaTile)

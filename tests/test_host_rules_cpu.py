@@ -97,3 +97,29 @@ def test_a_poll_limit_does_not_change_the_kernel(lib):
         sim.check(sim.iterate(20))
         assert sim.kernels() == ["aa_resident_kernel"]
     sim.close()
+
+
+@pytest.mark.parametrize("counts,storage,kind,tracer,staged", [
+    # Rows of several tiles, 16-bit storage in 3D: staged from what L2 no longer holds.
+    ((32, 48, 512), "f16", 1, "", False), ((70, 90, 512), "f16", 1, "", True),
+    ((32, 48, 1024), "f16", 0, "", False), ((70, 45, 1024), "bf16", 0, "", True),
+    ((32, 48, 512), "f16", 1, "32", False), ((48, 64, 512), "f16", 1, "32", True),
+    ((32, 48, 512), "f16", 0, "16", False), ((40, 90, 768), "bf16", 1, "16", True),
+    # Rows of one tile.
+    ((24, 48, 256), "f16", 1, "", False), ((64, 64, 256), "f16", 1, "", True),
+    ((64, 64, 256), "f16", 0, "32", True), ((64, 64, 256), "f16", 0, "16", True),
+    ((64, 64, 256), "f16", 1, "16", False), ((64, 90, 256), "f16", 1, "16", True),
+    # 2D.
+    ((4096, 2048), "f16", 1, "", False), ((2048, 512), "f16", 0, "32", False),
+    ((1500, 1536), "f16", 0, "32", True), ((1500, 1536), "f16", 1, "16", False),
+    ((1500, 2560), "f16", 1, "16", True), ((1500, 2560), "bf16", 0, "16", True),
+    ((1500, 2560), "f32", 0, "", True), ((1500, 2560), "f32", 1, "", False),
+    ((1500, 2560), "f64", 1, "64", False), ((1500, 2560), "f64", 0, "", True),
+])
+def test_staged_where_it_is_the_faster_kernel(lib, counts, storage, kind, tracer, staged):
+    """One domain on each side of every line of staged_pays (aa_launch.cuh) that is not obvious."""
+    sim = FakeSim(lib, counts, kind=kind, storage=storage, tracer=tracer)
+    sim.check(sim.iterate(2))
+    kernels = set(sim.kernels())
+    assert kernels == {"aa_tma_kernel"} if staged else "aa_tma_kernel" not in kernels
+    sim.close()
