@@ -135,11 +135,26 @@ size_t mail_bytes(lbm_sim& s) {
          resident_slots<K, NT>() * plan.args.published * 8;
 }
 
+// Whether a simulation that is stepped beside others (threads, streams) should still take the resident
+// kernel: resident launches whose CTAs do not fit the chip side by side take turns, while the single
+// steps of several small domains overlap. us a step and simulation, single steps / resident, in calls
+// of 200 steps by a thread each: 128^2 two at once 0.97 / 1.05, three 0.80 / 1.03, eight 0.36 / 1.02;
+// 256^2 two 1.29 / 1.33, three 1.00 / 1.31, eight 0.66 / 1.30; 400 x 350 three 1.46 / 1.77; 512 x 500
+// four 2.30 / 2.46, eight 2.35 / 2.46; 64^2, of which two fit, four 0.51 / 0.48, eight 0.30 / 0.47. The
+// line lies at three turns, below 200,000 cells. The results are the same either way.
+bool worth_waiting(const lbm_sim& s, const ResidentArgs& d) {
+  if (s.n >= 200000) return true;
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device);
+  return (int64_t)simulations_in_flight(s.device) * d.gy * d.gz <= 2 * (int64_t)sms;
+}
+
 template <int K, int NT, int KT>
 cudaError_t iterate(lbm_sim& s, int64_t steps) {
   ResidentPlan plan;
   if (s.mail[1] == nullptr || s.mail_tracers != NT || !plan_here<K, NT, KT>(s, plan))
     return cudaErrorNotSupported;
+  if (!worth_waiting(s, plan.args)) return cudaErrorNotSupported;
   return s.collision == 1 ? run<true, K, NT, KT>(s, plan, steps)
                           : run<false, K, NT, KT>(s, plan, steps);
 }

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -51,6 +52,24 @@ int activate(lbm_sim* s) {
   if (s == nullptr) return fail(LBM_ERR_ARGUMENT, "null simulation handle");
   cudaError_t e = cudaSetDevice(s->device);
   if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
+  return LBM_OK;
+}
+
+// Simulations in flight, by device (those beyond the last share its entry).
+constexpr int kDevices = 64;
+std::atomic<int> g_in_flight[kDevices];
+
+std::atomic<int>& in_flight_on(int device) { return g_in_flight[std::min(device, kDevices - 1)]; }
+
+void set_in_flight(lbm_sim* s, bool on) {
+  if (s->in_flight != on) in_flight_on(s->device) += on ? 1 : -1;
+  s->in_flight = on;
+}
+
+// Waits for the simulation's stream.
+int finish(lbm_sim* s) {
+  LBM_CUDA(cudaStreamSynchronize(s->stream));
+  set_in_flight(s, false);
   return LBM_OK;
 }
 
@@ -125,7 +144,7 @@ cudaError_t allocate(lbm_sim* s, const size_t* bytes, void** out, int count) {
 int check_status(lbm_sim* s) {
   int word = 0;
   LBM_CUDA(cudaMemcpyAsync(&word, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  LBM_CUDA(cudaStreamSynchronize(s->stream));
+  if (int rc = finish(s)) return rc;
   if (word & 2) {
     // Reported once: the bit is cleared so that the simulation can be restored and run again.
     const int rest = word & ~2;
@@ -146,6 +165,7 @@ void drop_graph(lbm_sim* s) {
 }
 
 void release(lbm_sim* s) {
+  set_in_flight(s, false);
   drop_graph(s);
   for (void* p : s->owned) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -210,6 +230,8 @@ int step_launch_fail(cudaError_t e) {
 }
 
 }  // namespace
+
+int lbm::simulations_in_flight(int device) { return in_flight_on(device); }
 
 void lbm::set_last_error(const std::string& msg) { g_error = msg; }
 
@@ -416,8 +438,7 @@ int lbm_upload_flags(lbm_sim* sim, const int32_t* flags) {
     LBM_CUDA(lbm::flags_to_u8(static_cast<const int32_t*>(sim->scratch), sim->flags + at, count,
                               sim->stream));
   }
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_upload_fluid(lbm_sim* sim, const float* rho, const float* vel) {
@@ -428,16 +449,14 @@ int lbm_upload_fluid(lbm_sim* sim, const float* rho, const float* vel) {
   if (vel) {
     if (int rc = upload_reals(sim, sim->vel, vel, sim->n * sim->dim)) return rc;
   }
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_upload_tracer(lbm_sim* sim, int tracer, const float* val) {
   if (int rc = activate(sim)) return rc;
   if (int rc = check_tracer(sim, tracer)) return rc;
   if (int rc = upload_reals(sim, sim->tracers[tracer].val, val, sim->n)) return rc;
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_equilibrate(lbm_sim* sim) {
@@ -477,8 +496,7 @@ static int transfer_populations(lbm_sim* sim, int tracer, float* host, bool to_d
   cudaFreeAsync(tmp, sim->stream);
   if (e == cudaErrorNotSupported) return fail(LBM_ERR_UNSUPPORTED, "no layout for this set");
   if (e != cudaSuccess) return cuda_fail(e, "populations transfer");
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_upload_f(lbm_sim* sim, const float* f) {
@@ -513,6 +531,7 @@ int lbm_iterate(lbm_sim* sim, int64_t iters) {
   const bool outer = cudaStreamIsCapturing(sim->stream, &cs) == cudaSuccess &&
                      cs != cudaStreamCaptureStatusNone;
   if (!outer) {
+    set_in_flight(sim, true);
     // (Not into a caller's graph: its replays would repeat the sequence numbers.)
     const cudaError_t e = lbm::iterate_resident(*sim, iters);
     if (e != cudaErrorNotSupported) return e == cudaSuccess ? LBM_OK : step_launch_fail(e);
@@ -557,8 +576,7 @@ int lbm_download_tracer(lbm_sim* sim, int tracer, float* val) {
   if (int rc = activate(sim)) return rc;
   if (int rc = check_tracer(sim, tracer)) return rc;
   if (int rc = download_reals(sim, val, sim->tracers[tracer].val, sim->n)) return rc;
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_download_fluid_f64(lbm_sim* sim, double* rho, double* vel) {
@@ -571,8 +589,7 @@ int lbm_download_fluid_f64(lbm_sim* sim, double* rho, double* vel) {
   if (vel)
     LBM_CUDA(cudaMemcpyAsync(vel, sim->vel, sim->n * sim->dim * sizeof(double),
                              cudaMemcpyDeviceToHost, sim->stream));
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_conservation(lbm_sim* sim, double* out, int len) {
@@ -586,8 +603,7 @@ int lbm_conservation(lbm_sim* sim, double* out, int len) {
   if (e != cudaSuccess) return cuda_fail(e, "conservation sums");
   LBM_CUDA(cudaMemcpyAsync(out, sim->sums, need * sizeof(double), cudaMemcpyDeviceToHost,
                            sim->stream));
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return LBM_OK;
+  return finish(sim);
 }
 
 int lbm_nonfinite(lbm_sim* sim, int* out) {
@@ -595,7 +611,7 @@ int lbm_nonfinite(lbm_sim* sim, int* out) {
   int word = 0;
   LBM_CUDA(cudaMemcpyAsync(&word, sim->status, sizeof(int), cudaMemcpyDeviceToHost, sim->stream));
   LBM_CUDA(cudaMemsetAsync(sim->status, 0, sizeof(int), sim->stream));
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
+  if (int rc = finish(sim)) return rc;
   if (out) *out = word & 1;
   return LBM_OK;
 }
@@ -641,8 +657,7 @@ int lbm_fluid_device(lbm_sim* sim, void** rho, void** vel) {
 
 int lbm_synchronize(lbm_sim* sim) {
   if (int rc = activate(sim)) return rc;
-  LBM_CUDA(cudaStreamSynchronize(sim->stream));
-  return check_status(sim);
+  return check_status(sim);  // waits for the stream
 }
 
 int lbm_stream(lbm_sim* sim, void** stream) {

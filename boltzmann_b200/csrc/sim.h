@@ -47,6 +47,9 @@ struct lbm_sim {
   bool graph_warm = false, graph_failed = false;
   const float* omega_field = nullptr;  // caller-owned per-cell om_pos, or null
 
+  // Steps enqueued by lbm_iterate that no synchronising call has waited for yet (see in_flight()).
+  bool in_flight = false;
+
   std::vector<void*> owned;  // the device allocations behind the arrays below and the tracers'
   // Fields on their way to or from the host: flags as int32 (in pieces where they do not fit), and
   // FP64 fields as floats. Its users follow one another on the stream.
@@ -97,6 +100,9 @@ cudaError_t launch_step_d3q27(const lbm_sim& sim, bool even, bool write_moments)
 // The whole call of `steps` steps (even, moments at the end) in one launch that keeps the domain on the
 // chip (aa_resident.cu). cudaErrorNotSupported, with nothing enqueued, when it does not apply.
 cudaError_t iterate_resident(lbm_sim& sim, int64_t steps);
+// The simulations of a device with steps in flight, as far as the host knows: from lbm_iterate to the
+// next call that waits for the simulation's stream.
+int simulations_in_flight(int device);
 // Bytes of one set of its message words for a simulation with `tracers` tracers; 0 when it does not apply.
 size_t resident_mail_bytes(lbm_sim& sim, int tracers);
 

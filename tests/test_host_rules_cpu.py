@@ -123,3 +123,30 @@ def test_staged_where_it_is_the_faster_kernel(lib, counts, storage, kind, tracer
     kernels = set(sim.kernels())
     assert kernels == {"aa_tma_kernel"} if staged else "aa_tma_kernel" not in kernels
     sim.close()
+
+
+def test_small_simulations_side_by_side_do_not_queue_for_the_chip(lib):
+    """Resident launches that would take three turns or more give way to single steps, which overlap,
+    while the simulations before them have not been waited for."""
+
+    def kernels(counts, together):
+        sims = [FakeSim(lib, counts) for _ in range(together)]
+        out = []
+        for s in sims:
+            s.check(s.iterate(14))
+            out.append(set(s.kernels()))
+        # A simulation that has been waited for does not count: one of them alone, in turn.
+        for s in sims:
+            s.check(lib.lbm_synchronize(s.h))
+        for s in sims:
+            s.check(s.iterate(14))
+            assert set(s.kernels()) == {"aa_resident_kernel"}
+            s.check(lib.lbm_synchronize(s.h))
+        for s in sims:
+            s.close()
+        return [k == {"aa_resident_kernel"} for k in out]
+
+    assert kernels((128, 128), 4) == [True, True, False, False]
+    assert kernels((64, 64), 6) == [True] * 4 + [False] * 2  # 64 of 148 CTAs each
+    assert kernels((600, 400), 4) == [True] * 4  # large enough to be faster in turns
+    assert kernels((12, 13), 20) == [True] * 20  # a few CTAs each
