@@ -342,7 +342,7 @@ def run_ours(args) -> None:
     barrier()
     torch.cuda.synchronize()
     sim._synchronize()
-    before = sim._launch_counts()
+    before = sim._kernel_launches()
     with ClockSampler(local) as clocks:
         t_wall0 = time.time()
         start.record(stream)
@@ -350,7 +350,7 @@ def run_ours(args) -> None:
         stop.record(stream)
         stop.synchronize()
         clocks.mark(t_wall0, time.time())
-    after = sim._launch_counts()
+    after = sim._kernel_launches()
     barrier()
     torch.cuda.synchronize()
     elapsed_ms = max_over_ranks(start.elapsed_time(stop))
@@ -362,11 +362,10 @@ def run_ours(args) -> None:
     total_steps = sim.iteration
     del sim
     # The kernels the library launched in the timed region, from its own counters.
-    direct, staged = after[0] - before[0], after[1] - before[1]
-    launches = direct + staged
-    kernel = ("aa_tma_kernel" if staged == launches else
-              "aa_step_kernel" if direct == launches else
-              f"aa_tma_kernel x{staged} + aa_step_kernel x{direct}")
+    by_kernel = {k: after[k] - before[k] for k in after if after[k] != before[k]}
+    launches = sum(by_kernel.values())
+    kernel = (next(iter(by_kernel)) if len(by_kernel) == 1 else
+              " + ".join(f"{k} x{v}" for k, v in by_kernel.items()))
 
     l2 = None
     if args.storage != "f64" and not args.no_l2:
@@ -453,7 +452,7 @@ def run_ours(args) -> None:
                 "runs": e2e_runs,
             },
             "gpu_launches": launches,
-            "launches_by_kernel": {"aa_tma_kernel": staged, "aa_step_kernel": direct},
+            "launches_by_kernel": by_kernel,
             "clocks": clocks.summary(),
             "finite": finite,
             "l2_vs_f64": l2,
@@ -555,6 +554,9 @@ def run_ensemble(args) -> None:
     finite_domains = int(group.sum(sum(
         bool(np.isfinite(ens.rho[sl]).all()) for sl in setup.domain_slices()
     )))
+    flat = tuned["tile"] in (0, 128) and tuned["blocks_per_sm"] == 0 and ens.flat
+    ens_kernel = ("ensemble_flat_kernel" if flat else
+                  "ensemble_rows_kernel" if tuned["tile"] == 0 else "ensemble_step_kernel")
     del ens
 
     e2 = fresh()
@@ -570,7 +572,6 @@ def run_ensemble(args) -> None:
     bpc = {"f32": 72.0, "f16": 36.0, "bf16": 36.0}[args.storage]
     peaks, peak_kind = measured_peaks()
     achieved = bpc * n * 2 * K / (graph_ms * 1e-3) / 1e9 / world  # per GPU
-    ens_kernel = "ensemble_rows_kernel" if tuned["tile"] == 0 else "ensemble_step_kernel"
     # DRAM bytes per cell update (ncu) of the kernel the tuned shape runs
     ens_traffic, ens_traffic_src = profiled_traffic(ens_kernel, "ensemble")
     cpu = None if (args.no_cpu_baseline or world > 1) else cpu_ensemble_rate(setup, args.cpu_seconds)
@@ -755,7 +756,7 @@ def run_closure(args) -> None:
             "frac": achieved_tf / peak_tf,
             "traffic": None,
             "peak_source": f"{peak_kind} (MEASURED_PEAKS.json bf16_tflops)",
-            "kernel": "closure forward (conv1 + conv32 mma.sync + conv3), batch 8 x 1024x512",
+            "kernel": "closure forward (conv1_fwd + conv32_tc + conv3_fwd), batch 8 x 1024x512",
             "flops_per_cell": 21_312,
             "forward_ms": fwd_s * 1e3,
         },
@@ -768,7 +769,7 @@ def run_closure(args) -> None:
             "how": f"run_closed_or_fine ({kind}) from host arrays, host wall clock, against the "
             "fine run's device time",
         },
-        "gpu_launches": coarse_steps + 5 * (coarse_steps // cfg.every),
+        "gpu_launches": coarse_steps + coarse_steps // cfg.every,
         "clocks": clocks.summary(),
         "pipeline_seconds": pipeline_s,
     }

@@ -241,7 +241,10 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
         e = launch_tma<L, TRT, K, EVEN, NT, EVEN, KT>(a, stream);
       else
         e = launch_tma<L, TRT, K, EVEN, NT, false, KT>(a, stream);
-      if (e == cudaSuccess) ++launches[1];
+      if (e == cudaSuccess) {
+        ++launches[lbm_sim::kStagedSteps];
+        ++launches[lbm_sim::kKernels + LBM_KERNEL_STAGED];
+      }
       return e;
     }
   }
@@ -252,14 +255,20 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
       const unsigned grid = (unsigned)(((long long)d.cells + 2 * kDirectThreads - 1) / (2 * kDirectThreads));
       const cudaError_t e = launch_step_kernel(aa_step2_kernel<L, TRT, K, EVEN, NT, KT>, grid,
                                                kDirectThreads, 0, stream, a, d);
-      if (e == cudaSuccess) ++launches[0];
+      if (e == cudaSuccess) {
+        ++launches[lbm_sim::kDirectSteps];
+        ++launches[lbm_sim::kKernels + LBM_KERNEL_STEP2];
+      }
       return e;
     }
   }
   const unsigned grid = (unsigned)(((long long)d.cells + kDirectThreads - 1) / kDirectThreads);
   const cudaError_t e = launch_step_kernel(aa_step_kernel<L, TRT, K, EVEN, NT, KT>, grid,
                                            kDirectThreads, 0, stream, a, d);
-  if (e == cudaSuccess) ++launches[0];
+  if (e == cudaSuccess) {
+    ++launches[lbm_sim::kDirectSteps];
+    ++launches[lbm_sim::kKernels + LBM_KERNEL_STEP];
+  }
   return e;
 }
 

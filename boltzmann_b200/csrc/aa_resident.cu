@@ -114,7 +114,8 @@ cudaError_t run(lbm_sim& s, const ResidentPlan& plan, int64_t steps) {
       return cudaErrorNotSupported;
     }
     s.mail_seq += (unsigned)(now / 2);
-    s.launches[0] += now;
+    s.launches[lbm_sim::kDirectSteps] += now;
+    ++s.launches[lbm_sim::kKernels + LBM_KERNEL_RESIDENT];
   }
   return cudaSuccess;
 }

@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <new>
 #include <string>
 #include <vector>
@@ -204,15 +205,16 @@ const lbm_sim::StepGraph* step_graph(lbm_sim* s, int64_t pairs) {
     cudaGraphExecDestroy(s->graphs.front().exec);
     s->graphs.erase(s->graphs.begin());
   }
-  lbm_sim::StepGraph g{pairs, nullptr, {0, 0}};
-  const int64_t before[2] = {s->launches[0], s->launches[1]};
+  lbm_sim::StepGraph g{pairs, nullptr, {}};
+  int64_t before[lbm_sim::kCounts];
+  std::copy(std::begin(s->launches), std::end(s->launches), before);
   cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return nullptr;
   cudaError_t le = cudaSuccess;
   for (int64_t p = 0; p < pairs && le == cudaSuccess; ++p) le = launch_pair(s, false);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s->stream, &graph);
-  for (int k = 0; k < 2; ++k) {
+  for (int k = 0; k < lbm_sim::kCounts; ++k) {
     g.launches[k] = s->launches[k] - before[k];
     s->launches[k] = before[k];
   }
@@ -551,8 +553,7 @@ int lbm_iterate(lbm_sim* sim, int64_t iters) {
         break;
       }
       LBM_CUDA(cudaGraphLaunch(g->exec, sim->stream));
-      sim->launches[0] += g->launches[0];
-      sim->launches[1] += g->launches[1];
+      for (int k = 0; k < lbm_sim::kCounts; ++k) sim->launches[k] += g->launches[k];
       left -= pairs;
     }
   }
@@ -634,8 +635,16 @@ int lbm_set_spin_limit(lbm_sim* sim, int64_t polls) {
 
 int lbm_launch_counts(lbm_sim* sim, int64_t* direct, int64_t* staged) {
   if (int rc = activate(sim)) return rc;
-  if (direct) *direct = sim->launches[0];
-  if (staged) *staged = sim->launches[1];
+  if (direct) *direct = sim->launches[lbm_sim::kDirectSteps];
+  if (staged) *staged = sim->launches[lbm_sim::kStagedSteps];
+  return LBM_OK;
+}
+
+int lbm_kernel_launches(lbm_sim* sim, int64_t* counts, int len) {
+  if (int rc = activate(sim)) return rc;
+  constexpr int kernels = lbm_sim::kCounts - lbm_sim::kKernels;
+  if (counts == nullptr || len < kernels) return fail(LBM_ERR_ARGUMENT, "output needs 4 counts");
+  std::copy_n(sim->launches + lbm_sim::kKernels, kernels, counts);
   return LBM_OK;
 }
 

@@ -572,6 +572,17 @@ PYBIND11_MODULE(boltzmann, m) {
              check(lbm_launch_counts(s.st->h, &direct, &staged));
              return py::make_tuple(direct, staged);
            })
+      .def("_kernel_launches",
+           [](const Simulation& s) {
+             // Launches of AA steps so far, by kernel.
+             int64_t counts[4];
+             check(lbm_kernel_launches(s.st->h, counts, 4));
+             py::dict out;
+             const char* names[4] = {"aa_step_kernel", "aa_step2_kernel", "aa_tma_kernel",
+                                     "aa_resident_kernel"};
+             for (int k = 0; k < 4; ++k) out[names[k]] = counts[k];
+             return out;
+           })
       .def("_synchronize", [](const Simulation& s) { check(lbm_synchronize(s.st->h)); })
       .def("_stream", [](const Simulation& s) {
         void* p = nullptr;

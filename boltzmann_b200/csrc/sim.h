@@ -7,6 +7,8 @@
 #include <string>
 #include <vector>
 
+#include "../../include/lbm_cuda.h"
+
 struct lbm_sim {
   struct Tracer {
     int q = 0;
@@ -33,15 +35,17 @@ struct lbm_sim {
   cudaStream_t stream = nullptr;
   int kernel_path = 0;  // LBM_PATH_AUTO / _DIRECT / _STAGED
   int64_t spin_limit = -1;  // polls of the kernels' waits (lbm_set_spin_limit); < 0: the default
-  // AA step launches since creation, per kernel variant: [0] direct, [1] TMA-staged.
-  mutable int64_t launches[2] = {0, 0};
+  // Since creation: AA steps by variant (the resident kernel's count as direct ones), and the launches
+  // of each kernel (enum lbm_kernel).
+  enum Count { kDirectSteps, kStagedSteps, kKernels, kCounts = kKernels + 4 };
+  mutable int64_t launches[kCounts] = {};
   // Step pairs captured as CUDA graphs and replayed by lbm_iterate, one per pair count (at most
   // four), dropped whenever a setter changes what a step launches; `warm` once a pair has run
   // outside any capture in the current state (each kernel's one-time launch set-up done).
   struct StepGraph {
     int64_t pairs;
     cudaGraphExec_t exec;
-    int64_t launches[2];  // what one replay adds to `launches`
+    int64_t launches[kCounts];  // what one replay adds to `launches`
   };
   std::vector<StepGraph> graphs;
   bool graph_warm = false, graph_failed = false;

@@ -174,10 +174,21 @@ LBM_API int lbm_set_kernel_path(lbm_sim* sim, int path);
  * a way to exercise that path. No reference counterpart. */
 LBM_API int lbm_set_spin_limit(lbm_sim* sim, int64_t polls);
 
-/* AA step launches since lbm_create, per kernel variant: the direct kernel (aa_step_kernel; the
- * steps of resident launches count here, one each) and the TMA-staged one (aa_tma_kernel). Host-side counters, no synchronisation. No reference
- * counterpart (instrumentation: which kernel a workload actually ran). */
+/* AA steps since lbm_create, per kernel variant: the direct kernels (aa_step_kernel, its two-cell
+ * form aa_step2_kernel, and the steps of the resident kernel) and the TMA-staged one (aa_tma_kernel).
+ * Host-side counters, no synchronisation. No reference counterpart (instrumentation). */
 LBM_API int lbm_launch_counts(lbm_sim* sim, int64_t* direct, int64_t* staged);
+
+/* Kernel launches of AA steps since lbm_create, by kernel: counts[enum lbm_kernel], len >= 4. A launch
+ * is one step, but for the resident kernel, which takes up to 4000. Host-side counters, no
+ * synchronisation. No reference counterpart (instrumentation: which kernel a workload actually ran). */
+enum lbm_kernel {
+  LBM_KERNEL_STEP = 0,     /* aa_step_kernel */
+  LBM_KERNEL_STEP2 = 1,    /* aa_step2_kernel: two cells a thread */
+  LBM_KERNEL_STAGED = 2,   /* aa_tma_kernel */
+  LBM_KERNEL_RESIDENT = 3, /* aa_resident_kernel */
+};
+LBM_API int lbm_kernel_launches(lbm_sim* sim, int64_t* counts, int len);
 
 /* Per-cell relaxation rate: `field` is a device array of N floats (omega+ of every cell) that
  * the caller owns and keeps alive, written on the simulation's stream (a learned closure's output);

@@ -150,3 +150,20 @@ def test_small_simulations_side_by_side_do_not_queue_for_the_chip(lib):
     assert kernels((64, 64), 6) == [True] * 4 + [False] * 2  # 64 of 148 CTAs each
     assert kernels((600, 400), 4) == [True] * 4  # large enough to be faster in turns
     assert kernels((12, 13), 20) == [True] * 20  # a few CTAs each
+
+
+@pytest.mark.parametrize("counts,storage,steps,launches", [
+    ((64, 64), "f32", 8004, [0, 0, 0, 3]), ((64, 64), "f32", 2, [2, 0, 0, 0]),
+    ((400, 390), "f16", 6, [0, 6, 0, 0]), ((50, 40, 30), "f32", 30, [30, 0, 0, 0]),
+    ((64, 64, 256), "f32", 30, [0, 0, 30, 0])])
+def test_launches_are_counted_by_kernel(lib, counts, storage, steps, launches):
+    sim = FakeSim(lib, counts, storage=storage)
+    sim.check(sim.iterate(steps))
+    got = (C.c_int64 * 4)()
+    sim.check(lib.lbm_kernel_launches(sim.h, got, 4))
+    assert list(got) == launches
+    direct, staged = C.c_int64(), C.c_int64()
+    sim.check(lib.lbm_launch_counts(sim.h, C.byref(direct), C.byref(staged)))
+    assert (direct.value, staged.value) == ((0, steps) if launches[2] else (steps, 0))
+    assert lib.lbm_kernel_launches(sim.h, got, 3) != 0 and lib.lbm_kernel_launches(sim.h, None, 4) != 0
+    sim.close()
