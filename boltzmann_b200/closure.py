@@ -224,7 +224,8 @@ def relaxation(net: Net, rho, vel, flags, nx: int, ny: int, tau0: float, omega, 
 
 
 def status() -> None:
-    """Raises if a fused relaxation kernel gave up waiting on its tensor cores (synchronous)."""
+    """Raises, once, if a closure kernel (the fused relaxation or layer 2 in training) gave up waiting
+    for its copies or tensor-core products since the last query (synchronous)."""
     _check(_lib.lbm_closure_status())
 
 
@@ -434,7 +435,8 @@ class TrainReport:
 
 
 def train(cfg: Config, data: Dataset, net: Net | None = None, log_every: int = 20) -> tuple[Net, TrainReport]:
-    """Adam on the masked MSE between the network output and sqrt(k_sgs) / scale."""
+    """Adam on the masked MSE between the network output and sqrt(k_sgs) / scale. Raises where the loss
+    is read, and at the end, if a kernel gave up waiting."""
     torch = _torch()
     S, nx, ny = data.rho.shape
     flags = coarse_setup(cfg).flags
@@ -465,6 +467,7 @@ def train(cfg: Config, data: Dataset, net: Net | None = None, log_every: int = 2
         opt.step(bufs.grad, stream, lr=lr)
         if it % log_every == 0 or it == cfg.iters - 1:
             report.losses.append((it, float(bufs.loss.item())))
+            status()  # a step whose kernels gave up has a wrong gradient
     e1.record()
     e1.synchronize()
     report.seconds = e0.elapsed_time(e1) / 1e3

@@ -1321,8 +1321,9 @@ __device__ __forceinline__ void cl_mbar_init(uint64_t* bar, unsigned count) {
                : "memory");
 }
 
-// Polls of the fused kernel's wait for its tensor-core products before it gives up
-// (lbm_closure_set_spin_limit); the wait that drains MMAs still in flight keeps the default.
+// Polls of a wait for tensor-core products before it gives up, in the fused kernel and in the epilogues
+// of the training kernels (lbm_closure_set_spin_limit); the waits of the warps that copy and issue, and
+// those that drain what is still in flight, keep the default.
 __device__ unsigned g_closure_spin_limit = kClosureSpinLimit;
 
 // Bounded wait for the phase with the given parity; false after `limit` polls.
@@ -2617,7 +2618,7 @@ int lbm_closure_status(void) {
   const int zero = 0;
   CL_CUDA(cudaMemcpyToSymbol(g_closure_status, &zero, sizeof(int)));
   return fail(LBM_ERR_STATE,
-              "closure relaxation: a kernel gave up waiting for its tensor-core products");
+              "closure: a kernel gave up waiting for its copies or tensor-core products");
 }
 
 int lbm_closure_coarsen(const float* rho, const float* vel, const float* c, int64_t nx, int64_t ny,

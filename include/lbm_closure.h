@@ -132,16 +132,17 @@ LBM_API int lbm_closure_relaxation(const float* params, const uint16_t* params_b
 #define LBM_CLOSURE_LAYER2_WARP_MMA 1
 LBM_API int lbm_closure_set_layer2_kernel(int kind);
 
-/* Polls that the lbm_closure_relaxation kernel makes, on the current device, while waiting for
- * its tensor-core products before it gives up (polls < 0: the default, 2^22). A kernel that gives
- * up records it for lbm_closure_status, still waits (with the default bound) for the products in
- * flight, frees its tensor memory and returns; 0 makes the wait give up at once, a way to exercise
- * that path. Synchronous. No reference counterpart. */
+/* Polls that a closure kernel makes, on the current device, while waiting for its tensor-core products
+ * before it gives up (polls < 0: the default, 2^22): the kernel of lbm_closure_relaxation, and those of
+ * layer 2 in lbm_closure_forward and lbm_closure_backward (LBM_CLOSURE_LAYER2_TCGEN05). A kernel that
+ * gives up records it for lbm_closure_status, still waits (with the default bound) for the copies and
+ * products in flight, frees its tensor memory and returns; 0 makes the wait give up at once, a way to
+ * exercise that path. Synchronous. No reference counterpart. */
 LBM_API int lbm_closure_set_spin_limit(int64_t polls);
 
-/* LBM_OK, or LBM_ERR_STATE when a lbm_closure_relaxation kernel on the current device gave up
- * waiting for its tensor-core products (bounded wait) since the last call; its omega is then
- * incomplete. Synchronous; clears the condition. */
+/* LBM_OK, or LBM_ERR_STATE when such a kernel on the current device gave up waiting (bounded waits)
+ * since the last call; its omega, activations or gradient are then incomplete, and a training step
+ * made of them must not be kept. Synchronous; clears the condition. */
 LBM_API int lbm_closure_status(void);
 
 /* Box filter of a fine state onto the coarse lattice (factor f, nx and ny multiples of f):
