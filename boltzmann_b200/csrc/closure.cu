@@ -699,8 +699,8 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
 // cell, P[q][tap] = sum_ci w3[tap][ci] a2[q][ci], whose nine shifted values each output adds: every
 // activation is read and widened once instead of nine times. FP32 on packed instructions (two
 // channels each): tensor cores would do it for less, but their accumulation leans to one side, and
-// the loss, an average over all cells, shows it. Three cells a thread, so that each shared-memory
-// weight load feeds four of them. Batch 8 x 1024 x 512: 216 -> 118 us.
+// the loss, an average over all cells, shows it. Two cells a thread, in three passes, so that each
+// shared-memory weight load feeds four of them. Batch 8 x 1024 x 512: 216 -> 118 us.
 
 constexpr int kC3R = 30;                          // output rows of a tile (kTY columns)
 constexpr int kC3RegR = kC3R + 2, kC3RegC = kHY;  // region with the halo
