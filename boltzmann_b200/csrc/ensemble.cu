@@ -114,9 +114,13 @@ __global__ void __launch_bounds__(512)
 // For ensembles whose populations sit in L2, where the row-staged kernel's ring (a row a stage, its
 // fill and drain every step, whole SMs waiting on a launch) is longer than the work. us a step, row-
 // staged and flat: 9 domains of 210,371 cells in all 5.6 / 3.3, 72 of 369,358 11.2 / 5.1, 64 of
-// 1,574,641 25.2 / 16.5, FP16 32 of 3,734,984 38.2 / 34.7; past L2 32 of 3,734,984 52.4 / 58.6, FP16
-// 128 of 13,045,701 130 / 168.
-constexpr size_t kFlatBytes = 90u << 20;  // of populations
+// 1,574,641 25.2 / 16.5. Both lines lie before L2 is full. Rows of some 500 cells suit the ring: 75 MB
+// 22.5 / 21.8, FP16 79 MB 42.9 / 42.7, 93 MB 28.5 / 30.4, 29.7 / 36.4 (TRT), FP16 47.7 / 57.4. Rows
+// of 64 to 128 do not: 93 MB 54.0 / 36.8, FP16 89.0 / 56.0. Past L2 32 domains of 3,734,984 52.4 / 58.6,
+// FP16 128 of 13,045,701 130 / 168.
+constexpr size_t kFlatBytes = 90u << 20;        // of populations
+constexpr size_t kFlatLongBytes = 80'000'000u;  // where staged rows have more than kFlatLong cells
+constexpr long long kFlatLong = 256;            // on average
 
 // A domain for threads that hold a cell index.
 struct FlatDomain {
@@ -740,7 +744,7 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
   e->ndomains = ndomains;
   e->collision = collision;
   e->storage = storage;
-  long long n = 0;
+  long long n = 0, rows = 0;
   for (int d = 0; d < ndomains; ++d) {
     const int64_t nx = counts[2 * d], ny = counts[2 * d + 1];
     if (nx <= 0 || ny <= 0) {
@@ -751,6 +755,7 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
     e->domains.push_back(dom);
     e->max_row = std::max(e->max_row, (int)ny);
     n += nx * ny;
+    rows += nx;
   }
   if (n >= ((long long)1 << 32)) {
     delete e;
@@ -777,7 +782,9 @@ int lbm_ensemble_create(int ndomains, const int64_t* counts, int collision,
   s.device = e->device;
   s.stream = e->stream;
   // Rows longer than the staged kernel's stages go through the tile kernel.
-  const bool flat = (size_t)n * 9 * lbm::pop_bytes(storage) <= kFlatBytes;
+  const bool long_rows = e->max_row <= kRowMax && n > kFlatLong * rows;
+  const bool flat =
+      (size_t)n * 9 * lbm::pop_bytes(storage) <= (long_rows ? kFlatLongBytes : kFlatBytes);
   e->tile = e->max_row <= kRowMax ? 0 : (flat ? lbm::kDirectThreads : 256);
   const size_t flag_bytes = ((size_t)n + 255) / 256 * 256;
   const size_t scratch = std::min((size_t)n * sizeof(int32_t), lbm::kFlagPiece);

@@ -23,7 +23,17 @@ _lib.lbm_last_error.restype = C.c_char_p
 
 MODES = {"persistent": 0, "graph": 1, "per_domain": 2}
 STORAGE = {"f32": 0, "f16": 1, "bf16": 2}
-FLAT_BYTES = 90 << 20  # populations of the largest ensemble that takes the flat kernel
+# Populations of the largest ensemble that takes the flat kernel; and where its rows can be staged and
+# have more than 256 cells on average.
+FLAT_BYTES, FLAT_LONG_BYTES = 90 << 20, 80_000_000
+
+
+def takes_flat(counts, storage: str) -> bool:
+    """Whether the library's default for an ensemble of these domains is the flat kernel."""
+    n, rows = sum(a * b for a, b in counts), sum(a for a, _ in counts)
+    long_rows = max(b for _, b in counts) <= 512 and n > 256 * rows
+    size = n * 9 * (4 if storage == "f32" else 2)
+    return size <= (FLAT_LONG_BYTES if long_rows else FLAT_BYTES)
 
 
 def _check(rc: int) -> None:
@@ -65,7 +75,7 @@ class Ensemble:
         # The library's default: the row-staged kernel (tile 0) when every row has at most 512
         # cells, else tiles of 256 cells, CTAs per SM as many as fit; for a small ensemble the flat
         # kernel (tiles 0 and 128).
-        self.flat = self.n * 9 * (4 if storage == "f32" else 2) <= FLAT_BYTES
+        self.flat = takes_flat(self.counts, storage)
         self.shape = (0 if max(b for _, b in self.counts) <= 512 else 128 if self.flat else 256, 0)
 
     def __del__(self):

@@ -247,8 +247,9 @@ LBM_API int lbm_ensemble_cells(lbm_ensemble* ens, int64_t* total);
  * per work item, loaded by TMA bulk copies into a shared-memory ring. A multiple of 32 in
  * [32, 512] selects the tile kernel with that many cells per tile (two per thread), loads straight
  * into registers. blocks_per_sm: CTAs per SM of the persistent grid (0 = as many as fit). Small
- * ensembles (at most 90 MB of populations) take a flat kernel with the shapes 0, 0 and 128, 0: one
- * cell a thread over all domains' cells in order, rows of any length; it is their default.
+ * ensembles (at most 90 MiB of populations, 80 MB where every row has at most 512 cells and the
+ * average more than 256) take a flat kernel with the shapes 0, 0 and 128, 0: one cell a thread over
+ * all domains' cells in order, rows of any length; it is their default.
  * Chosen by the autotuner (boltzmann_b200.autotune); every shape gives the same bits. */
 LBM_API int lbm_ensemble_set_shape(lbm_ensemble* ens, int tile_cells, int blocks_per_sm);
 LBM_API int lbm_ensemble_upload(lbm_ensemble* ens, const int32_t* flags, const float* rho,

@@ -8,7 +8,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from tests.fake_runtime import FakeSim, load
+from tests.fake_runtime import STORAGE, FakeSim, load
 
 
 @pytest.fixture(scope="module")
@@ -167,3 +167,24 @@ def test_launches_are_counted_by_kernel(lib, counts, storage, steps, launches):
     assert (direct.value, staged.value) == ((0, steps) if launches[2] else (steps, 0))
     assert lib.lbm_kernel_launches(sim.h, got, 3) != 0 and lib.lbm_kernel_launches(sim.h, None, 4) != 0
     sim.close()
+
+
+@pytest.mark.parametrize("counts,storage,kernel", [
+    ([(400, 505)] * 10, "f32", "flat"), ([(500, 505)] * 10, "f32", "rows"),
+    ([(500, 512)] * 16, "f16", "flat"), ([(500, 512)] * 20, "bf16", "rows"),
+    ([(300, 100)] * 85, "f32", "flat"), ([(300, 100)] * 88, "f32", "rows"),
+    ([(100, 256)] * 100, "f32", "flat"), ([(100, 257)] * 100, "f32", "rows"),
+    ([(100, 600)] * 43, "f32", "flat"), ([(100, 600)] * 44, "f32", "step"),
+    ([(64, 512), (256, 64)], "f32", "flat")])
+def test_flat_ensembles(lib, counts, storage, kernel):
+    """The default kernel on each side of the flat kernel's lines, and the Python class's copy of them."""
+    from boltzmann_b200.ensemble import takes_flat
+
+    h, om = C.c_void_p(), (C.c_float * len(counts))(*[1.5] * len(counts))
+    arr = (C.c_int64 * (2 * len(counts)))(*[c for pair in counts for c in pair])
+    assert lib.lbm_ensemble_create(len(counts), arr, 0, om, om, STORAGE[storage], C.byref(h)) == 0
+    lib.fake_take_log()
+    assert lib.lbm_ensemble_iterate(h, C.c_int64(2), 0) == 0, lib.lbm_last_error()
+    assert f"ensemble_{kernel}_kernel" in lib.fake_take_log().decode()
+    assert takes_flat(counts, storage) == (kernel == "flat")
+    lib.lbm_ensemble_destroy(h)
