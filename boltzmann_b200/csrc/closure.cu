@@ -700,42 +700,47 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
 // activation is read and widened once instead of nine times. FP32 on packed instructions (two
 // channels each): tensor cores would do it for less, but their accumulation leans to one side, and
 // the loss, an average over all cells, shows it. Two cells a thread, in three passes, so that each
-// shared-memory weight load feeds four of them. Batch 8 x 1024 x 512: 216 -> 118 us.
+// shared-memory weight load feeds four of them; on small batches in one pass on lower tiles (conv3_low).
+// Batch 8 x 1024 x 512: 216 -> 118 us.
 
-constexpr int kC3R = 30;                          // output rows of a tile (kTY columns)
-constexpr int kC3RegR = kC3R + 2, kC3RegC = kHY;  // region with the halo
-constexpr int kC3Cells = kC3RegR * kC3RegC;       // 2112
-constexpr int kC3Per = 2, kC3Threads = 352;       // three passes of two cells a thread
-constexpr size_t kConv3Smem = (size_t)9 * kC3Cells * 4 + (size_t)9 * C * 4;
-static_assert(kC3Cells % (kC3Threads * kC3Per) == 0 && kC3Threads % 32 == 0, "whole passes");
+constexpr int kC3R = 30, kC3Low = 6;         // output rows of a tile (kTY columns)
+constexpr int kC3RegC = kHY;                 // columns of the region with the halo
+constexpr int kC3Per = 2, kC3Threads = 352;  // cells a thread takes in a pass
+template <int R>
+constexpr int kC3Cells = (R + 2) * kC3RegC;  // 2112 in three passes, 528 in one
+template <int R>
+constexpr size_t kConv3Smem = (size_t)9 * kC3Cells<R> * 4 + (size_t)9 * C * 4;
 
+template <int R>
 __global__ void __launch_bounds__(kC3Threads, 2)
     conv3_fwd_kernel(Grid g, const bf16* __restrict__ a2, const bf16* __restrict__ w3,
                      const float* __restrict__ b3, float* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* ps = reinterpret_cast<float*>(smem_raw);  // [9][kC3Cells]
-  float* ws = ps + 9 * kC3Cells;                   // [tap][ci]
+  constexpr int kCells = kC3Cells<R>;
+  constexpr bool kWhole = kCells % (kC3Threads * kC3Per) == 0;  // no cell short in the last pass
+  float* ps = reinterpret_cast<float*>(smem_raw);  // [9][kCells]
+  float* ws = ps + 9 * kCells;                   // [tap][ci]
   for (int i = threadIdx.x; i < 9 * C; i += blockDim.x) ws[i] = bf(w3[i]);
   const float bias = b3[0];
   for (int64_t t = blockIdx.x; t < g.tiles; t += gridDim.x) {
     int64_t b, x0, y0;
     {
-      const int64_t per = g.tx * g.ty;  // this kernel's tiles are kC3R x kTY (see the launcher)
+      const int64_t per = g.tx * g.ty;  // this kernel's tiles are R x kTY (see the launcher)
       b = t / per;
       const int64_t r = t - b * per;
-      x0 = (r / g.ty) * kC3R;
+      x0 = (r / g.ty) * R;
       y0 = (r % g.ty) * kTY;
     }
     __syncthreads();  // the previous tile's P has been read (and, at first, ws written)
 #pragma unroll 1
-    for (int q0 = threadIdx.x; q0 < kC3Cells; q0 += kC3Per * kC3Threads) {
+    for (int q0 = threadIdx.x; q0 < kCells; q0 += kC3Per * kC3Threads) {
       uint4 v[kC3Per][C / 8];
 #pragma unroll
       for (int p = 0; p < kC3Per; ++p) {
         const int q = q0 + p * kC3Threads;
         const int r = q / kC3RegC, c = q - r * kC3RegC;
         const int64_t x = x0 - 1 + r, yy = y0 - 1 + c;
-        const bool in = x >= 0 && x < g.nx && yy >= 0 && yy < g.ny;
+        const bool in = (kWhole || q < kCells) && x >= 0 && x < g.nx && yy >= 0 && yy < g.ny;
         const uint4* src = reinterpret_cast<const uint4*>(a2 + (in ? g.cell(b, x, yy) : 0) * C);
 #pragma unroll
         for (int k = 0; k < C / 8; ++k) v[p][k] = in ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
@@ -770,17 +775,18 @@ __global__ void __launch_bounds__(kC3Threads, 2)
       for (int p = 0; p < kC3Per; ++p)
 #pragma unroll
         for (int tap = 0; tap < 9; ++tap)
-          ps[tap * kC3Cells + q0 + p * kC3Threads] = acc[p][tap].x + acc[p][tap].y;
+          if (kWhole || q0 + p * kC3Threads < kCells)
+            ps[tap * kCells + q0 + p * kC3Threads] = acc[p][tap].x + acc[p][tap].y;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kC3R * kTY; i += kC3Threads) {
+    for (int i = threadIdx.x; i < R * kTY; i += kC3Threads) {
       const int r = i / kTY, c = i - r * kTY;
       const int64_t x = x0 + r, yy = y0 + c;
       if (x >= g.nx || yy >= g.ny) continue;
       float s = 0.0f;
 #pragma unroll
       for (int tap = 0; tap < 9; ++tap)
-        s += ps[tap * kC3Cells + (r + tap / 3) * kC3RegC + c + tap % 3];
+        s += ps[tap * kCells + (r + tap / 3) * kC3RegC + c + tap % 3];
       y[g.cell(b, x, yy)] = s + bias;
     }
   }
@@ -2331,6 +2337,17 @@ bool shape_ok(int64_t nx, int64_t ny, int64_t batch) {
   return nx >= 2 && ny >= 2 && batch >= 1 && nx * ny * batch < (int64_t(1) << 40);
 }
 
+// Whether layer 3 takes its low tiles: where they need no more than twice the turns of the high ones at
+// two CTAs an SM, that is on small and thin batches. us, low / high: 32 x 32 3.8 / 8.2, 64 x 512 x 2
+// 6.5 / 9.5, 3 x 4000 x 8 9.7 / 23.5, 128 x 256 x 4 8.8 / 9.7, 300 x 200 x 4 15.6 / 16.3, 512 x 256 x 2
+// 13.0 / 10.1, 1024 x 512 24.8 / 17.3. The same bits.
+bool conv3_low(int64_t nx, int64_t ny, int64_t batch, int sms) {
+  auto turns = [&](int rows) {
+    return (tiles_of(nx, ny, batch, rows, kTY).tiles + 2 * sms - 1) / (2 * sms);
+  };
+  return turns(kC3Low) <= 2 * turns(kC3R);
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 cudaError_t set_smem(const void* fn, size_t bytes) {
@@ -2404,7 +2421,8 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
     if (cudaError_t e = set_smem((const void*)conv32_kernel<false>, kConv32Smem)) return e;
     if (cudaError_t e = set_smem((const void*)conv32_kernel<true>, kConv32Smem)) return e;
     if (cudaError_t e = set_smem((const void*)conv32_tc_kernel<false>, kTSmem)) return e;
-    if (cudaError_t e = set_smem((const void*)conv3_fwd_kernel, kConv3Smem)) return e;
+    if (cudaError_t e = set_smem((const void*)conv3_fwd_kernel<kC3R>, kConv3Smem<kC3R>)) return e;
+    if (cudaError_t e = set_smem((const void*)conv3_fwd_kernel<kC3Low>, kConv3Smem<kC3Low>)) return e;
     return cudaSuccess;
   });
   CL_CUDA(setup);
@@ -2431,11 +2449,17 @@ int lbm_closure_forward(const float* params, const uint16_t* params_bf16, const 
         params + LBM_CLOSURE_OFF_B2, nullptr, z2, reinterpret_cast<bf16*>(a2));
   }
   CL_CUDA(cudaGetLastError());
-  const Grid g3 = tiles_of(nx, ny, batch, kC3R, kTY);
-  const int grid3 = (int)std::min<int64_t>(g3.tiles, (int64_t)sms * 2);
-  conv3_fwd_kernel<<<grid3, kC3Threads, kConv3Smem, s>>>(g3, reinterpret_cast<const bf16*>(a2),
-                                                         wb + LBM_CLOSURE_OFF_W3,
-                                                         params + LBM_CLOSURE_OFF_B3, y);
+  auto conv3 = [&](auto rows) {
+    constexpr int R = decltype(rows)::value;
+    const Grid g3 = tiles_of(nx, ny, batch, R, kTY);
+    const int grid3 = (int)std::min<int64_t>(g3.tiles, (int64_t)sms * 2);
+    conv3_fwd_kernel<R><<<grid3, kC3Threads, kConv3Smem<R>, s>>>(
+        g3, reinterpret_cast<const bf16*>(a2), wb + LBM_CLOSURE_OFF_W3, params + LBM_CLOSURE_OFF_B3, y);
+  };
+  if (conv3_low(nx, ny, batch, sms))
+    conv3(std::integral_constant<int, kC3Low>{});
+  else
+    conv3(std::integral_constant<int, kC3R>{});
   CL_CUDA(cudaGetLastError());
   return LBM_OK;
 }
