@@ -229,6 +229,17 @@ bool staged_pays(const StepArgs<typename Pop<K>::real>& a) {
   return cells >= (one_tile ? (TRT ? 1200000 : 750000) : 1400000);
 }
 
+// Whether a step of the one-cell direct kernel is launched as a dependent one: with cells of much work
+// (FP64, or a run-time number of tracers) not where its grid fills half to three quarters of the chip's
+// CTA slots. The next grid's CTAs then find room on some SMs only while this one runs, and the SMs that
+// took more of them end last. us a step, dependent / plain: 36^3 FP64 with two tracers 8.6 / 7.1, 1 x 70000
+// 5.6 / 4.9, 300 x 200 5.4 / 5.0; 350 x 300 with two tracers 4.5 / 4.0, 62 x 17 x 48 5.0 / 4.6. With less
+// work a cell it pays there, too: 400 x 350 2.5 / 2.7, FP16 2.3 / 2.6, 40^3 FP16 3.2 / 3.5.
+template <int K, int NT>
+bool dependent_pays(long long ctas, long long room) {
+  return (K != kF64 && NT >= 0) || 2 * ctas <= room || 4 * ctas >= 3 * room;
+}
+
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
 cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t stream,
                        int64_t* launches) {
@@ -254,7 +265,7 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
     if ((long long)d.cells >= kPairDirectCells) {
       const unsigned grid = (unsigned)(((long long)d.cells + 2 * kDirectThreads - 1) / (2 * kDirectThreads));
       const cudaError_t e = launch_step_kernel(aa_step2_kernel<L, TRT, K, EVEN, NT, KT>, grid,
-                                               kDirectThreads, 0, stream, a, d);
+                                               kDirectThreads, 0, stream, true, a, d);
       if (e == cudaSuccess) {
         ++launches[lbm_sim::kDirectSteps];
         ++launches[lbm_sim::kKernels + LBM_KERNEL_STEP2];
@@ -262,9 +273,22 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
       return e;
     }
   }
-  const unsigned grid = (unsigned)(((long long)d.cells + kDirectThreads - 1) / kDirectThreads);
-  const cudaError_t e = launch_step_kernel(aa_step_kernel<L, TRT, K, EVEN, NT, KT>, grid,
-                                           kDirectThreads, 0, stream, a, d);
+  constexpr int threads = DirectForm<L, K, NT>::threads;
+  const unsigned grid = (unsigned)(((long long)d.cells + threads - 1) / threads);
+  auto kern = aa_step_kernel<L, TRT, K, EVEN, NT, KT>;
+  static DeviceOnce once;
+  static std::atomic<long long> room{0};
+  const cudaError_t setup_err = once([&] {
+    int device = 0, sms = 148, fit = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, 0);
+    room = (long long)sms * fit;
+    return e;
+  });
+  if (setup_err != cudaSuccess) return setup_err;
+  const cudaError_t e = launch_step_kernel(kern, grid, threads, 0, stream,
+                                           dependent_pays<K, NT>(grid, room), a, d);
   if (e == cudaSuccess) {
     ++launches[lbm_sim::kDirectSteps];
     ++launches[lbm_sim::kKernels + LBM_KERNEL_STEP];

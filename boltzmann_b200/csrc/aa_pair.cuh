@@ -333,7 +333,9 @@ constexpr long long kPairDirectCells = 148LL * 1024;
 // CTA's 256 consecutive cells. A 16-bit cell keeps half the bytes of an FP32 one in flight and
 // spends as many instructions; two cells on packed instructions mend both. 200^3 BGK 221 -> 194
 // us a step, 3000 x 1001 TRT with a 16-bit tracer 41.9 -> 38.6, 2000 x 1000 18.4 -> 16.1. Four CTAs
-// an SM for D3Q27 (three 220, five 214), six for D2Q9 (five 42.4, eight 45.0).
+// an SM for D3Q27 (three 220, five 214), six for D2Q9 (five 42.4, eight 45.0). The next step is let in at
+// the start: behind the loads, as in the one-cell kernel, it held the update up (BGK, 128 x 100 x 512
+// 159 -> 173, 4096 x 2048 with a 32-bit tracer 127 -> 135).
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT>
 __global__ void __launch_bounds__(kDirectThreads, L::Q >= 27 ? 4 : 6)
     aa_step2_kernel(const __grid_constant__ StepArgs<float> a,

@@ -24,9 +24,9 @@
 //
 // Bound by the instruction stream of the cell update on the larger domains (77% of issue slots at
 // 1000 x 501), by the latency of one exchange and two updates a pair on the smallest. us a step,
-// single-step launches and this kernel: 64^2 1.56 / 1.00, 256^2 2.31 / 1.33, 300^2 with a tracer
-// 2.79 / 1.92, 512 x 500 3.81 / 2.48, 1000 x 501 TRT 6.02 / 4.36, 32 x 2000 2.22 / 1.34, FP16 500^2
-// 3.28 / 2.56, FP64 400^2 4.31 / 3.73. (Two exchanges a pair without the ring's redundant cells: 1.75
+// single-step launches and this kernel: 64^2 1.57 / 1.00, 256^2 1.98 / 1.33, 300^2 with a tracer
+// 2.89 / 1.92, 512 x 500 3.68 / 2.48, 1000 x 501 TRT 6.01 / 4.36, 32 x 2000 1.99 / 1.34, FP16 500^2
+// 3.29 / 2.56, FP64 256^2 3.28 / 2.74. (Two exchanges a pair without the ring's redundant cells: 1.75
 // for 256^2, 5.61 for 1000 x 501. Slots at a run-time stride: 4.93 for 1000 x 501. At most 512
 // threads a CTA: 5.03.)
 #pragma once

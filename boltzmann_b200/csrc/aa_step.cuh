@@ -639,8 +639,8 @@ __device__ __forceinline__ void update_cell(const StepArgs<typename Pop<K>::real
 }
 
 // Programmatic dependent launch: the next step's grid may be scheduled as soon as every CTA of this
-// one has started (launch_dependents), so its launch, its index arithmetic and this grid's tail
-// overlap; it touches memory only after this grid has completed (wait).
+// one has called for it (launch_dependents) or ended, so its launch, its index arithmetic and this
+// grid's tail overlap; it touches memory only after this grid has completed (wait).
 __device__ __forceinline__ void grid_trigger_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -649,13 +649,14 @@ __device__ __forceinline__ void grid_wait_previous() {
 }
 
 // Launches a step kernel as a programmatic dependent of the previous one on the stream (the kernels
-// wait for it on the device before they touch memory).
+// wait for it on the device before they touch memory), or as a plain launch.
 template <class... Params, class... Args>
 cudaError_t launch_step_kernel(void (*kern)(Params...), unsigned grid, unsigned threads,
-                               size_t smem, cudaStream_t stream, const Args&... args) {
+                               size_t smem, cudaStream_t stream, bool dependent,
+                               const Args&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -677,14 +678,17 @@ constexpr int kDirectThreads = 128;
 // FP32 (six spill, 15% slower on 32^3), six for 16-bit populations. FP64 and D2Q9 without a tracer
 // are better off keeping them (256^2: 2.22 us a step against 2.32; the constant-bank table, cold in
 // every CTA, 2.57); D2Q9 with a tracer gains from forming them anew at ten CTAs (300^2: 3.15 ->
-// 2.81).
+// 2.81). FP64 in 3D takes CTAs of half the threads, which small domains spread more evenly (30^3 3.91 ->
+// 3.69), and with tracers eight of them an SM (32^3 with two 6.8 -> 5.6, 160^3 with one 367 -> 350;
+// without one six are better, 293 against 299).
 template <class L, int K, int NT>
 struct DirectForm {
   static constexpr bool k27 = L::Q >= 27;
   static constexpr bool table = k27 && K != kF64;
   static constexpr bool renew = table || (NT == 1 && (k27 || K != kF64));
+  static constexpr int threads = K == kF64 && k27 ? kDirectThreads / 2 : kDirectThreads;
   static constexpr int blocks =
-      K == kF64 ? (k27 ? 3 : 5) : (k27 ? (K == kF32 ? 5 : 6) : (NT == 1 ? 10 : 8));
+      K == kF64 ? (k27 ? (NT == 0 ? 6 : 8) : 5) : (k27 ? (K == kF32 ? 5 : 6) : (NT == 1 ? 10 : 8));
 };
 
 // Direct variant: one cell per thread, loads straight into registers; for domains whose rows do not
@@ -692,13 +696,17 @@ struct DirectForm {
 // small domains, by the instruction stream and the loads in flight on large ones.
 // Threads take the cells in order whatever the row length (two divisions by invariants): a CTA per
 // row left lanes without a cell on rows that are no multiple of 32 (half of them on 48 x 62 x 17)
-// and short CTAs on long ones. With the dependent launches: 64^2 1.94 -> 1.56 us a step, 300^2 with
-// a tracer 3.83 -> 3.15, 1000 x 501 7.13 -> 6.00, 100 x 90 x 35 (BF16, tracer) 20.5 -> 11.6.
+// and short CTAs on long ones. With the dependent launches: 64^2 1.98 -> 1.57 us a step, 300^2 with
+// a tracer 4.0 -> 2.9, 1000 x 501 7.2 -> 6.0, 100 x 90 x 35 (BF16, tracer) 18.0 -> 9.4.
+// The next grid is let in once this one's loads are under way. Let in at the start, its CTAs took slots,
+// more of them on some SMs than on others, before this grid's had begun their loads: 32^3 with a tracer
+// 3.45 us a step (3.2 in plain launches of a CTA a row), now 3.15, FP16 3.98 (3.15), now 2.89; 200^3
+// 301 -> 281, 160^3 FP64 323 -> 290, 4096 x 2048 114 -> 103.
 // NT: number of fused tracers known at compile time (0 or 1), or -1 for a runtime count.
 // Every load a cell needs is issued before the first branch on any loaded value, so each thread
 // has one memory phase (walls load populations they then ignore; they are a small fraction).
 template <class L, bool TRT, int K, bool EVEN, int NT, int KT = default_tracer_kind<K>()>
-__global__ void __launch_bounds__(kDirectThreads, DirectForm<L, K, NT>::blocks)
+__global__ void __launch_bounds__(DirectForm<L, K, NT>::threads, DirectForm<L, K, NT>::blocks)
     aa_step_kernel(const __grid_constant__ StepArgs<typename Pop<K>::real> a,
                    const __grid_constant__ DirectArgs d) {
   using P = Pop<K>;
@@ -707,8 +715,7 @@ __global__ void __launch_bounds__(kDirectThreads, DirectForm<L, K, NT>::blocks)
   using TP = TracerPop<KT>;
   using Form = DirectForm<L, K, NT>;
 
-  grid_trigger_next();
-  const unsigned cell = blockIdx.x * (unsigned)kDirectThreads + threadIdx.x;
+  const unsigned cell = blockIdx.x * (unsigned)Form::threads + threadIdx.x;
   const unsigned row = d.by_nz.div(cell);
   const int z = (int)(cell - row * (unsigned)a.nz);
   const unsigned x = L::D == 2 ? 0u : d.by_ny.div(row);
@@ -723,6 +730,7 @@ __global__ void __launch_bounds__(kDirectThreads, DirectForm<L, K, NT>::blocks)
     aa_load<TL, TP, EVEN, false, Form::table>(a.tr[0].g, d.slots.g, a.n, c, g);
   Real cval = 0;
   if (a.acc_mode == kAccBoussinesq) cval = a.coupled_val[c.cell];
+  grid_trigger_next();
   update_cell<L, TRT, K, EVEN, NT, GlobalSink<Form::table, Form::renew>, KT>(
       a, c, flag, f, g, cval, a.om_pos, a.om_neg,
       GlobalSink<Form::table, Form::renew>{Form::table ? &d.slots : nullptr});

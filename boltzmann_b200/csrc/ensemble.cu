@@ -113,11 +113,11 @@ __global__ void __launch_bounds__(512)
 // ---- The flat kernel: all domains' cells in order, one a thread, as dependent launches (aa_step.cuh).
 // For ensembles whose populations sit in L2, where the row-staged kernel's ring (a row a stage, its
 // fill and drain every step, whole SMs waiting on a launch) is longer than the work. us a step, row-
-// staged and flat: 9 domains of 210,371 cells in all 5.6 / 3.3, 72 of 369,358 11.2 / 5.1, 64 of
-// 1,574,641 25.2 / 16.5. Both lines lie before L2 is full. Rows of some 500 cells suit the ring: 75 MB
-// 22.5 / 21.8, FP16 79 MB 42.9 / 42.7, 93 MB 28.5 / 30.4, 29.7 / 36.4 (TRT), FP16 47.7 / 57.4. Rows
-// of 64 to 128 do not: 93 MB 54.0 / 36.8, FP16 89.0 / 56.0. Past L2 32 domains of 3,734,984 52.4 / 58.6,
-// FP16 128 of 13,045,701 130 / 168.
+// staged and flat: 5 domains of 286,708 cells in all 6.7 / 4.0, 33 of 296,474 8.3 / 4.2, 16 of 1,787,296
+// 23.0 / 17.9. Both lines lie before L2 is full. Rows of some 500 cells suit the ring: 75 MB 22.5 / 21.1,
+// FP16 79 MB 42.8 / 41.1, and at 93 MB, with the next step let in at the start, 28.5 / 30.4, 29.7 / 36.4
+// (TRT), FP16 47.7 / 57.4. Rows of 64 to 128 do not: 93 MB 53.3 / 34.1, FP16 89.0 / 52.8. Past L2 32
+// domains of 3,734,984 52.4 / 58.6, FP16 128 of 13,045,701 130 / 168.
 constexpr size_t kFlatBytes = 90u << 20;        // of populations
 constexpr size_t kFlatLongBytes = 80'000'000u;  // where staged rows have more than kFlatLong cells
 constexpr long long kFlatLong = 256;            // on average
@@ -143,7 +143,6 @@ __global__ void __launch_bounds__(lbm::kDirectThreads, 8)
   using namespace lbm;
   using P = Pop<K>;
   using Real = typename P::real;
-  grid_trigger_next();
   const unsigned cell = blockIdx.x * (unsigned)kDirectThreads + threadIdx.x;
   if (cell >= e.cells) return;
   // The tables never change, so they are read before the previous step has ended.
@@ -167,6 +166,7 @@ __global__ void __launch_bounds__(lbm::kDirectThreads, 8)
   Real f[D2Q9::Q];
   aa_load<D2Q9, P, EVEN, dev_in<K>()>(a.f, nullptr, a.n, c, f);
   Real g[1];
+  grid_trigger_next();
   update_cell<D2Q9, TRT, K, EVEN, 0, GlobalSink<>, default_tracer_kind<K>(), true>(
       a, c, flag, f, g, Real(0), (Real)dom.om_pos, (Real)dom.om_neg);
 }
@@ -566,7 +566,7 @@ cudaError_t launch_flat(lbm_ensemble* e, bool even, bool write_moments) {
   const FlatArgs args{e->d_flat, e->d_first, (unsigned)e->n};
   auto kern = even ? ensemble_flat_kernel<TRT, K, true> : ensemble_flat_kernel<TRT, K, false>;
   const unsigned grid = (unsigned)((e->n + lbm::kDirectThreads - 1) / lbm::kDirectThreads);
-  return lbm::launch_step_kernel(kern, grid, lbm::kDirectThreads, 0, e->stream, a, args);
+  return lbm::launch_step_kernel(kern, grid, lbm::kDirectThreads, 0, e->stream, true, a, args);
 }
 
 // The flat kernel's tables, in one allocation.

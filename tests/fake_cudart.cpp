@@ -23,7 +23,7 @@ constexpr int kSms = 148, kSharedOptIn = 232448;
 std::mutex g_mu;
 std::map<const void*, std::string> g_names;             // kernels by host address
 std::map<std::pair<int, const void*>, int> g_dynamic;   // opted-in shared memory, by device
-std::string g_log;                                      // "<device> <kernel>\n" for each launch
+std::string g_log;  // "<device> <kernel>\n" for each launch, "+dependent" behind a dependent one
 int g_cooperative = kSms;                               // CTAs of a cooperative grid that fit
 int g_pass = 0, g_fail = 0;                             // launches until the one that fails, its error
 
@@ -41,7 +41,7 @@ cudaError_t result(cudaError_t e) {
   return e;
 }
 
-cudaError_t launch(const void* f, dim3 grid, size_t smem, bool cooperative) {
+cudaError_t launch(const void* f, dim3 grid, size_t smem, bool cooperative, bool dependent) {
   std::lock_guard<std::mutex> lock(g_mu);
   if (g_fail != 0 && g_pass-- == 0) {
     const auto e = static_cast<cudaError_t>(g_fail);
@@ -53,7 +53,7 @@ cudaError_t launch(const void* f, dim3 grid, size_t smem, bool cooperative) {
     return result(cudaErrorInvalidValue);
   if (cooperative && (long long)grid.x * grid.y * grid.z > g_cooperative)
     return result(cudaErrorCooperativeLaunchTooLarge);
-  g_log += std::to_string(t_device) + " " + g_names[f] + "\n";
+  g_log += std::to_string(t_device) + " " + g_names[f] + (dependent ? "+dependent\n" : "\n");
   return cudaSuccess;
 }
 
@@ -100,13 +100,16 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) {
-  return launch(f, grid, smem, false);
+  return launch(f, grid, smem, false, false);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  bool cooperative = false;
-  for (unsigned k = 0; k < c->numAttrs; ++k)
+  bool cooperative = false, dependent = false;
+  for (unsigned k = 0; k < c->numAttrs; ++k) {
     if (c->attrs[k].id == cudaLaunchAttributeCooperative) cooperative = c->attrs[k].val.cooperative;
-  return launch(f, c->gridDim, c->dynamicSmemBytes, cooperative);
+    if (c->attrs[k].id == cudaLaunchAttributeProgrammaticStreamSerialization)
+      dependent = c->attrs[k].val.programmaticStreamSerializationAllowed;
+  }
+  return launch(f, c->gridDim, c->dynamicSmemBytes, cooperative, dependent);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   std::lock_guard<std::mutex> lock(g_mu);

@@ -188,3 +188,20 @@ def test_flat_ensembles(lib, counts, storage, kernel):
     assert f"ensemble_{kernel}_kernel" in lib.fake_take_log().decode()
     assert takes_flat(counts, storage) == (kernel == "flat")
     lib.lbm_ensemble_destroy(h)
+
+
+@pytest.mark.parametrize("counts,storage,tracers,dependent", [
+    ((30, 20, 10), "f32", 0, True), ((60, 50, 40), "f32", 0, True), ((60, 50, 40), "f64", 0, True),
+    ((16, 16, 16), "f64", 1, True), ((18, 18, 18), "f64", 1, False), ((23, 23, 23), "f32", 2, False),
+    ((40, 30, 30), "f32", 2, True), ((200, 20), "f32", 3, True)])
+def test_dependent_launches(lib, counts, storage, tracers, dependent):
+    """Cells of much work (FP64, several tracers) are not launched as dependents where the grid fills
+    half to three quarters of the chip's slots: here one CTA an SM, 148."""
+    sim = FakeSim(lib, counts, storage=storage, tracer="32" if tracers else None)
+    for _ in range(tracers - 1):
+        sim.check(lib.lbm_add_tracer(sim.h, {2: 5, 3: 7}[len(counts)], 0, C.c_float(1.5), C.c_float(0),
+                                     C.byref(C.c_int())))
+    lib.fake_take_log()
+    sim.check(sim.iterate(2))
+    assert [name.endswith("+dependent") for _, name in sim.launched()] == [dependent] * 2
+    sim.close()
