@@ -184,49 +184,49 @@ cudaError_t launch_tma(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
 }
 
 // Whether the TMA-staged kernel is the faster one for rows of whole 256-cell tiles (fused tracers: none
-// or one). It keeps more loads in flight per SM with fewer instructions, the direct kernel more warps
+// or one). It keeps more loads in flight per SM with fewer instructions, the direct kernels more warps
 // at work: domains that sit in L2, and FP32 or FP64 cells with more arithmetic per byte, are better off
-// direct. In 16 bits rows of several tiles pay from some 95 MB of populations, of one tile, whose even
-// steps return by rows too, from half of that. us a step, direct / staged, each the median of a second
-// under its own load:
-//   D2Q9  FP32         2048x1024 20.8 / 26.1, 1500x2560 53.0 / 52.4 (TRT 53.4 / 54.0), 4096x2048
-//                      114 / 111 (TRT 115.2 / 114.9)
-//         with tracer  2048x512 14.6 / 18.7, 2048x1024 43.6 / 43.3; 4096x2048 166 / 174 in a periodic
-//                      box, 176 / 171 in a channel
-//         FP64         2048x512 22.8 / 26.9, 1500x2560 105 / 101; with a tracer, TRT, 164 / 179
+// direct. Rows of one tile, whose even steps return by rows too, suit it best. us a step, direct /
+// staged, each the median of some tenths of a second under its own load:
+//   D2Q9  FP32         2048x1024 20.2 / 26.3, 1500x2560 47.8 / 52.4, 4096x2048 103 / 112, in a channel
+//                      with TRT 109 / 114
+//         with tracer  2048x1024 42.2 / 43.3; 4096x2048 159 / 175 in a periodic box, in a channel with
+//                      TRT 170.3 / 170.3
+//         FP64         2048x512 21.4 / 27.2, 1500x2560 94 / 101, 4096x2048 207 / 211
 //         FP16         2048x1024 16.8 / 21.6, 4096x2048 73.4 / 77.4 (TRT 78.3 / 78.0)
-//         FP32 tracer  2048x512 12.8 / 15.4, 1500x1536 33.6 / 31.2, 8000x768 94.6 / 90.2
+//         FP32 tracer  2048x512 12.8 / 15.4, 2048x1024 28.3 / 28.1, 1500x1536 33.6 / 31.2, 8000x768
+//                      94.6 / 90.2
 //         FP16 tracer  1000x2560 31.5 / 33.1, 1500x2560 52.9 / 50.9, 4096x2048 113 / 111; TRT
 //                      1500x1536 29.4 / 30.2, 1000x2560 34.2 / 33.5, 4096x2048 121 / 111
-//   D3Q27 FP32 BGK     24x48x256 8.1 / 10.1, 48x64x256 24.4 / 24.0, 128x100x512 245 / 241
-//         FP32 TRT     48x64x256 25.4 / 31.8, 100x100x256 101 / 107, 128x100x512 255 / 356;
-//                      with a tracer 100x100x256 121 / 132, 128x100x512 307 / 436
-//         FP64         24x48x256 19.5 / 20.5, 48x64x256 64.3 / 60.8; with a tracer 82.4 / 74.9
+//   D3Q27 FP32 BGK     48x64x256 23.5 / 24.0, 64x64x256 with a relaxation field 43.4 / 41.1, 256^3
+//                      617 / 583; 128x100x512 231 / 241
+//         FP32 TRT     100x100x256 92.9 / 107, 256^3 612 / 668; with a tracer 120 / 132
+//         FP64         100x100x256 182.3 / 182.4, 256^3 1173 / 1170, 24x48x1024 85.0 / 93.7; with a
+//                      tracer 224 / 226, 105 / 114
 //         FP16 BGK     24x48x256 7.7 / 8.6, 48x64x256 17.4 / 15.9; 48x64x512 35.9 / 38.2, 40x90x512
 //                      44.3 / 43.7, 128x100x512 159 / 157
-//         FP16 TRT     24x48x256 7.9 / 9.4, 48x64x256 18.3 / 18.1, 100x100x256 73.4 / 53.8; 48x64x512
-//                      38.8 / 40.6, 40x90x512 50.2 / 46.9, 128x100x512 184 / 160, 100x100x1024 286 / 249
-//         FP32 tracer  24x48x256 9.7 / 11.4, 48x64x256 23.8 / 22.4; 32x48x512 23.7 / 26.4, 24x48x1024
-//                      43.3 / 41.4, 128x100x512 248 / 222 (TRT 272 / 234)
-//         FP16 tracer  24x48x256 9.7 / 11.3, 48x64x256 22.6 / 21.8; 24x48x1024 36.4 / 38.2, 48x64x512
-//                      54.5 / 51.3, 128x100x512 226 / 202; TRT 64x64x256 32.2 / 33.7, 64x90x256
-//                      52.9 / 48.0, 48x64x512 56.1 / 55.7, 128x100x512 230 / 215
+//         FP16 TRT     24x48x256 7.9 / 9.4, 48x64x256 18.4 / 18.1, 256^3 464 / 362; 48x64x512 37.7 /
+//                      41.0, 40x90x512 47.6 / 47.3, 128x100x512 175 / 160
+//         FP32 tracer  48x64x256 21.2 / 22.3, 64x64x256 30.8 / 30.6, 100x100x256 87.0 / 79.3; 128x100x512
+//                      219 / 223; TRT 64x64x256 32.0 / 37.1, 64x90x256 52.6 / 52.2, 128x100x512 226 / 234
+//         FP16 tracer  48x64x256 21.9 / 21.8, 64x90x256 48.6 / 42.1; 24x48x1024 34.3 / 38.3, 48x64x512
+//                      51.5 / 51.3, 128x100x512 214 / 201; TRT 64x90x256 45.7 / 48.3, 100x100x256 80.7 /
+//                      79.2, 128x100x512 201 / 215
 // KT: storage kind of the tracer's populations.
 template <class L, bool TRT, int K, int NT, int KT>
 bool staged_pays(const StepArgs<typename Pop<K>::real>& a) {
   const long long cells = (long long)a.nx * a.ny * a.nz;
-  constexpr bool wide_tracer = KT == kF32;
-  if (L::D == 2) {
-    if (K == kF64) return NT == 0 && cells >= 1500000;
-    if (K == kF32) return cells >= (NT == 0 ? (TRT ? 6000000 : 3500000) : 2000000);
-    return NT != 0 && cells >= (wide_tracer ? 2200000 : (TRT ? 2500000 : 3000000));
-  }
-  if (K == kF32 && (TRT || NT != 0)) return false;
-  if (!dev_in<K>()) return cells >= 700000;
   const bool one_tile = a.nz == kTmaTile;
+  constexpr bool wide_tracer = KT == kF32;
+  if (K == kF64) return false;
+  if (L::D == 2) {
+    if (K == kF32) return NT != 0 && cells >= 6000000;
+    return NT != 0 && cells >= (wide_tracer ? 2000000 : (TRT ? 2500000 : 3000000));
+  }
+  if (K == kF32) return !TRT && NT == 0 && one_tile && cells >= 700000;
   if (NT == 0) return cells >= (one_tile ? 700000 : 1700000);
-  if (wide_tracer) return cells >= (one_tile ? 750000 : 1100000);
-  return cells >= (one_tile ? (TRT ? 1200000 : 750000) : 1400000);
+  if (wide_tracer) return one_tile && cells >= (TRT ? 1400000 : 1000000);
+  return one_tile ? cells >= (TRT ? 2000000 : 750000) : !TRT && cells >= 1400000;
 }
 
 // Whether a step of the one-cell direct kernel is launched as a dependent one: with cells of much work
@@ -262,7 +262,7 @@ cudaError_t launch_one(const StepArgs<typename Pop<K>::real>& a, cudaStream_t st
   const DirectArgs d = make_direct_args<L>(a, sizeof(typename Pop<K>::type),
                                            sizeof(typename TracerPop<KT>::type));
   if constexpr (pair_form<L, TRT, K, NT>()) {
-    if ((long long)d.cells >= kPairDirectCells) {
+    if ((long long)d.cells >= pair_direct_cells<L>()) {
       const unsigned grid = (unsigned)(((long long)d.cells + 2 * kDirectThreads - 1) / (2 * kDirectThreads));
       const cudaError_t e = launch_step_kernel(aa_step2_kernel<L, TRT, K, EVEN, NT, KT>, grid,
                                                kDirectThreads, 0, stream, true, a, d);

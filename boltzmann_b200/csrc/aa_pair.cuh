@@ -325,9 +325,15 @@ template <class L, bool TRT, int K, int NT>
 constexpr bool pair_form() {
   return dev_in<K>() && ((L::Q >= 27 && !TRT && NT == 0) || (L::D == 2 && (NT == 0 || NT == 1)));
 }
-// Smallest domain (cells) for the direct two-cell kernel, 1024 cells an SM: below it the CTAs of
-// 256 cells would leave SMs short of warps.
-constexpr long long kPairDirectCells = 148LL * 1024;
+// Smallest domain (cells) for the direct two-cell kernel: below it its CTAs, half as many, leave SMs short
+// of warps. us a step, one cell a thread / two: 450 x 400 2.66 / 2.92, 500 x 451 3.12 / 2.93 (TRT 3.30 /
+// 2.92), 2000 x 1001 18.2 / 16.2; with a tracer 3.2 / 3.6, 4.0 / 3.8, 23.8 / 23.2 (between, at 600 x 501
+// and 1000 x 501, 4.6 / 4.8 and 6.8 / 7.0); 60 x 60 x 50 5.5 / 5.9, 90 x 90 x 80 15.1 / 15.0, 180 x 150 x
+// 100 72.7 / 67.6.
+template <class L>
+constexpr long long pair_direct_cells() {
+  return L::D == 2 ? 200000 : 700000;
+}
 
 // The direct kernel with two cells a thread, for 16-bit populations: cells t and t + 128 of the
 // CTA's 256 consecutive cells. A 16-bit cell keeps half the bytes of an FP32 one in flight and

@@ -139,10 +139,11 @@ size_t mail_bytes(lbm_sim& s) {
 // Whether a simulation that is stepped beside others (threads, streams) should still take the resident
 // kernel: resident launches whose CTAs do not fit the chip side by side take turns, while the single
 // steps of several small domains overlap. us a step and simulation, single steps / resident, in calls
-// of 200 steps by a thread each: 128^2 two at once 0.97 / 1.05, three 0.80 / 1.03, eight 0.36 / 1.02;
-// 256^2 two 1.29 / 1.33, three 1.00 / 1.31, eight 0.66 / 1.30; 400 x 350 three 1.46 / 1.77; 512 x 500
-// four 2.30 / 2.46, eight 2.35 / 2.46; 64^2, of which two fit, four 0.51 / 0.48, eight 0.30 / 0.47. The
-// line lies at three turns, below 200,000 cells. The results are the same either way.
+// of 200 steps by a thread each: 128^2 two at once 0.87 / 1.04, three 0.71 / 1.03, eight 0.33 / 1.02;
+// 256^2 two 1.16 / 1.33, three 0.92 / 1.31, eight 0.64 / 1.30; 400 x 350 three 1.41 / 1.77; 512 x 500
+// four 2.29 / 2.46, eight 2.32 / 2.46; 64^2, of which two fit, four 0.45 / 0.48, eight 0.27 / 0.47. The
+// line lies at three turns, below 200,000 cells: a simulation that shares the chip for part of a call
+// only is not sent to single steps by that. The results are the same either way.
 bool worth_waiting(const lbm_sim& s, const ResidentArgs& d) {
   if (s.n >= 200000) return true;
   int sms = 0;
@@ -181,6 +182,10 @@ auto with_variant(const lbm_sim& s, int nt, F fn) {
   }
 }
 
+// FP64, whose updates take longest, gains by the kernel on small domains only: 256^2 2.74 us a step, 3.40
+// in single steps; 300 x 299 3.7 and 3.6, with a tracer 4.8 and 4.4, 512 x 500 6.7 and 6.4.
+bool resident_size(const lbm_sim& s) { return s.storage != kF64 || s.n <= 80000; }
+
 struct MailBytes {
   lbm_sim& s;
   template <int K, int NT, int KT>
@@ -200,16 +205,16 @@ struct Iterate {
 }  // namespace
 
 size_t resident_mail_bytes(lbm_sim& s, int tracers) {
-  if (s.dim != 2 || s.q != D2Q9::Q || tracers > 1) return 0;
+  if (s.dim != 2 || s.q != D2Q9::Q || tracers > 1 || !resident_size(s)) return 0;
   return with_variant(s, tracers, MailBytes{s});
 }
 
 cudaError_t iterate_resident(lbm_sim& s, int64_t steps) {
   // A launch costs the way of the domain into and out of shared memory (6 us for 64^2, 16 us for
-  // 1000 x 501), which some steps have to earn: measured even with single steps at 4 of them for
-  // 64^2, 6 for 256^2, 10 for 512 x 500, 14 for 700 x 451 in FP16.
+  // 1000 x 501), which some steps have to earn: measured even with single steps at 6 of them for 64^2, 8
+  // for 256^2, 12 for 512 x 500, 14 for 700 x 451 in FP16.
   if (s.dim != 2 || s.q != D2Q9::Q || s.kernel_path != 0 || s.tracers.size() > 1 ||
-      steps < 4 + s.n / 32768)
+      steps < 6 + s.n / 32768 || !resident_size(s))
     return cudaErrorNotSupported;
   return with_variant(s, (int)s.tracers.size(), Iterate{s, steps});
 }

@@ -33,23 +33,26 @@ def _run(counts, reps, storage, kind, tracer):
 
 
 # Cells modulo the 256 of a CTA: 3 (no second cells, and threads without a first), 128 (no second
-# cells), 200 (some), 255. The kernel starts at 148 x 1024 = 151,552 cells.
-@pytest.mark.parametrize("counts,reps", [((1, 30311), (5, 1)), ((32, 79), (6, 10)),
-                                         ((3, 6323), (8, 1)), ((31, 59), (1, 83))])
+# cells), 200 (some), 255. The kernel starts at 200,000 cells in 2D and 700,000 in 3D.
+LINE = {2: 200000, 3: 700000}
+
+
+@pytest.mark.parametrize("counts,reps", [((11, 449), (1, 41)), ((32, 45), (14, 10)),
+                                         ((24, 241), (7, 5)), ((33, 65), (19, 5))])
 @pytest.mark.parametrize("storage,tracer", [("f16", ""), ("bf16", "32"), ("f16", "16")])
 @pytest.mark.parametrize("kind", [0, 1])
 def test_domains_that_end_within_a_cta_2d(counts, reps, storage, tracer, kind):
     _check(counts, reps, storage, kind, tracer)
 
 
-@pytest.mark.parametrize("counts,reps", [((1, 17, 1783), (5, 1, 1)), ((4, 8, 79), (3, 4, 5))])
+@pytest.mark.parametrize("counts,reps", [((15, 17, 107), (5, 11, 1)), ((8, 35, 67), (16, 5, 1))])
 @pytest.mark.parametrize("storage", ["f16", "bf16"])
 def test_domains_that_end_within_a_cta_3d(counts, reps, storage):
     _check(counts, reps, storage, 0, "")
 
 
 def _check(counts, reps, storage, kind, tracer):
-    assert np.prod(counts) < 151552 <= np.prod(counts) * np.prod(reps)
+    assert np.prod(counts) < LINE[len(counts)] <= np.prod(counts) * np.prod(reps)
     small = _run(counts, [1] * len(counts), storage, kind, tracer)
     large = _run(counts, reps, storage, kind, tracer)
     for a, b in zip(small, large):

@@ -18,7 +18,7 @@ def lib(tmp_path_factory):
 
 @pytest.mark.parametrize("counts,storage,kernel", [((64, 64), "f32", "aa_resident_kernel"),
                                                    ((200, 150), "f16", "aa_resident_kernel"),
-                                                   ((64, 64, 256), "f32", "aa_tma_kernel")])
+                                                   ((64, 64, 256), "f16", "aa_tma_kernel")])
 def test_kernels_are_set_up_on_every_device(lib, counts, storage, kernel):
     """Shared memory above 48 KB is opted into per device: a simulation on a second GPU of the
     process runs as one on the first, in either order and again."""
@@ -100,24 +100,30 @@ def test_a_poll_limit_does_not_change_the_kernel(lib):
 
 
 @pytest.mark.parametrize("counts,storage,kind,tracer,staged", [
-    # Rows of several tiles, 16-bit storage in 3D: staged from what L2 no longer holds.
+    # 3D in 16 bits, rows of several tiles and of one.
     ((32, 48, 512), "f16", 1, "", False), ((70, 90, 512), "f16", 1, "", True),
     ((32, 48, 1024), "f16", 0, "", False), ((70, 45, 1024), "bf16", 0, "", True),
-    ((32, 48, 512), "f16", 1, "32", False), ((48, 64, 512), "f16", 1, "32", True),
-    ((32, 48, 512), "f16", 0, "16", False), ((40, 90, 768), "bf16", 1, "16", True),
-    # Rows of one tile.
+    ((128, 100, 512), "f16", 1, "32", False), ((128, 100, 512), "f16", 0, "32", False),
+    ((32, 48, 512), "f16", 0, "16", False), ((40, 90, 768), "bf16", 0, "16", True),
+    ((40, 90, 768), "f16", 1, "16", False),
     ((24, 48, 256), "f16", 1, "", False), ((64, 64, 256), "f16", 1, "", True),
-    ((64, 64, 256), "f16", 0, "32", True), ((64, 64, 256), "f16", 0, "16", True),
-    ((64, 64, 256), "f16", 1, "16", False), ((64, 90, 256), "f16", 1, "16", True),
+    ((48, 64, 256), "f16", 0, "32", False), ((64, 64, 256), "f16", 0, "32", True),
+    ((64, 64, 256), "f16", 1, "32", False), ((64, 90, 256), "f16", 1, "32", True),
+    ((64, 64, 256), "f16", 0, "16", True), ((64, 90, 256), "f16", 1, "16", False),
+    ((100, 100, 256), "f16", 1, "16", True),
+    # 3D in full precision.
+    ((24, 48, 256), "f32", 0, "", False), ((48, 64, 256), "f32", 0, "", True),
+    ((128, 128, 256), "f32", 1, "", False), ((128, 64, 512), "f32", 0, "", False),
+    ((128, 128, 256), "f32", 0, "32", False), ((100, 100, 256), "f64", 0, "", False),
     # 2D.
     ((4096, 2048), "f16", 1, "", False), ((2048, 512), "f16", 0, "32", False),
     ((1500, 1536), "f16", 0, "32", True), ((1500, 1536), "f16", 1, "16", False),
     ((1500, 2560), "f16", 1, "16", True), ((1500, 2560), "bf16", 0, "16", True),
-    ((1500, 2560), "f32", 0, "", True), ((1500, 2560), "f32", 1, "", False),
-    ((1500, 2560), "f64", 1, "64", False), ((1500, 2560), "f64", 0, "", True),
+    ((4096, 2048), "f32", 0, "", False), ((4096, 2048), "f32", 1, "32", True),
+    ((2048, 1024), "f32", 1, "32", False), ((1500, 2560), "f64", 0, "", False),
 ])
 def test_staged_where_it_is_the_faster_kernel(lib, counts, storage, kind, tracer, staged):
-    """One domain on each side of every line of staged_pays (aa_launch.cuh) that is not obvious."""
+    """One domain on each side of every line of staged_pays (aa_launch.cuh)."""
     sim = FakeSim(lib, counts, kind=kind, storage=storage, tracer=tracer)
     sim.check(sim.iterate(2))
     kernels = set(sim.kernels())
@@ -154,8 +160,8 @@ def test_small_simulations_side_by_side_do_not_queue_for_the_chip(lib):
 
 @pytest.mark.parametrize("counts,storage,steps,launches", [
     ((64, 64), "f32", 8004, [0, 0, 0, 3]), ((64, 64), "f32", 2, [2, 0, 0, 0]),
-    ((400, 390), "f16", 6, [0, 6, 0, 0]), ((50, 40, 30), "f32", 30, [30, 0, 0, 0]),
-    ((64, 64, 256), "f32", 30, [0, 0, 30, 0])])
+    ((500, 410), "f16", 6, [0, 6, 0, 0]), ((50, 40, 30), "f32", 30, [30, 0, 0, 0]),
+    ((64, 64, 256), "f16", 30, [0, 0, 30, 0])])
 def test_launches_are_counted_by_kernel(lib, counts, storage, steps, launches):
     sim = FakeSim(lib, counts, storage=storage)
     sim.check(sim.iterate(steps))
@@ -188,6 +194,20 @@ def test_flat_ensembles(lib, counts, storage, kernel):
     assert f"ensemble_{kernel}_kernel" in lib.fake_take_log().decode()
     assert takes_flat(counts, storage) == (kernel == "flat")
     lib.lbm_ensemble_destroy(h)
+
+
+@pytest.mark.parametrize("counts,storage,steps,kernel", [
+    ((64, 64), "f32", 4, "aa_step_kernel"), ((64, 64), "f32", 6, "aa_resident_kernel"),
+    ((500, 400), "f32", 12, "aa_resident_kernel"), ((500, 400), "f32", 10, "aa_step_kernel"),
+    ((280, 280), "f64", 10, "aa_resident_kernel"), ((290, 290), "f64", 10, "aa_step_kernel"),
+    ((499, 400), "f16", 2, "aa_step_kernel"), ((501, 400), "f16", 2, "aa_step2_kernel"),
+    ((60, 160, 72), "f16", 2, "aa_step_kernel"), ((61, 160, 72), "bf16", 2, "aa_step2_kernel"),
+    ((501, 400), "f32", 2, "aa_step_kernel")])
+def test_kernels_on_each_side_of_their_lines(lib, counts, storage, steps, kernel):
+    sim = FakeSim(lib, counts, storage=storage)
+    sim.check(sim.iterate(steps))
+    assert set(sim.kernels()) == {kernel}
+    sim.close()
 
 
 @pytest.mark.parametrize("counts,storage,tracers,dependent", [
