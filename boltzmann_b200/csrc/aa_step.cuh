@@ -692,7 +692,7 @@ struct DirectForm {
 };
 
 // Direct variant: one cell per thread, loads straight into registers; for domains whose rows do not
-// split into whole tiles, and small ones. Bound by the latency of one dependent chain per step on
+// split into whole tiles, and for those where it is the faster kernel (staged_pays). Bound by the latency of one dependent chain per step on
 // small domains, by the instruction stream and the loads in flight on large ones.
 // Threads take the cells in order whatever the row length (two divisions by invariants): a CTA per
 // row left lanes without a cell on rows that are no multiple of 32 (half of them on 48 x 62 x 17)

@@ -1,5 +1,5 @@
-// TMA-staged variant of the AA step: the main kernel for domains whose contiguous axis is a
-// multiple of 256 cells (kTmaTile).
+// TMA-staged variant of the AA step, for domains whose contiguous axis is a multiple of 256 cells
+// (kTmaTile), where it is the faster kernel (staged_pays, aa_launch.cuh).
 //
 // Work unit: a tile of T consecutive cells of one grid row (T threads, one cell each). A
 // persistent CTA walks its tiles with an S-stage ring in shared memory. For every tile, the

@@ -55,7 +55,7 @@ enum lbm_storage {
 };
 
 enum lbm_kernel_path {
-  LBM_PATH_AUTO = 0,   /* staged for large domains whose rows split into 256-cell tiles */
+  LBM_PATH_AUTO = 0,   /* the fastest kernel for the domain and storage */
   LBM_PATH_DIRECT = 1, /* one cell per thread, loads straight into registers */
   LBM_PATH_STAGED = 2  /* TMA bulk copies into a shared-memory ring (rows of 256k cells only) */
 };
