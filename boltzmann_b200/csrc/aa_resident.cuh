@@ -22,7 +22,7 @@
 //
 // The cells of a tile that touch no other tile are updated while the messages are under way.
 //
-// Bound by the instruction stream of the cell update on the larger domains (77% of issue slots at
+// Bound by the instruction stream of the cell update on the larger domains (76% of issue slots at
 // 1000 x 501), by the latency of one exchange and two updates a pair on the smallest. us a step,
 // single-step launches and this kernel: 64^2 1.57 / 1.00, 256^2 1.98 / 1.33, 300^2 with a tracer
 // 2.89 / 1.92, 512 x 500 3.68 / 2.48, 1000 x 501 TRT 6.01 / 4.36, 32 x 2000 1.99 / 1.34, FP16 500^2
